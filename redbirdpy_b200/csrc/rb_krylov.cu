@@ -1314,21 +1314,35 @@ constexpr int64_t kMaxCols = 128;  // columns per Krylov block
 __device__ __forceinline__ double sq_abs(double v) { return v * v; }
 __device__ __forceinline__ double sq_abs(cdouble v) { return v.x * v.x + v.y * v.y; }
 
-// out[i * k + c] = sum over instance i's rows of |X[r][c]|^2: one block per
-// instance, warps over rows, lanes over columns, summed in a fixed order
+// Squared norms of the instances' rows, in parts: an instance's rows are cut
+// into seg_parts(ninst) equal runs and block (i, p) sums run p, warps over
+// rows and lanes over columns (4 rows in flight per warp), into
+// part[(i * np + p) * k + c]; the kernels that use a norm add its np parts in
+// order (seg_sum), so the sums are the same from run to run.  The kernel is a
+// plain read of X (bound: HBM), which needs every SM: one block per instance
+// kept 64 instances (0.7 M rows of 32 FP64 columns) on 64 SMs with one row in
+// flight per warp, 3.1 ms per call, and the largest instance alone set the end.
 constexpr int kSegWarps = 8;
+constexpr int kSegPartsMax = 64;
+static int64_t seg_parts(int64_t ninst) {
+  // about 8 blocks per SM over all instances
+  return std::max<int64_t>(1, std::min<int64_t>(kSegPartsMax, ceil_div(148 * 8, std::max<int64_t>(ninst, 1))));
+}
 template <typename T64>
 __global__ void __launch_bounds__(kSegWarps * 32)
-seg_norm_kernel(int64_t ninst, int64_t k, const int64_t* __restrict__ row_ptr, const T64* __restrict__ X,
-                double* __restrict__ out) {
+seg_norm_kernel(int64_t ninst, int64_t np, int64_t k, const int64_t* __restrict__ row_ptr,
+                const T64* __restrict__ X, double* __restrict__ part) {
   __shared__ double sm[kSegWarps][kMaxCols];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  for (int64_t i = blockIdx.x; i < ninst; i += gridDim.x) {
+  for (int64_t t = blockIdx.x; t < ninst * np; t += gridDim.x) {
+    const int64_t i = t / np, p = t - i * np;
+    const int64_t i0 = row_ptr[i], len = row_ptr[i + 1] - i0;
+    const int64_t r0 = i0 + len * p / np, r1 = i0 + len * (p + 1) / np;
     double a[kMaxCols / 32];
 #pragma unroll
     for (int q = 0; q < kMaxCols / 32; ++q) a[q] = 0.0;
-    const int64_t r1 = row_ptr[i + 1];
-    for (int64_t r = row_ptr[i] + w; r < r1; r += kSegWarps) {
+#pragma unroll 4
+    for (int64_t r = r0 + w; r < r1; r += kSegWarps) {
       const T64* xr = X + r * k;
 #pragma unroll
       for (int q = 0; q < kMaxCols / 32; ++q)
@@ -1339,27 +1353,38 @@ seg_norm_kernel(int64_t ninst, int64_t k, const int64_t* __restrict__ row_ptr, c
       if (lane + 32 * q < k) sm[w][lane + 32 * q] = a[q];
     __syncthreads();
     for (int64_t c = threadIdx.x; c < k; c += blockDim.x) {
-      double t = 0.0;
+      double s = 0.0;
 #pragma unroll
-      for (int q = 0; q < kSegWarps; ++q) t += sm[q][c];
-      out[i * k + c] = t;
+      for (int q = 0; q < kSegWarps; ++q) s += sm[q][c];
+      part[t * k + c] = s;
     }
     __syncthreads();
   }
 }
 
-__global__ void seg_bnorm_kernel(int64_t m, const double* __restrict__ s2, OuterState* __restrict__ seg) {
+// the squared norm of (instance, column) j = i k + c from its np parts
+__device__ __forceinline__ double seg_sum(const double* __restrict__ part, int64_t np, int64_t k, int64_t j) {
+  const int64_t i = j / k, c = j - i * k;
+  double s = 0.0;
+#pragma unroll 4
+  for (int64_t p = 0; p < np; ++p) s += part[(i * np + p) * k + c];
+  return s;
+}
+
+__global__ void seg_bnorm_kernel(int64_t m, int64_t np, int64_t k, const double* __restrict__ part,
+                                 OuterState* __restrict__ seg) {
   const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (j >= m) return;
-  seg[j] = outer_start(s2[j]);
+  seg[j] = outer_start(seg_sum(part, np, k, j));
 }
 
 // the rules of fin_outer_kernel, per (instance, column)
-__global__ void seg_outer_kernel(int64_t m, const double* __restrict__ s2, OuterState* __restrict__ seg, double tol,
-                                 double stall, double inner_tol, double itol_min) {
+__global__ void seg_outer_kernel(int64_t m, int64_t np, int64_t k, const double* __restrict__ part,
+                                 OuterState* __restrict__ seg, double tol, double stall, double inner_tol,
+                                 double itol_min) {
   const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (j >= m || !seg[j].active) return;
-  const double s = s2[j];
+  const double s = seg_sum(part, np, k, j);
   OuterState o = seg[j];
   const double rel = sqrt(s) / o.bnorm;
   o.prev = o.relres;
@@ -1695,11 +1720,11 @@ struct SolveBufs {
 struct SegBufs {
   const rb_instances* in = nullptr;
   int64_t ncol = 0;        // the caller's columns (relres layout)
-  double* s2 = nullptr;    // ninst x k squared norms
+  double* s2 = nullptr;    // ninst x seg_parts x k partial squared norms
   OuterState* seg = nullptr;  // ninst x k
 };
 static size_t seg_carve(Carver& cv, SegBufs& sb, int64_t ninst, int64_t k) {
-  sb.s2 = cv.take<double>(ninst * k);
+  sb.s2 = cv.take<double>(ninst * seg_parts(ninst) * k);
   sb.seg = cv.take<OuterState>(ninst * k);
   return cv.used;
 }
@@ -2001,13 +2026,14 @@ static int solve_block(const rb_csr& A, const double* B, T64* X, int64_t ldx, in
   launches += 2;
   const bool segm = sb.in != nullptr;
   const int64_t ninst = segm ? sb.in->ninst : 0, nseg = ninst * k;
-  const unsigned sgg = (unsigned)std::min<int64_t>(std::max<int64_t>(ninst, 1), 148 * 8);
+  const int64_t snp = seg_parts(ninst);
+  const unsigned sgg = (unsigned)std::min<int64_t>(std::max<int64_t>(ninst * snp, 1), 148 * 16);
   const unsigned sgm = (unsigned)ceil_div(std::max<int64_t>(nseg, 1), 256);
   const int32_t* rinst = segm ? sb.in->row_inst : nullptr;
   const OuterState* scale_state = segm ? sb.seg : b.os;
   if (segm) {
-    seg_norm_kernel<double><<<sgg, kSegWarps * 32, 0, st>>>(ninst, k, sb.in->row_ptr, B, sb.s2);
-    seg_bnorm_kernel<<<sgm, 256, 0, st>>>(nseg, sb.s2, sb.seg);
+    seg_norm_kernel<double><<<sgg, kSegWarps * 32, 0, st>>>(ninst, snp, k, sb.in->row_ptr, B, sb.s2);
+    seg_bnorm_kernel<<<sgm, 256, 0, st>>>(nseg, snp, k, sb.s2, sb.seg);
     RB_LAUNCH_CHECK();
     launches += 2;
   }
@@ -2024,8 +2050,8 @@ static int solve_block(const rb_csr& A, const double* B, T64* X, int64_t ldx, in
     RB_CUDA_TRY(cudaMemsetAsync(b.counter + 1, 0, sizeof(int32_t), st));
     const double itol_min = sizeof(T) == sizeof(T64) ? o.inner_tol : std::min(o.inner_tol, 1e-6);
     if (segm) {
-      seg_norm_kernel<T64><<<sgg, kSegWarps * 32, 0, st>>>(ninst, k, sb.in->row_ptr, b.R64, sb.s2);
-      seg_outer_kernel<<<sgm, 256, 0, st>>>(nseg, sb.s2, sb.seg, o.tol, stall, o.inner_tol, itol_min);
+      seg_norm_kernel<T64><<<sgg, kSegWarps * 32, 0, st>>>(ninst, snp, k, sb.in->row_ptr, b.R64, sb.s2);
+      seg_outer_kernel<<<sgm, 256, 0, st>>>(nseg, snp, k, sb.s2, sb.seg, o.tol, stall, o.inner_tol, itol_min);
       seg_summary_kernel<<<(unsigned)ceil_div(k, 128), 128, 0, st>>>(ninst, k, sb.seg, b.os, b.counter + 1);
       launches += 2;
     } else {
