@@ -467,6 +467,18 @@ int rb_adjoint_fields(const void* phi, int64_t nn, int64_t ld, int64_t dcol0, co
                       const int64_t* row0, const int64_t* det0, int64_t ninst, int32_t kind, void* lam,
                       void* stream);
 
+/* The backward pass's gradients in one pass over the tets: gm[n] (nodal mua at
+ * fixed D, may be NULL) and gd[n] (nodal D, may be NULL) =
+ *   Re sum_s phi[:, s]^T (-dA/dp_n) lam[:, s],  s < ns,
+ * the column sums of rb_jac's RB_JAC_MUA_NODAL / RB_JAC_D rows of the pairs
+ * (s, lam_s) (femlhs's node-based weights, redbirdpy/forward.py:177-228).
+ * phi: row stride ldp, lam: row stride ldl, both RB_F64 or both RB_C128;
+ * work: rb_jac_grad_work_bytes(ne), 16-byte aligned. */
+size_t rb_jac_grad_work_bytes(int64_t ne);
+int rb_jac_grad(const rb_mesh* mesh, const void* phi, int64_t ldp, const void* lam, int64_t ldl, int64_t ns,
+                int32_t kind, const double* evol, const double* ddd, double* gm, double* gd, void* work,
+                size_t work_bytes, void* stream);
+
 /* ------------------------------------------------------ Gauss-Newton step
  * reginvunder (redbirdpy/recon.py:429-509) on the device:
  *   H = alpha J J^T            rb_gram: tcgen05 tensor cores, TF32 inputs,

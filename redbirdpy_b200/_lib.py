@@ -94,6 +94,9 @@ _SIGS = {
     "rb_point_rhs": (ctypes.c_int, [_vp, _vp, _vp, _i64, _i64, _i64, _i64, _vp, _vp]),
     "rb_prop_from_labels": (ctypes.c_int, [_vp, _i64, _vp, _i64, _i32, _vp, _vp, _vp]),
     "rb_adjoint_fields": (ctypes.c_int, [_vp, _i64, _i64, _i64, _vp, _i64, _vp, _vp, _i64, _i32, _vp, _vp]),
+    "rb_jac_grad_work_bytes": (_sz, [_i64]),
+    "rb_jac_grad": (ctypes.c_int, [ctypes.POINTER(RbMesh), _vp, _i64, _vp, _i64, _i64, _i32, _vp, _vp, _vp, _vp, _vp,
+                                   _sz, _vp]),
     "rb_femgetdet": (ctypes.c_int, [_vp, _vp, _vp, _i64, _vp, _i64, _i64, _i32, _vp, _vp]),
     "rb_wide_rhs": (ctypes.c_int, [_vp, _i64, _i64, _i64, _i64, _i64, _vp, _vp]),
     "rb_wide_getdet_work_bytes": (_sz, [_i64, _i64, _i32]),

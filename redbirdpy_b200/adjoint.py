@@ -15,10 +15,10 @@ convention: g = dL/dRe + i dL/dIm for complex detector values):
 (A is symmetric, complex-symmetric in the frequency domain).  lambda is the
 transposed solve of the backward, formed from the detector columns already in
 hand; ``resolve=True`` solves A lambda_s = sum_d conj(g[d, s]) b_d afresh
-instead.  The contraction is rb_jac's per-node bilinear form evaluated on the
-(source, lambda) column pairs, with the exact derivatives of the node-based
-assembly: 'mua_nodal' (mua at fixed D) and 'D' (the nodal D whose element
-mean femlhs uses, redbirdpy/forward.py:177-228).
+instead.  The contraction (rb_jac_grad, one pass over the tets) is rb_jac's
+bilinear form summed over the (source, lambda) column pairs, with the exact
+derivatives of the node-based assembly: 'mua_nodal' (mua at fixed D) and 'D'
+(the nodal D whose element mean femlhs uses, redbirdpy/forward.py:177-228).
 """
 
 import numpy as np
@@ -296,16 +296,8 @@ class _DetectorValues(torch.autograd.Function):
             engine.call("rb_adjoint_fields", engine.ptr(phi), phi.shape[0], phi.shape[1], S, engine.ptr(g), S,
                         engine.ptr(model.row0), engine.ptr(model.det0), model.ninst, kind, engine.ptr(lam),
                         engine.stream())
-        fields = torch.cat([phi[:, :S], lam], dim=1).contiguous()
-        pairs = np.column_stack([np.arange(S), S + np.arange(S), np.ones(S, dtype=np.int64)])
-        grads = []
-        for what, need in (("mua_nodal", ctx.needs_input_grad[0]), ("D", ctx.needs_input_grad[1])):
-            if not need:
-                grads.append(None)
-                continue
-            J = engine.jacobian(model.mesh, fields, pairs, what, out_dtype=torch.float64)
-            grads.append((J.real if J.is_complex() else J).sum(dim=0))
-        return grads[0], grads[1], None, None
+        gm, gd = engine.jacobian_grad(model.mesh, phi, lam, S, *ctx.needs_input_grad[:2])
+        return gm, gd, None, None
 
 
 def detector_values(model, mua, dcoef, resolve=False):

@@ -940,6 +940,23 @@ def jacobian_elem(mesh, phi, sd, evol=None):
     return Je
 
 
+def jacobian_grad(mesh, phi, lam, ns, mua=True, dcoef=True):
+    """(gm, gd): sums over the column pairs (phi[:, s], lam[:, s]), s < ns, of
+    the exact node-based rows 'mua_nodal' and 'D' (real parts), one pass over
+    the tets without forming a row (rb_jac_grad); None for one not asked."""
+    if ns > 64:
+        raise ValueError("rb_jac stages at most 128 phi columns and 64 detectors per call")
+    phi, lam = phi.contiguous(), lam.contiguous()
+    kind = _lib.RB_C128 if phi.is_complex() else _lib.RB_F64
+    gm = torch.empty(mesh.nn, dtype=torch.float64, device=phi.device) if mua else None
+    gd = torch.empty(mesh.nn, dtype=torch.float64, device=phi.device) if dcoef else None
+    wb = _lib.lib().rb_jac_grad_work_bytes(mesh.ne)
+    work = torch.empty(wb, dtype=torch.uint8, device=phi.device)
+    call("rb_jac_grad", ctypes.byref(mesh.struct), ptr(phi), phi.shape[1], ptr(lam), lam.shape[1], ns, kind,
+         ptr(mesh.evol), ptr(mesh.ddd if dcoef else None), ptr(gm), ptr(gd), ptr(work), wb, stream())
+    return gm, gd
+
+
 # ------------------------------------------------------------ Gauss-Newton
 def _pad4(n):
     return (n + 3) // 4 * 4
