@@ -1522,6 +1522,7 @@ static int64_t solve_cols(int64_t k) {
 static bool shape_covers(const Shape& s, int64_t k) { return (int64_t)s.S * s.L * s.V >= k; }
 }  // namespace rb
 #include "rb_spmm_blk.cuh"
+#include "rb_small.cuh"
 namespace rb {
 
 // D[i][c] = S[i][c] for c < ks, 0 beyond (row-major, ld ks and kd)
@@ -2136,6 +2137,38 @@ static int solve_block(const rb_csr& A, const double* B, T64* X, int64_t ldx, in
   return RB_OK;
 }
 
+// The small-system form of femsolve_t's solve: one launch, then the outcome
+template <typename T64, typename T>
+static int solve_small(const rb_csr& A, const double* B, T64* X, int64_t k, const rb_solve_opts& o,
+                       rb_solve_info& info, SmallOut* out, const T* val, const T* dinv, const SmallPlan& p,
+                       Carver& cv, cudaStream_t st) {
+  const T* sval = cv.take<T>((size_t)p.slots * p.cl);
+  const uint16_t* scol = cv.take<uint16_t>((size_t)p.slots * p.cl);
+  const int32_t* soff = cv.take<int32_t>(small_soff(p.cl, p.rpt));
+  if (!sval || !scol || !soff) return fail(RB_EARG, "rb_femsolve: workspace too small");
+  SmallArgs<T64, T> a{(int32_t)A.n, (int32_t)k, p.nr, p.cap, A.indptr, A.indices, (const T64*)A.val64, val, dinv,
+                      soff, sval, scol, p.slots, B, X, o.tol, o.inner_tol, std::min(o.inner_tol, 1e-6), 0.25, o.maxiter, o.max_outer, o.use_x0, out};
+  RB_TRY((small_launch<T64, T>(a, p, st)));
+  std::vector<SmallOut> h(k);
+  RB_CUDA_TRY(cudaMemcpyAsync(h.data(), out, sizeof(SmallOut) * k, cudaMemcpyDeviceToHost, st));
+  RB_CUDA_TRY(cudaStreamSynchronize(st));
+  double worst = 0.0;
+  int flag = 0, iters = 0;
+  for (const SmallOut& c : h) {
+    worst = std::isfinite(c.relres) ? std::max(worst, c.relres) : c.relres;
+    if (c.done == 0 || (c.done == 2 && c.relres > 1e-10)) flag = std::max(flag, 1);
+    if ((c.status == 2 && c.relres > 1e-10) || c.done == 3) flag = 2;
+    iters = std::max(iters, c.iters);
+    info.outer = std::max(info.outer, c.outer);
+    info.sweep_iters_max = std::max(info.sweep_iters_max, c.sweep_max);
+  }
+  info.iters += iters;
+  info.flag = std::max(info.flag, flag);
+  info.launches += 2;
+  info.relres = std::max(info.relres, worst);
+  return RB_OK;
+}
+
 template <typename T64, typename T>
 static int femsolve_t(const rb_csr& A, const double* B, T64* X, int64_t nrhs, const rb_solve_opts& o,
                       rb_solve_info& info, void* work, size_t work_bytes, const T* val, const T* dinv,
@@ -2147,6 +2180,18 @@ static int femsolve_t(const rb_csr& A, const double* B, T64* X, int64_t nrhs, co
   SolveBufs<T64, T> b;
   carve(cv, b, n, A.nnz, kb);
   if (!b.scan_work) return fail(RB_EARG, "rb_femsolve: workspace too small");
+  // A small system without coarse space or instances: the whole solve in one
+  // launch (rb_small.cuh) where its clusters hold the matrix.  Options that
+  // ask for the separate kernels (their timing, a fixed budget, a lane
+  // layout) keep them.
+  if constexpr (sizeof(T) != sizeof(T64)) {
+    if (!o.coarse && !o.instances && !o.profile && o.check_every > 0 && o.spmm_lanes == 0) {
+      const SmallPlan sp = small_plan<T64, T>(n, A.nnz, nrhs);
+      static_assert(sizeof(SmallOut) <= sizeof(ColState), "the outcome words share the column states' space");
+      if (sp.ok)
+        return solve_small<T64, T>(A, B, X, nrhs, o, info, reinterpret_cast<SmallOut*>(b.cs), val, dinv, sp, cv, st);
+    }
+  }
   double* Bp = nullptr;
   T64* Xp = nullptr;
   if (kb != nrhs) {
@@ -2263,6 +2308,7 @@ size_t rb_femsolve_work_bytes(int64_t n, int64_t nnz, int64_t nrhs, int32_t is_c
     else cv.take<double>(n * k);
     bytes = cv.used;
   }
+  if (precision != RB_FP64) bytes += is_complex ? small_bytes<cfloat>(n, nnz) : small_bytes<float>(n, nnz);
   return bytes + 4096;
 }
 

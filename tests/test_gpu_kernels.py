@@ -53,3 +53,72 @@ def test_tet_gradient_equals_summed_jacobian_rows(ns, cplx):
         assert (g_ - J.sum(0)).abs().max() <= 1e-13 * 16 * scale, what
     only = engine.jacobian_grad(mesh, phi, lam, ns, True, False)
     assert only[1] is None and torch.equal(only[0], got[0])
+
+
+def _system(n, cplx, seed, dense_row=False):
+    """A random sparse symmetric (complex: with a positive imaginary part),
+    diagonally dominant matrix, optionally with one full row and column."""
+    from scipy import sparse
+
+    rng = np.random.default_rng(seed)
+    i = rng.integers(0, n, 5 * n)
+    j = np.clip(i + rng.integers(-40, 41, 5 * n), 0, n - 1)
+    v = rng.uniform(-1, 0, 5 * n) * (1 + (0.2j if cplx else 0))
+    A = sparse.coo_matrix((v, (i, j)), shape=(n, n)).tocsr()
+    A = A + A.T
+    if dense_row:
+        r = sparse.coo_matrix((np.full(n, -1e-3), (np.full(n, n // 2), np.arange(n))), shape=(n, n)).tocsr()
+        A = A + r + r.T
+    d = np.asarray(abs(A).sum(1)).ravel() + rng.uniform(0.05, 0.1, n)
+    return (A + sparse.diags(d * (1 + (0.1j if cplx else 0)))).tocsr()
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("n,k,dense_row", [(1, 1, False), (5, 3, False), (33, 2, True), (2047, 5, False),
+                                           (2049, 1, False), (4097, 9, True), (8193, 37, False), (16385, 2, False),
+                                           (32767, 3, False)])
+def test_one_launch_solve_of_small_systems(n, k, dense_row, cplx):
+    """The one-launch solve at the edges of its layouts (fewer rows than
+    blocks, one row past a thread's share, a row too long for its slice, odd
+    column counts, a zero column) against SuperLU and the separate kernels.
+    Both refine to the FP64 floor of well-conditioned systems (condition
+    below 1e3): 1e-11 of the largest entry."""
+    from scipy.sparse.linalg import splu
+
+    A = _system(n, cplx, n + k, dense_row)
+    rng = np.random.default_rng(1)
+    B = rng.standard_normal((n, k))
+    if k > 1:
+        B[:, k // 2] = 0.0
+    mat = engine.DeviceMatrix.from_scipy(A)
+    Bd = torch.as_tensor(B, device="cuda")
+    X, info = engine.solve(mat, Bd)
+    assert info["flag"] == 0 and info["launches"] == 2, info
+    ref = splu(A.tocsc()).solve(B.astype(A.dtype))
+    scale = np.abs(ref).max()
+    assert np.abs(X.cpu().numpy() - ref).max() <= 1e-11 * scale
+    if k > 1:
+        assert not X[:, k // 2].any()
+    X2, info2 = engine.solve(mat, Bd, profile=True)
+    assert info2["flag"] == 0 and info2["launches"] > 2
+    assert (X - X2).abs().max() <= 1e-11 * scale
+    X3, info3 = engine.solve(mat, Bd, x0=X)  # from the solution
+    assert info3["flag"] == 0 and info3["launches"] == 2
+    assert (X3 - X).abs().max() <= 1e-11 * scale
+
+
+def test_one_launch_solve_reports_failure():
+    """A capped solve ends unconverged (flag 1), a non-finite column is
+    flagged (2) while the others still solve."""
+    A = _system(700, False, 3)
+    mat = engine.DeviceMatrix.from_scipy(A)
+    B = torch.randn((700, 4), device="cuda", dtype=torch.float64, generator=torch.Generator("cuda").manual_seed(2))
+    _, info = engine.solve(mat, B, maxiter=1, max_outer=1)
+    assert info["flag"] == 1 and info["launches"] == 2
+    good, _ = engine.solve(mat, B)
+    B2 = B.clone()
+    B2[5, 1] = float("nan")
+    X, info = engine.solve(mat, B2)
+    assert info["flag"] == 2
+    keep = [0, 2, 3]
+    assert (X[:, keep] - good[:, keep]).abs().max() <= 1e-12 * good.abs().max()
