@@ -228,9 +228,8 @@ def run_b200(args):
     # the product's own bytes: the CSR matrix (FP32 values, int32 indices) and
     # x and y once each, whatever plan the kernel walks
     spmm_bytes = nnz * (4 + 4) + 4 * (n + 1) + 2 * k * n * 4
-    # r, q read + r written (FP32), dinv and the aggregate row list read, the
-    # restricted residual (nc x k) written (x += a p is in the p-update)
-    upd_bytes = 3 * k * n * 4 + 8 * n + 4 * k * infos[-1]["coarse_nc"]
+    # r, q read + r written (FP32) (x += a p is in the p-update)
+    upd_bytes = 3 * k * n * 4
     sp_ms = sum(i["spmm_ms"] for i in pinfos) / max(1, sum(i["spmm_launches"] for i in pinfos))
     up_ms = sum(i["update_ms"] for i in pinfos) / max(1, sum(i["update_launches"] for i in pinfos))
     peak, peak_kind = peaks()
@@ -293,7 +292,9 @@ def run_b200(args):
         traffic = json.load(open(tp))
     it = infos[-1]
     spk = it.get("spmm_kernel", "spmm_pair_kernel")
-    spmm_desc = {"spmm_blk_kernel": "spmm_blk_kernel (FP32 CSR SpMM over 2x2x2 spatial row groups, one gather per "
+    spmm_desc = {"vc_spmm_kernel": "vc_spmm_kernel (FP32 SpMM of the scaled matrix over 2x2x2 spatial row groups, one gather "
+                                   "per group column, 128 RHS, fused p.Ap)",
+                 "spmm_blk_kernel": "spmm_blk_kernel (FP32 CSR SpMM over 2x2x2 spatial row groups, one gather per "
                                     "group column, 128 RHS, fused p.Ap)",
                  "spmm_pair_kernel": "spmm_pair_kernel (FP32 CSR SpMM, two rows per warp over their column union, "
                                      "128 RHS, fused p.Ap)"}[spk]
@@ -305,7 +306,7 @@ def run_b200(args):
         "data": "synthetic",
         "config": {"workload": "box 100x100x50 mm, 1 mm Kuhn (520251 nodes, 3000000 tets), 64 src + 64 det, CW",
                    "nnz": nnz, "nrhs": nrhs,
-                   "precision": "mixed (FP32 PCG in FP64 refinement; Jacobi + aggregation coarse space)",
+                   "precision": "mixed (FP32 PCG in FP64 refinement; three-level V-cycle)",
                    "l2": "working set > L2 (5 x 266 MB vectors), no flush", "parallelism": f"replicas x{world}"},
         "fp64_value": round(world * nrhs / (ms_fp64 * 1e-3), 3), "fp64_ms_per_step": round(ms_fp64, 3),
         "mixed_speedup_vs_fp64": round(ms_fp64 / ms_mixed, 3),
@@ -322,11 +323,11 @@ def run_b200(args):
                      "algorithmic_bytes": spmm_bytes, "launch_ms": round(sp_ms, 4),
                      "traffic": traffic.get(spk + "<EPI_PQDOT>"),
                      "traffic_source": "stored: an earlier ncu capture of this workload, not measured in this run"},
-        "roofline_update": {"kernel": "cg_update_agg_kernel<float> (r update + r.z, r.r, coarse restriction)",
+        "roofline_update": {"kernel": "vc_update_kernel<float> (r update + r.r)",
                             "achieved": round(up_gbs, 1) if up_gbs else None,
                             "unit": "GB/s", "frac": round(up_gbs / peak, 4) if up_gbs else None,
                             "algorithmic_bytes": upd_bytes, "launch_ms": round(up_ms, 4),
-                            "traffic": traffic.get("cg_update_agg_kernel<float,32,4>"),
+                            "traffic": traffic.get("vc_update_kernel<float,32,1>"),
                             "traffic_source": "stored (earlier ncu capture)"},
         "roofline_assembly": {"kernel": asm_kernel + " (+ dcoeff prologue)", "achieved": round(asm_gbs, 1),
                               "unit": "GB/s", "frac": round(asm_gbs / peak, 4), "algorithmic_bytes": asm_bytes,

@@ -292,6 +292,26 @@ int rb_rowgroups_union_count(const rb_csr* A, const int32_t* rows, int64_t ng, i
                              int64_t* nu /* host */, void* work, size_t work_bytes, void* stream);
 int rb_rowgroups_union_fill(const rb_csr* A, const int32_t* rows, int64_t ng, const int32_t* uptr,
                             int32_t* ucol, uint8_t* umask, void* stream);
+/* The group level of the V-cycle preconditioner (rb_femsolve_mid; no
+ * counterpart in the reference): the row groups as aggregates.  grp[i] is the
+ * group of row i, mptr / mcol (ng + 1, nnz1) each group's neighbour groups
+ * (ascending, itself included), coarse the aggregates of the groups (a
+ * rb_coarse over ng rows).  Built once per mesh: count fills grp and mptr and
+ * returns nnz1 (RB_ESIZE when a group has more than 64 neighbours: solve
+ * without this level); work: rb_rowgroups_union_work_bytes(ng).  Unlike
+ * rb_rowgroups::coef, nothing here is written by a solve. */
+typedef struct rb_midlevel {
+  const rb_rowgroups* groups; /* host pointer; its coef is not used */
+  const int32_t* grp;
+  const int32_t* mptr;
+  const int32_t* mcol;
+  int64_t nnz1;
+  const rb_coarse* coarse;    /* host pointer */
+} rb_midlevel;
+int rb_midlevel_count(const rb_rowgroups* groups, int64_t n, int32_t* grp, int32_t* mptr, int64_t* nnz1 /* host */,
+                      void* work, size_t work_bytes, void* stream);
+int rb_midlevel_fill(const rb_rowgroups* groups, const int32_t* grp, const int32_t* mptr, int32_t* mcol,
+                     void* stream);
 /* Independent systems stacked block-diagonally in one matrix (a batch of
  * instances): rows row_ptr[i] .. row_ptr[i+1]-1 belong to instance i.  With
  * it the refinement tests ||b_i - A_i x_i|| / ||b_i|| of every (instance,
@@ -361,6 +381,12 @@ size_t rb_femsolve_work_bytes(int64_t n, int64_t nnz, int64_t nrhs, int32_t is_c
 int rb_femsolve(const rb_csr* A, const double* B, void* X, int64_t nrhs,
                 const rb_solve_opts* opts, rb_solve_info* info /* host */, void* work,
                 size_t work_bytes, void* stream);
+/* rb_femsolve (mixed precision) with the three-level V-cycle preconditioner:
+ * opts->coarse, groups and instances must be NULL, check_every >= 1, and
+ * n x (nrhs rounded up to 4) < 2^31.  work: rb_femsolve_mid_work_bytes. */
+size_t rb_femsolve_mid_work_bytes(const rb_csr* A, const rb_midlevel* mid, int64_t nrhs);
+int rb_femsolve_mid(const rb_csr* A, const rb_midlevel* mid, const double* B, void* X, int64_t nrhs,
+                    const rb_solve_opts* opts, rb_solve_info* info, void* work, size_t work_bytes, void* stream);
 
 /* FP32 (complex64) copy of the values and the reciprocal diagonal of a CSR
  * matrix given in FP64 (for matrices that did not come from rb_femlhs).

@@ -52,6 +52,11 @@ class RbRowGroups(ctypes.Structure):
                 ("coef", _vp)]
 
 
+class RbMidlevel(ctypes.Structure):
+    _fields_ = [("groups", ctypes.POINTER(RbRowGroups)), ("grp", _vp), ("mptr", _vp), ("mcol", _vp), ("nnz1", _i64),
+                ("coarse", ctypes.POINTER(RbCoarse))]
+
+
 class RbInstances(ctypes.Structure):
     _fields_ = [("ninst", _i64), ("row_ptr", _vp), ("row_inst", _vp), ("status", _vp), ("relres", _vp)]
 
@@ -113,6 +118,12 @@ _SIGS = {
     "rb_rowgroups_union_count": (ctypes.c_int, [ctypes.POINTER(RbCsr), _vp, _i64, _vp, ctypes.POINTER(_i64), _vp,
                                                 _sz, _vp]),
     "rb_rowgroups_union_fill": (ctypes.c_int, [ctypes.POINTER(RbCsr), _vp, _i64, _vp, _vp, _vp, _vp]),
+    "rb_midlevel_count": (ctypes.c_int, [ctypes.POINTER(RbRowGroups), _i64, _vp, _vp, ctypes.POINTER(_i64), _vp, _sz,
+                                         _vp]),
+    "rb_midlevel_fill": (ctypes.c_int, [ctypes.POINTER(RbRowGroups), _vp, _vp, _vp, _vp]),
+    "rb_femsolve_mid_work_bytes": (_sz, [ctypes.POINTER(RbCsr), ctypes.POINTER(RbMidlevel), _i64]),
+    "rb_femsolve_mid": (ctypes.c_int, [ctypes.POINTER(RbCsr), ctypes.POINTER(RbMidlevel), _vp, _vp, _i64,
+                                       ctypes.POINTER(RbSolveOpts), ctypes.POINTER(RbSolveInfo), _vp, _sz, _vp]),
     "rb_femsolve": (ctypes.c_int, [ctypes.POINTER(RbCsr), _vp, _vp, _i64, ctypes.POINTER(RbSolveOpts),
                                    ctypes.POINTER(RbSolveInfo), _vp, _sz, _vp]),
     "rb_csr_prepare": (ctypes.c_int, [ctypes.POINTER(RbCsr), _vp, _vp, _vp, _vp]),

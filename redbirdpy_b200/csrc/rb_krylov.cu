@@ -1991,11 +1991,44 @@ static int inner_solve(const rb_csr& A, const T* val, const T* dinv, int64_t k, 
   return RB_OK;
 }
 
+// FP32 copy of the values and reciprocal diagonal of a CSR matrix
+template <typename T64, typename T32>
+__global__ void csr_prepare_kernel(int64_t n, const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices,
+                                   const T64* __restrict__ v64, T32* __restrict__ v32, T64* __restrict__ d64,
+                                   T32* __restrict__ d32) {
+  for (int64_t row = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; row < n; row += (int64_t)gridDim.x * blockDim.x) {
+    T64 dg = s_zero(T64());
+    for (int32_t p = indptr[row]; p < indptr[row + 1]; ++p) {
+      const T64 v = v64[p];
+      if (v32) {
+        if constexpr (Scalar<T64>::is_complex) v32[p] = T32{(float)v.x, (float)v.y};
+        else v32[p] = (T32)v;
+      }
+      if (indices[p] == row) dg = s_add(dg, v);
+    }
+    T64 r;
+    if constexpr (Scalar<T64>::is_complex) {
+      const double d = dg.x * dg.x + dg.y * dg.y;
+      r = make_double2(dg.x / d, -dg.y / d);
+    } else {
+      r = 1.0 / dg;
+    }
+    if (d64) d64[row] = r;
+    if (d32) {
+      if constexpr (Scalar<T64>::is_complex) d32[row] = T32{(float)r.x, (float)r.y};
+      else d32[row] = (T32)r;
+    }
+  }
+}
+}  // namespace rb
+#include "rb_vcycle.cuh"
+namespace rb {
+
 template <typename T64, typename T>
 static int solve_block(const rb_csr& A, const double* B, T64* X, int64_t ldx, int64_t k, const rb_solve_opts& o,
                        rb_solve_info& info, SolveBufs<T64, T>& b, const T* val, const T* dinv,
                        const GroupPlan* gp, const RowGroupsDev* rg, const CoarseOp<T>* co, const SegBufs& sb,
-                       cudaStream_t st) {
+                       const VcBufs<T64, T>* vc, cudaStream_t st) {
   const int64_t n = A.n;
   const Shape sh = pick_shape(n, k, Bps<T>::value);      // inner (FP32 or FP64) vector kernels
   Shape shs = pick_spmm_shape<T>(n, k);                  // inner SpMM
@@ -2042,12 +2075,14 @@ static int solve_block(const rb_csr& A, const double* B, T64* X, int64_t ldx, in
   const bool budget = o.check_every == 0;
   KernelTimer tm;
   tm.on = o.profile != 0 && !budget;
-  tm.with_coarse = o.coarse != nullptr;
+  tm.with_coarse = o.coarse != nullptr || vc != nullptr;
   int total_iters = 0, outer = 0;
   int sweep_flag = 0;
   for (outer = 0; outer <= o.max_outer; ++outer) {
-    // R64 = B - A X (FP64)
-    RB_TRY((spmm_t<T64, EPI_RESID>(A, (const T64*)A.val64, X, b.R64, B, b.part_b, k, sh64, st)));
+    // R64 = B - A X (FP64); a cycle solve from X = 0 starts from B itself
+    // (part_b still holds the partials of ||b||^2)
+    const bool from_b = vc != nullptr && outer == 0 && !o.use_x0;
+    if (!from_b) RB_TRY((spmm_t<T64, EPI_RESID>(A, (const T64*)A.val64, X, b.R64, B, b.part_b, k, sh64, st)));
     RB_CUDA_TRY(cudaMemsetAsync(b.counter + 1, 0, sizeof(int32_t), st));
     const double itol_min = sizeof(T) == sizeof(T64) ? o.inner_tol : std::min(o.inner_tol, 1e-6);
     if (segm) {
@@ -2070,6 +2105,23 @@ static int solve_block(const rb_csr& A, const double* B, T64* X, int64_t ldx, in
       RB_CUDA_TRY(cudaMemcpyAsync(&nact, b.counter + 1, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
       RB_CUDA_TRY(cudaStreamSynchronize(st));
       if (nact == 0 || outer == o.max_outer) break;
+    }
+    if constexpr (sizeof(T) != sizeof(T64)) {
+      if (vc) {
+        if (from_b) vc_cast_kernel<T64, double, T><<<eg, 256, 0, st>>>(n, k, B, vc->s64, b.os, b.R, b.P, b.Xs);
+        else vc_cast_kernel<T64, T64, T><<<eg, 256, 0, st>>>(n, k, b.R64, vc->s64, b.os, b.R, b.P, b.Xs);
+        RB_LAUNCH_CHECK();
+        int it = 0;
+        RB_TRY((vc_inner<T64, T>(A, vc->op, k, b.part_a, b.part_b, b.Xs, b.R, b.P, b.Q, b.cs, b.os, b.counter,
+                                 o.inner_tol, o.maxiter, gp, &it, &launches, tm, st)));
+        total_iters += it;
+        info.sweep_iters_max = std::max(info.sweep_iters_max, it);
+        if (it >= o.maxiter) sweep_flag = 1;
+        vc_correct_kernel<T64, T><<<eg, 256, 0, st>>>(n, k, b.Xs, vc->s64, b.os, X);
+        RB_LAUNCH_CHECK();
+        launches += 2;
+        continue;
+      }
     }
     cast_scale_kernel<T64, T><<<eg, 256, 0, st>>>(n, k, b.R64, scale_state, rinst, b.R);
     RB_LAUNCH_CHECK();
@@ -2172,10 +2224,10 @@ static int solve_small(const rb_csr& A, const double* B, T64* X, int64_t k, cons
 template <typename T64, typename T>
 static int femsolve_t(const rb_csr& A, const double* B, T64* X, int64_t nrhs, const rb_solve_opts& o,
                       rb_solve_info& info, void* work, size_t work_bytes, const T* val, const T* dinv,
-                      cudaStream_t st) {
+                      cudaStream_t st, const rb_midlevel* mid = nullptr) {
   const int64_t n = A.n;
   if (nrhs > kMaxCols) return fail(RB_ESIZE, "rb_femsolve: more than %lld right-hand sides per call", (long long)kMaxCols);
-  const int64_t kb = solve_cols(nrhs);  // columns of the solve (padded when the layout needs it)
+  const int64_t kb = mid ? vc_cols(nrhs) : solve_cols(nrhs);  // columns of the solve (padded when the layout needs it)
   Carver cv{reinterpret_cast<char*>(work), work_bytes};
   SolveBufs<T64, T> b;
   carve(cv, b, n, A.nnz, kb);
@@ -2185,7 +2237,7 @@ static int femsolve_t(const rb_csr& A, const double* B, T64* X, int64_t nrhs, co
   // ask for the separate kernels (their timing, a fixed budget, a lane
   // layout) keep them.
   if constexpr (sizeof(T) != sizeof(T64)) {
-    if (!o.coarse && !o.instances && !o.profile && o.check_every > 0 && o.spmm_lanes == 0) {
+    if (!mid && !o.coarse && !o.instances && !o.profile && o.check_every > 0 && o.spmm_lanes == 0) {
       const SmallPlan sp = small_plan<T64, T>(n, A.nnz, nrhs);
       static_assert(sizeof(SmallOut) <= sizeof(ColState), "the outcome words share the column states' space");
       if (sp.ok)
@@ -2220,6 +2272,27 @@ static int femsolve_t(const rb_csr& A, const double* B, T64* X, int64_t nrhs, co
     RB_TRY((coarse_setup<T64, T>(A, cb, st)));
     info.launches += 3 + 5 * (int)ceil_div(cb.op.nc, kGjB);
   }
+  // the three-level cycle: its arrays, then the matrix-dependent setup
+  VcBufs<T64, T> vb;
+  if constexpr (sizeof(T) != sizeof(T64)) {
+    if (mid) {
+      const rb_rowgroups& g = *mid->groups;
+      vc_carve(cv, vb, n, A.nnz, g.ng, g.nu, mid->nnz1, mid->coarse->nc, kb);
+      if (!vb.cb.err) return fail(RB_EARG, "rb_femsolve_mid: workspace too small");
+      vb.op.rg.ng = g.ng;
+      vb.op.rg.rows = g.rows;
+      vb.op.rg.uptr = g.uptr;
+      vb.op.rg.ucol = g.ucol;
+      vb.op.rg.umask = g.umask;
+      vb.op.mptr = mid->mptr;
+      vb.op.mcol = mid->mcol;
+      vb.cb.op.agg = mid->coarse->agg;
+      vb.cb.op.agg_ptr = mid->coarse->agg_ptr;
+      vb.cb.op.agg_rows = mid->coarse->agg_rows;
+      RB_TRY((vc_setup<T64, T>(A, *mid, vb, st)));
+      info.launches += 12 + 5 * (int)ceil_div(vb.cb.op.nc, kGjB);
+    }
+  }
   GroupPlan gp{nullptr, nullptr, nullptr, 0};
   // spatial row groups (blocked SpMM) when the caller built them for this
   // pattern and the column count fits; else the row-pair / row-group plans
@@ -2232,7 +2305,9 @@ static int femsolve_t(const rb_csr& A, const double* B, T64* X, int64_t nrhs, co
     RB_TRY(rg_fill_coef<T>(A, val, rgd, st));
     info.launches += 1;
   }
-  const bool plan = !use_rg && ((GrpCfg<T>::enabled && grp_cols_ok(kb)) ||
+  // a complex cycle's p.Ap product walks row pairs where their layout fits
+  // (faster than its row groups: complex64 groups hold 64 columns per warp)
+  const bool plan = !use_rg && (!mid || Scalar<T>::is_complex) && ((GrpCfg<T>::enabled && grp_cols_ok(kb)) ||
                                 (PairCfg<T>::enabled && pair_cols_ok<T>(kb) && n * kb < (int64_t(1) << 31)));
   if (plan && n > 0)
     RB_TRY(build_group_plan<GrpCfg<T>::G>(A, b.gcnt, b.gptr, b.ucol, b.umask, b.scan_work, b.scan_bytes, &gp, st));
@@ -2246,43 +2321,13 @@ static int femsolve_t(const rb_csr& A, const double* B, T64* X, int64_t nrhs, co
     }
   }
   RB_TRY((solve_block<T64, T>(A, Bp ? Bp : B, Xp ? Xp : X, kb, kb, o, info, b, val, dinv, gp.ng ? &gp : nullptr,
-                              use_rg ? &rgd : nullptr, o.coarse ? &cb.op : nullptr, sb, st)));
+                              use_rg ? &rgd : nullptr, o.coarse ? &cb.op : nullptr, sb, mid ? &vb : nullptr, st)));
   if (Xp) {
     copy_cols_kernel<T64><<<eg, 256, 0, st>>>(n, kb, nrhs, Xp, X);
     RB_LAUNCH_CHECK();
     info.launches += o.use_x0 ? 3 : 2;
   }
   return RB_OK;
-}
-
-// FP32 copy of the values and reciprocal diagonal of a CSR matrix
-template <typename T64, typename T32>
-__global__ void csr_prepare_kernel(int64_t n, const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices,
-                                   const T64* __restrict__ v64, T32* __restrict__ v32, T64* __restrict__ d64,
-                                   T32* __restrict__ d32) {
-  for (int64_t row = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; row < n; row += (int64_t)gridDim.x * blockDim.x) {
-    T64 dg = s_zero(T64());
-    for (int32_t p = indptr[row]; p < indptr[row + 1]; ++p) {
-      const T64 v = v64[p];
-      if (v32) {
-        if constexpr (Scalar<T64>::is_complex) v32[p] = T32{(float)v.x, (float)v.y};
-        else v32[p] = (T32)v;
-      }
-      if (indices[p] == row) dg = s_add(dg, v);
-    }
-    T64 r;
-    if constexpr (Scalar<T64>::is_complex) {
-      const double d = dg.x * dg.x + dg.y * dg.y;
-      r = make_double2(dg.x / d, -dg.y / d);
-    } else {
-      r = 1.0 / dg;
-    }
-    if (d64) d64[row] = r;
-    if (d32) {
-      if constexpr (Scalar<T64>::is_complex) d32[row] = T32{(float)r.x, (float)r.y};
-      else d32[row] = (T32)r;
-    }
-  }
 }
 
 }  // namespace rb
@@ -2376,6 +2421,58 @@ int rb_femsolve(const rb_csr* A, const double* B, void* X, int64_t nrhs, const r
                                       (const double*)A->val64, (const double*)A->dinv64, st);
   return femsolve_t<double, float>(*A, B, (double*)X, nrhs, o, *info, work, work_bytes,
                                    (const float*)A->val32, (const float*)A->dinv32, st);
+}
+
+size_t rb_femsolve_mid_work_bytes(const rb_csr* A, const rb_midlevel* mid, int64_t nrhs) {
+  if (!A || !mid || !mid->groups || !mid->coarse) return 0;
+  const int64_t k0 = std::min<int64_t>(std::max<int64_t>(nrhs, 1), kMaxCols), k = vc_cols(k0);
+  const rb_rowgroups& g = *mid->groups;
+  Carver cv{nullptr, 0};
+  auto count = [&](auto& b, auto& v, auto zero) {
+    carve(cv, b, A->n, A->nnz, k);
+    if (k != k0) {
+      cv.take<double>(A->n * k);
+      cv.take<decltype(zero)>(A->n * k);
+    }
+    vc_carve(cv, v, A->n, A->nnz, g.ng, g.nu, mid->nnz1, mid->coarse->nc, k);
+  };
+  if (A->is_complex) {
+    SolveBufs<cdouble, cfloat> b;
+    VcBufs<cdouble, cfloat> v;
+    count(b, v, cdouble{});
+  } else {
+    SolveBufs<double, float> b;
+    VcBufs<double, float> v;
+    count(b, v, 0.0);
+  }
+  return cv.used + 4096;
+}
+
+int rb_femsolve_mid(const rb_csr* A, const rb_midlevel* mid, const double* B, void* X, int64_t nrhs,
+                    const rb_solve_opts* opts, rb_solve_info* info, void* work, size_t work_bytes, void* stream) {
+  if (!A || !mid || !B || !X || !opts || !info || !work) return fail(RB_EARG, "rb_femsolve_mid: null argument");
+  if (nrhs < 1 || A->n < 1) return fail(RB_EARG, "rb_femsolve_mid: empty system");
+  if (nrhs > kMaxCols) return fail(RB_ESIZE, "rb_femsolve_mid: at most %lld right-hand sides per call", (long long)kMaxCols);
+  const rb_solve_opts& o = *opts;
+  if (o.precision != RB_MIXED || o.coarse || o.groups || o.instances || o.check_every < 1 || o.maxiter < 1 ||
+      o.max_outer < 1 || !(o.tol > 0) || !(o.inner_tol > 0))
+    return fail(RB_EARG, "rb_femsolve_mid: bad options");
+  if (!A->val64 || !A->dinv64 || !A->val32 || !A->dinv32 || !A->indptr || !A->indices)
+    return fail(RB_EARG, "rb_femsolve_mid: matrix arrays missing");
+  const rb_rowgroups* g = mid->groups;
+  const rb_coarse* c = mid->coarse;
+  if (!g || g->ng < 1 || !g->rows || !g->uptr || !g->ucol || !g->umask || !mid->grp || !mid->mptr || !mid->mcol ||
+      mid->nnz1 < 1 || !c || c->nc < 1 || c->nc > kCoarseMax || c->nc > g->ng || !c->agg || !c->agg_ptr || !c->agg_rows)
+    return fail(RB_EARG, "rb_femsolve_mid: incomplete level");
+  if (A->n * vc_cols(nrhs) >= (int64_t(1) << 31)) return fail(RB_ESIZE, "rb_femsolve_mid: n x columns above 2^31");
+  if (work_bytes < rb_femsolve_mid_work_bytes(A, mid, nrhs)) return fail(RB_EARG, "rb_femsolve_mid: workspace too small");
+  *info = rb_solve_info{};
+  cudaStream_t st = as_stream(stream);
+  if (A->is_complex)
+    return femsolve_t<cdouble, cfloat>(*A, B, (cdouble*)X, nrhs, o, *info, work, work_bytes, (const cfloat*)A->val32,
+                                       (const cfloat*)A->dinv32, st, mid);
+  return femsolve_t<double, float>(*A, B, (double*)X, nrhs, o, *info, work, work_bytes, (const float*)A->val32,
+                                   (const float*)A->dinv32, st, mid);
 }
 
 int rb_spmm(const rb_csr* A, int32_t kind, const void* X, void* Y, int64_t nrhs, void* stream) {

@@ -104,6 +104,44 @@ __global__ void rg_union_kernel(int64_t ng, const int32_t* __restrict__ rows, co
   }
 }
 
+// ------------------------------------------- group-level pattern (V-cycle)
+__global__ void mid_group_of_kernel(int64_t ng, const int32_t* __restrict__ rows, int32_t* __restrict__ grp) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < ng * kRGRows;
+       i += (int64_t)gridDim.x * blockDim.x)
+    if (rows[i] >= 0) grp[rows[i]] = (int32_t)(i / kRGRows);
+}
+
+// the groups that hold a column of group g's union (count, or the ascending
+// list); a group with more than kMidNeighbours of them sets *over
+constexpr int kMidNeighbours = 64;
+template <bool FILL>
+__global__ void mid_pattern_kernel(int64_t ng, const int32_t* __restrict__ uptr, const int32_t* __restrict__ ucol,
+                                   const int32_t* __restrict__ grp, int32_t* __restrict__ cnt_or_ptr,
+                                   int32_t* __restrict__ mcol, int32_t* __restrict__ over) {
+  for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < ng; g += (int64_t)gridDim.x * blockDim.x) {
+    int32_t list[kMidNeighbours];
+    int n = 0;
+    for (int32_t u = uptr[g]; u < uptr[g + 1]; ++u) {
+      const int32_t h = grp[ucol[u]];
+      int j = n;  // insertion into the ascending list
+      while (j > 0 && list[j - 1] > h) --j;
+      if (j > 0 && list[j - 1] == h) continue;
+      if (n == kMidNeighbours) {
+        if (!FILL) *over = 1;
+        break;
+      }
+      for (int q = n; q > j; --q) list[q] = list[q - 1];
+      list[j] = h;
+      ++n;
+    }
+    if (FILL) {
+      for (int j = 0; j < n; ++j) mcol[cnt_or_ptr[g] + j] = list[j];
+    } else {
+      cnt_or_ptr[g] = n;
+    }
+  }
+}
+
 struct RgWork {
   int32_t *key, *cnt, *gcnt, *start, *gofs, *fill, *tmp;
   char* scan;
@@ -211,6 +249,41 @@ int rb_rowgroups_union_fill(const rb_csr* A, const int32_t* rows, int64_t ng, co
   const unsigned grid = (unsigned)std::min<int64_t>(ceil_div(ng, 128), 148 * 32);
   rg_union_kernel<true><<<grid, 128, 0, st>>>(ng, rows, A->indptr, A->indices, const_cast<int32_t*>(uptr), ucol,
                                               umask);
+  RB_LAUNCH_CHECK();
+  return RB_OK;
+}
+
+int rb_midlevel_count(const rb_rowgroups* rg, int64_t n, int32_t* grp, int32_t* mptr, int64_t* nnz1_out, void* work,
+                      size_t work_bytes, void* stream) {
+  if (!rg || rg->ng < 1 || !rg->rows || !rg->uptr || !rg->ucol || !grp || !mptr || !nnz1_out || !work || n < 1)
+    return fail(RB_EARG, "rb_midlevel_count: bad arguments");
+  const int64_t ng = rg->ng;
+  if (work_bytes < rb_rowgroups_union_work_bytes(ng)) return fail(RB_EARG, "rb_midlevel_count: workspace too small");
+  cudaStream_t st = as_stream(stream);
+  int32_t* cnt = reinterpret_cast<int32_t*>(work);  // ng counts, then the overflow word
+  char* scan = reinterpret_cast<char*>(work) + ((size_t)(ng + 1) * 4 + 255) / 256 * 256;
+  const unsigned grid = (unsigned)std::min<int64_t>(ceil_div(ng, 128), 148 * 32);
+  RB_CUDA_TRY(cudaMemsetAsync(cnt + ng, 0, 4, st));
+  mid_group_of_kernel<<<(unsigned)std::min<int64_t>(ceil_div(ng * kRGRows, 256), 148 * 16), 256, 0, st>>>(ng, rg->rows,
+                                                                                                       grp);
+  mid_pattern_kernel<false><<<grid, 128, 0, st>>>(ng, rg->uptr, rg->ucol, grp, cnt, nullptr, cnt + ng);
+  RB_LAUNCH_CHECK();
+  RB_TRY(scan_exclusive(cnt, mptr, ng, scan, scan_work_bytes(ng), st));
+  int32_t h[2] = {0, 0};
+  RB_CUDA_TRY(cudaMemcpyAsync(h, mptr + ng, 4, cudaMemcpyDeviceToHost, st));
+  RB_CUDA_TRY(cudaMemcpyAsync(h + 1, cnt + ng, 4, cudaMemcpyDeviceToHost, st));
+  RB_CUDA_TRY(cudaStreamSynchronize(st));
+  if (h[1]) return fail(RB_ESIZE, "rb_midlevel_count: a group has more than %d neighbours", kMidNeighbours);
+  *nnz1_out = h[0];
+  return RB_OK;
+}
+
+int rb_midlevel_fill(const rb_rowgroups* rg, const int32_t* grp, const int32_t* mptr, int32_t* mcol, void* stream) {
+  if (!rg || rg->ng < 1 || !rg->uptr || !rg->ucol || !grp || !mptr || !mcol)
+    return fail(RB_EARG, "rb_midlevel_fill: bad arguments");
+  const unsigned grid = (unsigned)std::min<int64_t>(ceil_div(rg->ng, 128), 148 * 32);
+  mid_pattern_kernel<true><<<grid, 128, 0, as_stream(stream)>>>(rg->ng, rg->uptr, rg->ucol, grp,
+                                                                const_cast<int32_t*>(mptr), mcol, nullptr);
   RB_LAUNCH_CHECK();
   return RB_OK;
 }

@@ -49,6 +49,7 @@ class DeviceMesh:
             self.bbox = (np.nanmin(node[:, :3], axis=0), np.nanmax(node[:, :3], axis=0)) if self.nn else None
         self._coarse = {}
         self._groups = None
+        self._mid = False  # not built yet
         self._edge = None
         if self.ne:
             sel = np.arange(0, self.ne, max(1, self.ne // 65536))
@@ -159,6 +160,19 @@ class DeviceMesh:
                 return None
             self._groups = RowGroups(self, self._edge)
         return self._groups
+
+    def mid_level(self):
+        """The MidLevel of the V-cycle preconditioner (built once), or None
+        when the mesh has no row groups or a group has too many neighbours."""
+        if self._mid is False:
+            rg = self.row_groups()
+            try:
+                self._mid = None if rg is None else MidLevel(self, rg)
+            except _lib.RedbirdError as e:
+                if e.code != _lib.RB_ESIZE:
+                    raise
+                self._mid = None
+        return self._mid
 
     def deldotdel_host(self):
         return self.ddd.cpu().numpy()
@@ -619,6 +633,60 @@ class RowGroups:
                                        self.umask.data_ptr(), self.nu, self.coef.data_ptr())
 
 
+def mid_coarse_target(ng):
+    """Default aggregate count of the V-cycle's dense level for ng groups:
+    ng / 32 within [64, 1024], never above ng / 8.  Measured (solve, ms; the
+    setup grows with the count, the iterations fall): 520k nodes x 128 (67,626
+    groups) 256 aggregates 64.4, 726 56.5, 1183 53.8, 2048 53.5; complex 726
+    124.0, 1183 112.5, 2048 123.3; 67,626 nodes x 64 (8,788 groups) 256 6.0,
+    605 6.6, 1183 7.5; 43,218 x 37 (5,775 groups) 126 4.9, 288 4.9, 600 5.5."""
+    return int(max(1, min(max(64, min(1024, ng // 32)), ng // 8)))
+
+
+class _GroupNodes:
+    """What CoarseSpace needs of a mesh, over the row groups: one position
+    per group (its first node's)."""
+
+    def __init__(self, mesh, rg):
+        self.device, self.bbox, self.nn = mesh.device, mesh.bbox, rg.ng
+        self.node = mesh.node[rg.rows[: 8 * rg.ng].view(rg.ng, 8)[:, 0].long()].contiguous()
+
+
+class MidLevel:
+    """The group level of the V-cycle preconditioner (``rb_midlevel``): the
+    row groups as aggregates of the nodes, their neighbour pattern, and the
+    dense level's aggregates of the groups.  Built once per mesh."""
+
+    def __init__(self, mesh, rg):
+        dev = mesh.device
+        self.groups = rg
+        self.grp = torch.empty(mesh.nn, dtype=torch.int32, device=dev)
+        self.mptr = torch.empty(rg.ng + 1, dtype=torch.int32, device=dev)
+        wb = _lib.lib().rb_rowgroups_union_work_bytes(rg.ng)
+        work = torch.empty(wb, dtype=torch.uint8, device=dev)
+        nnz1 = ctypes.c_int64(0)
+        call("rb_midlevel_count", ctypes.byref(rg.struct), mesh.nn, ptr(self.grp), ptr(self.mptr),
+             ctypes.byref(nnz1), ptr(work), wb, stream())
+        self.nnz1 = int(nnz1.value)
+        self.mcol = torch.empty(max(self.nnz1, 1), dtype=torch.int32, device=dev)
+        call("rb_midlevel_fill", ctypes.byref(rg.struct), ptr(self.grp), ptr(self.mptr), ptr(self.mcol), stream())
+        self.coarse = CoarseSpace(_GroupNodes(mesh, rg), mid_coarse_target(rg.ng))
+        self.struct = _lib.RbMidlevel(ctypes.pointer(rg.struct), self.grp.data_ptr(), self.mptr.data_ptr(),
+                                      self.mcol.data_ptr(), self.nnz1, ctypes.pointer(self.coarse.struct))
+
+
+def _resolve_mid(mat, n, k, prec, coarse, groups, instances, budget):
+    """The MidLevel a solve takes, or None: with every choice left to the
+    engine ('auto'), a mixed-precision solve of one system assembled on a
+    mesh of at least COARSE_MIN_NODES nodes."""
+    if coarse != "auto" or groups != "auto" or prec != _lib.RB_MIXED or instances is not None or budget is not None:
+        return None
+    mesh = getattr(mat, "mesh", None)
+    if not hasattr(mesh, "mid_level") or n < COARSE_MIN_NODES or n * (min(k, 128) + 4) >= 2 ** 31:
+        return None
+    return mesh.mid_level()
+
+
 def _resolve_groups(mat, groups):
     """RowGroups for solve(groups=...): 'auto' (real matrices assembled on a
     DeviceMesh), a RowGroups, or None/False for the per-row SpMM kernels."""
@@ -734,6 +802,18 @@ class SolveTuner:
 solve_tuner = SolveTuner()
 
 
+def _add_info(info, inf):
+    """One library call's RbSolveInfo into solve's info dict."""
+    info["iters"] += inf.iters
+    info["outer"] = max(info["outer"], inf.outer)
+    info["flag"] = max(info["flag"], inf.flag) if info["flag"] is not None else None
+    info["launches"] += inf.launches
+    info["sweep_iters_max"] = max(info.get("sweep_iters_max", 0), inf.sweep_iters_max)
+    info["relres"] = max(info["relres"], inf.relres)
+    for key in ("spmm_ms", "update_ms", "spmm_launches", "update_launches", "coarse_ms", "coarse_launches"):
+        info[key] += getattr(inf, key)
+
+
 def solve(mat, B, precision="mixed", tol=DEFAULT_TOL, inner_tol=None, maxiter=2000, max_outer=10,
           check_every=10, profile=False, x0=None, coarse="auto", groups="auto", instances=None, budget=None,
           spmm_lanes=0):
@@ -744,8 +824,11 @@ def solve(mat, B, precision="mixed", tol=DEFAULT_TOL, inner_tol=None, maxiter=20
     entirely in FP64.  Up to 128 columns per library call; wider B is solved
     in column blocks.  ``x0`` (nn x k, the solution's dtype) is an initial
     guess: the refinement starts from its FP64 residual instead of from zero.
-    ``coarse`` adds the aggregation coarse space to the Jacobi preconditioner
-    (see _resolve_coarse; 'auto' uses it on meshes of 20000 nodes or more).
+    With ``coarse`` and ``groups`` left at 'auto', a mixed-precision solve on a
+    mesh of 20000 nodes or more takes the three-level V-cycle preconditioner
+    (MidLevel; a solve that it does not bring to convergence is redone with
+    the two-level form).  ``coarse`` otherwise adds the aggregation coarse
+    space to the Jacobi preconditioner (see _resolve_coarse).
     ``inner_tol`` (relative residual of each FP32 correction sweep) defaults to
     1e-5 with a coarse space and 1e-4 without: on the 520k-node box at 128
     columns, 1e-5 took 3 sweeps / 130 iterations / 113.5 ms against 4 / 150 /
@@ -777,12 +860,13 @@ def solve(mat, B, precision="mixed", tol=DEFAULT_TOL, inner_tol=None, maxiter=20
         coarse = False
         if instances is None:
             instances = Instances([0, n], B.device)
-    cs = _resolve_coarse(mat, coarse)
+    mid = _resolve_mid(mat, n, k, prec, coarse, groups, instances, budget) if k else None
+    cs = _resolve_coarse(mat, coarse) if mid is None else None
     if inner_tol is None:
-        inner_tol = 1e-5 if cs is not None else 1e-4
+        inner_tol = 1e-5 if cs is not None or mid is not None else 1e-4
     if prec == _lib.RB_FP64 and inner_tol > 1e-6:
         inner_tol = max(tol, 1e-15)
-    rg = _resolve_groups(mat, groups) if prec == _lib.RB_MIXED else None
+    rg = _resolve_groups(mat, groups) if prec == _lib.RB_MIXED and mid is None else None
     if instances is not None and instances.n != n:
         raise ValueError("instances do not cover the matrix's rows")
     opts = _lib.RbSolveOpts(prec, int(max_outer), int(maxiter), int(check_every), float(tol), float(inner_tol),
@@ -801,25 +885,42 @@ def solve(mat, B, precision="mixed", tol=DEFAULT_TOL, inner_tol=None, maxiter=20
             Xb = X[:, c0:c0 + kb].contiguous() if x0 is not None else torch.empty((n, kb), dtype=xdt, device=B.device)
         else:
             Xb = X
+        inf = _lib.RbSolveInfo()
+        if mid is not None:
+            wb = _lib.lib().rb_femsolve_mid_work_bytes(ctypes.byref(mat.struct), ctypes.byref(mid.struct), kb)
+            try:
+                work = torch.empty(wb, dtype=torch.uint8, device=B.device)
+            except torch.cuda.OutOfMemoryError:
+                work = None  # the two-level form needs a fifth less
+            if work is not None:
+                call("rb_femsolve_mid", ctypes.byref(mat.struct), ctypes.byref(mid.struct), ptr(Bb), ptr(Xb), kb,
+                     ctypes.byref(opts), ctypes.byref(inf), ptr(work), wb, stream())
+            if work is None or inf.flag != 0:
+                # the cycle assumes a definite operator (positive diagonal,
+                # real part); what it does not solve gets the two-level form
+                work = None
+                cs, rg = _resolve_coarse(mat, coarse), _resolve_groups(mat, groups)
+                opts.coarse = ctypes.pointer(cs.struct) if cs is not None else None
+                opts.groups = ctypes.pointer(rg.struct) if rg is not None else None
+                mid = None
+                if x0 is not None:
+                    Xb.copy_(x0[:, c0:c0 + kb])
+        if mid is not None:
+            if Xb is not X:
+                X[:, c0:c0 + kb] = Xb
+            _add_info(info, inf)
+            continue
         wb = _lib.lib().rb_femsolve_work_bytes(n, mat.struct.nnz, kb, int(mat.is_complex), prec)
         if cs is not None:
             wb += _lib.lib().rb_coarse_work_bytes(cs.nc, kb, int(mat.is_complex), prec)
         if instances is not None:
             wb += _lib.lib().rb_instances_work_bytes(instances.ninst, kb)
         work = torch.empty(wb, dtype=torch.uint8, device=B.device)
-        inf = _lib.RbSolveInfo()
         call("rb_femsolve", ctypes.byref(mat.struct), ptr(Bb), ptr(Xb), kb, ctypes.byref(opts), ctypes.byref(inf),
              ptr(work), wb, stream())
         if Xb is not X:
             X[:, c0:c0 + kb] = Xb
-        info["iters"] += inf.iters
-        info["outer"] = max(info["outer"], inf.outer)
-        info["flag"] = max(info["flag"], inf.flag) if info["flag"] is not None else None
-        info["launches"] += inf.launches
-        info["sweep_iters_max"] = max(info.get("sweep_iters_max", 0), inf.sweep_iters_max)
-        info["relres"] = max(info["relres"], inf.relres)
-        for key in ("spmm_ms", "update_ms", "spmm_launches", "update_launches", "coarse_ms", "coarse_launches"):
-            info[key] += getattr(inf, key)
+        _add_info(info, inf)
         if instances is not None:
             inst_status.append(instances.status.clone() if budget is not None else instances.status.cpu().numpy())
             inst_relres.append(rel)
@@ -831,11 +932,12 @@ def solve(mat, B, precision="mixed", tol=DEFAULT_TOL, inner_tol=None, maxiter=20
     elif instances is not None:
         info["inst_status"] = np.max(np.stack(inst_status), axis=0)
         info["inst_relres"] = torch.cat(inst_relres, dim=1).cpu().numpy()
-    info["coarse_nc"] = cs.nc if cs is not None else 0
+    info["coarse_nc"] = mid.coarse.nc if mid is not None else cs.nc if cs is not None else 0
     # the FP32 product of the last column block: the row-group kernel when
     # groups were given and the block width suits its lane layout
     kb = k - 128 * ((k - 1) // 128) if k else 0
-    info["spmm_kernel"] = ("spmm_blk_kernel" if rg is not None and 65 <= kb <= 128 and kb % 4 == 0
+    info["spmm_kernel"] = ("vc_spmm_kernel" if mid is not None and not (mat.is_complex and kb > 124)
+                           else "spmm_blk_kernel" if rg is not None and 65 <= kb <= 128 and kb % 4 == 0
                            else "spmm_pair_kernel")
     return X, info
 

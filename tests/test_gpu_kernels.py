@@ -122,3 +122,73 @@ def test_one_launch_solve_reports_failure():
     assert info["flag"] == 2
     keep = [0, 2, 3]
     assert (X[:, keep] - good[:, keep]).abs().max() <= 1e-12 * good.abs().max()
+
+
+def _box_cfg(cells, h, omega, ns, nd, seed=0, hole=False):
+    """A prepared box with nodal properties (a 4x mua / 3x mus inclusion) and
+    random optodes inside; ``hole`` leaves out a ball of tets, so that groups
+    and aggregates are partly empty."""
+    rng = np.random.default_rng(seed)
+    size = np.array(cells) * h
+    node, elem = kuhn_box(size, h)
+    inside = np.all((node > 0.5 * h) & (node < size - 0.5 * h), axis=1)
+    node[inside] += rng.uniform(-0.12, 0.12, (int(inside.sum()), 3)) * h
+    if hole:
+        c = node[elem - 1].mean(axis=1)
+        elem = elem[np.linalg.norm(c - size * [0.3, 0.3, 0.3], axis=1) > 0.2 * size.min()]
+        used = np.unique(elem)
+        remap = np.zeros(node.shape[0] + 1, dtype=np.int64)
+        remap[used] = np.arange(1, used.size + 1)
+        node, elem = node[used - 1], remap[elem]
+    nn = node.shape[0]
+    prop = np.column_stack([rng.uniform(0.008, 0.012, nn), rng.uniform(0.9, 1.1, nn), np.zeros(nn),
+                            np.full(nn, 1.37)])
+    inc = np.linalg.norm(node - size * [0.6, 0.5, 0.4], axis=1) < 0.15 * size.min()
+    prop[inc, :2] *= [4, 3]
+    pts = rng.uniform(0.55, 0.9, (ns + nd, 3)) * size * [1, 1, 0]
+    cfg = dict(node=node, elem=elem, prop=prop, srcpos=pts[:ns], srcdir=np.array([[0, 0, 1.0]]), detpos=pts[ns:],
+               detdir=np.array([[0, 0, 1.0]]), omega=omega)
+    return rbb.meshprep(cfg)[0]
+
+
+@pytest.mark.parametrize("omega", [0.0, 2 * np.pi * 1e8])
+@pytest.mark.parametrize("cells,cols,hole", [((28, 27, 25), (1, 2), True), ((28, 27, 25), (17, 20), True),
+                                             ((40, 24, 20), (31, 33), False), ((28, 27, 25), (33, 34), False),
+                                             ((27, 28, 26), (64, 64), True), ((28, 27, 25), (70, 61), False)])
+def test_vcycle_solve_matches_the_two_level_form(cells, cols, hole, omega):
+    """The three-level cycle at lane layouts from 4 to 128 columns (padded
+    counts, both column slices of complex solves, more than one block of 128)
+    on meshes with partly empty groups: the solution of the two-level and
+    Jacobi-only forms, each refined to the FP64 floor (the bars of the
+    two-level form's own tests: phi 1e-9, detectors 1e-6), in fewer
+    iterations, and again from a perturbed start."""
+    from redbirdpy_b200.forward import forward_device
+
+    cfg = _box_cfg(cells, 1.5, omega, *cols, hole=hole)
+    d1, p1, _, mat, i1 = forward_device(cfg)
+    assert mat.n >= engine.COARSE_MIN_NODES and engine.mesh_of(cfg).mid_level() is not None
+    assert i1["flag"] == 0 and i1["relres"] <= 1e-12 and i1["coarse_nc"] > 0
+    d0, p0, _, _, i0 = forward_device(cfg, coarse=True)
+    assert i0["flag"] == 0 and i1["iters"] < 0.7 * i0["iters"], (i1["iters"], i0["iters"])
+    assert (p1 - p0).abs().max() <= 1e-9 * p0.abs().max()
+    assert ((d1 - d0).abs() / d0.abs()).max() <= 1e-6
+    _, p2, _, _, i2 = forward_device(cfg, x0=p1 * (1 + 1e-3))
+    assert i2["flag"] == 0 and (p2 - p0).abs().max() <= 1e-9 * p0.abs().max()
+
+
+def test_vcycle_zero_and_non_finite_columns():
+    """A zero column stays exactly zero; a non-finite one is flagged and the
+    others still solve (through the two-level form)."""
+    cfg = _box_cfg((28, 27, 25), 1.5, 0.0, 3, 2)
+    mesh = engine.mesh_of(cfg)
+    mat = engine.assemble(mesh, engine.Optics.from_cfg(mesh, cfg))
+    B = engine.locate_optodes(mesh, cfg).rhs(mesh)
+    B[:, 1] = 0.0
+    X, info = engine.solve(mat, B)
+    assert info["flag"] == 0 and not X[:, 1].any()
+    B2 = B.clone()
+    B2[7, 2] = float("inf")
+    X2, info2 = engine.solve(mat, B2)
+    assert info2["flag"] == 2
+    keep = [0, 1, 3, 4]
+    assert (X2[:, keep] - X[:, keep]).abs().max() <= 1e-9 * X.abs().max()
