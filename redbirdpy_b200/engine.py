@@ -1068,6 +1068,30 @@ def _pad8(n):
     return (n + 7) // 8 * 8
 
 
+def _jac_what(name, mode):
+    """The RB_JAC_* quantity of a GN parameter."""
+    if name == "mua":
+        return _lib.RB_JAC_MUA_REF if mode == "reference" else _lib.RB_JAC_MUA_NODAL
+    if name == "D":
+        return _lib.RB_JAC_D
+    raise ValueError(f"unknown parameter {name}")
+
+
+def _jac_params(mesh, whats, phi, phi_kind, colsd, nc, det0, ndet, ps, pd, gnsd, J, ldj, out_kind, stride, node0, count):
+    """The rows of every parameter (rb_jac_multi), parameter p's columns from
+    p * stride."""
+    npar = len(whats)
+    wb = _lib.lib().rb_jac_multi_work_bytes(mesh.rmax)
+    if gnsd >= 0 or out_kind not in (_lib.RB_JAC_SPLIT_F32_ACC64, _lib.RB_JAC_F32_ACC64):
+        wb = 0  # not the pipelined kernel's: no workspace
+    work = torch.empty(wb, dtype=torch.uint8, device=phi.device) if wb else None
+    need_ddd = _lib.RB_JAC_D in whats
+    call("rb_jac_multi", ctypes.byref(mesh.struct), npar, (ctypes.c_int32 * npar)(*whats),
+         (ctypes.c_int64 * npar)(*(p * stride for p in range(npar))), ptr(phi), phi_kind, phi.shape[1], ptr(colsd), nc,
+         det0, ndet, ptr(ps), ptr(pd), gnsd, ptr(J), ldj, out_kind, mesh.rmax, mesh.emax, ptr(mesh.evol),
+         ptr(mesh.ddd if need_ddd else None), node0, count, ptr(work), wb, stream())
+
+
 def jacobian_matrix(mesh, phi, sd, params=("mua",), mode="reference", dtype=torch.float32, acc64=False):
     """The real Jacobian of the GN step (FP32, or BF16 with ``dtype``), rows x
     columns = (nsd or 2 nsd) x (len(params) * nn), stored with a row stride
@@ -1083,7 +1107,7 @@ def jacobian_matrix(mesh, phi, sd, params=("mua",), mode="reference", dtype=torc
     rows = 2 * nsd if cplx else nsd
     nn = mesh.nn
     bf = dtype == torch.bfloat16
-    ldj = _pad8(len(params) * nn) if bf else _pad4(len(params) * nn)
+    ldj = _pad8(len(params) * nn)  # (FP32: whole 32-byte sectors per row)
     # every column below len(params) * nn is written by rb_jac; only the
     # row padding (read by the gram's aligned tiles) is cleared here
     J = torch.empty((rows, ldj), dtype=dtype, device=phi.device)
@@ -1098,17 +1122,8 @@ def jacobian_matrix(mesh, phi, sd, params=("mua",), mode="reference", dtype=torc
     phi_kind = {torch.float64: _lib.RB_F64, torch.complex128: _lib.RB_C128, torch.float32: _lib.RB_F32,
                 torch.complex64: _lib.RB_C64}[phi.dtype]
     colsd, ps, pd = _i32(cols, phi.device), _i32(psrc, phi.device), _i32(pdet, phi.device)
-    for p, name in enumerate(params):
-        if name == "mua":
-            w = _lib.RB_JAC_MUA_REF if mode == "reference" else _lib.RB_JAC_MUA_NODAL
-        elif name == "D":
-            w = _lib.RB_JAC_D
-        else:
-            raise ValueError(f"unknown parameter {name}")
-        sub = J[:, p * nn:]
-        call("rb_jac", ctypes.byref(mesh.struct), w, ptr(phi), phi_kind, phi.shape[1], ptr(colsd), len(cols), det0,
-             ndet, ptr(ps), ptr(pd), _grid_nsd(psrc, pdet, det0, ndet), ptr(sub), ldj, out_kind, mesh.rmax,
-             mesh.emax, ptr(mesh.evol), ptr(mesh.ddd if w == _lib.RB_JAC_D else None), stream())
+    _jac_params(mesh, [_jac_what(name, mode) for name in params], phi, phi_kind, colsd, len(cols), det0, ndet, ps, pd,
+                _grid_nsd(psrc, pdet, det0, ndet), J, ldj, out_kind, nn, 0, nn)
     _jac_checked()
     return J, len(params) * nn
 
@@ -1263,8 +1278,7 @@ class SlabJacobian:
         self.K = len(self.params) * self.nn
         self.width = int(max(1, min(width, self.nn)))
         self.bf = dtype == torch.bfloat16
-        pad = _pad8 if self.bf else _pad4
-        self._pad = pad
+        pad = self._pad = _pad8
         self.buf = torch.empty(self.rows * pad(len(self.params) * self.width), dtype=dtype, device=phi.device)
         if self.bf:
             self.out_kind = _lib.RB_JAC_SPLIT_BF16 if self.cplx else _lib.RB_JAC_BF16
@@ -1274,14 +1288,7 @@ class SlabJacobian:
             self.out_kind = _lib.RB_JAC_SPLIT_F32 if self.cplx else _lib.RB_F32
         self.phi_kind = {torch.float64: _lib.RB_F64, torch.complex128: _lib.RB_C128, torch.float32: _lib.RB_F32,
                          torch.complex64: _lib.RB_C64}[phi.dtype]
-        self.whats = []
-        for name in self.params:
-            if name == "mua":
-                self.whats.append(_lib.RB_JAC_MUA_REF if mode == "reference" else _lib.RB_JAC_MUA_NODAL)
-            elif name == "D":
-                self.whats.append(_lib.RB_JAC_D)
-            else:
-                raise ValueError(f"unknown parameter {name}")
+        self.whats = [_jac_what(name, mode) for name in self.params]
         self.passes = 0
 
     def ranges(self):
@@ -1297,13 +1304,8 @@ class SlabJacobian:
         Js = self.buf[: self.rows * ld].view(self.rows, ld)
         if ld > ks:
             Js[:, ks:].zero_()
-        m = self.mesh
-        for p, w in enumerate(self.whats):
-            sub = Js[:, p * c:]
-            call("rb_jac_range", ctypes.byref(m.struct), w, ptr(self.phi), self.phi_kind, self.phi.shape[1],
-                 ptr(self.colsd), len(self.cols), self.det0, self.ndet, ptr(self.ps), ptr(self.pd), self.gnsd,
-                 ptr(sub), ld, self.out_kind, m.rmax, m.emax, ptr(m.evol), ptr(m.ddd if w == _lib.RB_JAC_D else None),
-                 a, c, stream())
+        _jac_params(self.mesh, self.whats, self.phi, self.phi_kind, self.colsd, len(self.cols), self.det0, self.ndet,
+                    self.ps, self.pd, self.gnsd, Js, ld, self.out_kind, c, a, c)
         _jac_checked()
         return Js, ks
 

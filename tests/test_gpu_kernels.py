@@ -192,3 +192,59 @@ def test_vcycle_zero_and_non_finite_columns():
     assert info2["flag"] == 2
     keep = [0, 1, 3, 4]
     assert (X2[:, keep] - X[:, keep]).abs().max() <= 1e-9 * X.abs().max()
+
+
+def _delaunay_cfg(seed=0):
+    """An irregular mesh: rows of more than 16 neighbours."""
+    from scipy.spatial import Delaunay
+
+    rng = np.random.default_rng(seed)
+    g = np.stack(np.meshgrid(*[np.arange(6.0)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    node = g + rng.uniform(-0.25, 0.25, g.shape)
+    elem = Delaunay(node).simplices + 1
+    x = node[elem - 1]
+    vol = np.abs(np.einsum("ij,ij->i", np.cross(x[:, 1] - x[:, 0], x[:, 2] - x[:, 0]), x[:, 3] - x[:, 0])) / 6
+    elem = elem[vol > 1e-6]
+    prop = np.tile([0.01, 1.0, 0.0, 1.37], (node.shape[0], 1))
+    cfg = dict(node=node, elem=elem, prop=prop, srcpos=np.array([[2.0, 2.0, 0]]), srcdir=np.array([[0, 0, 1.0]]),
+               detpos=np.array([[3.0, 3.0, 0]]), detdir=np.array([[0, 0, 1.0]]), omega=0)
+    return rbb.meshprep(cfg)[0]
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("mesh_kind", ["box", "delaunay"])
+@pytest.mark.parametrize("ns,nd", [(4, 4), (12, 8), (4, 64), (64, 4), (28, 36), (64, 64)])
+def test_grid_jacobian_rows_equal_the_general_kernels(ns, nd, mesh_kind, cplx):
+    """The pipelined kernel of the FP64-formed FP32 rows (both parameters, and
+    node slabs of odd widths) = rb_jac's rows per quantity, bit for bit: the
+    same products in the same order."""
+    mesh = engine.mesh_of(_mesh((7, 5, 4)) if mesh_kind == "box" else _delaunay_cfg())
+    assert (mesh.rmax <= 16) == (mesh_kind == "box") and mesh.rmax <= 32 and mesh.emax <= 64
+    g = torch.Generator("cuda").manual_seed(ns * 100 + nd)
+    dt = torch.complex128 if cplx else torch.float64
+    phi = torch.randn((mesh.nn, ns + nd + 1), generator=g, device="cuda", dtype=dt)
+    s, d = np.meshgrid(np.arange(ns), ns + np.arange(nd))
+    sd = np.column_stack([s.ravel(), d.ravel(), np.ones(ns * nd)])
+    kind = engine._lib.RB_JAC_SPLIT_F32_ACC64 if cplx else engine._lib.RB_JAC_F32_ACC64
+    cols, det0, ndet, psrc, pdet, colsd, ps, pd, gnsd = engine._pair_dev(sd, phi.device)
+    assert gnsd < 0
+    rows = (2 if cplx else 1) * ns * nd
+    nn = mesh.nn
+    for mode, whats in (("exact", (engine._lib.RB_JAC_MUA_NODAL, engine._lib.RB_JAC_D)),
+                        ("reference", (engine._lib.RB_JAC_MUA_REF,))):
+        params = ("mua", "D")[: len(whats)]
+        J, K = engine.jacobian_matrix(mesh, phi, sd, params, mode, acc64=True)
+        ref = torch.full_like(J, float("nan"))
+        for p, w in enumerate(whats):
+            engine.call("rb_jac", engine.ctypes.byref(mesh.struct), w, engine.ptr(phi),
+                        engine._lib.RB_C128 if cplx else engine._lib.RB_F64, phi.shape[1], engine.ptr(colsd),
+                        len(cols), det0, ndet, engine.ptr(ps), engine.ptr(pd), gnsd, engine.ptr(ref[:, p * nn:]),
+                        ref.shape[1], kind, mesh.rmax, mesh.emax, engine.ptr(mesh.evol), engine.ptr(mesh.ddd),
+                        engine.stream())
+        assert torch.equal(J[:, :K], ref[:, :K])
+        op = engine.SlabJacobian(mesh, phi, sd, params, mode, width=37, acc64=True)
+        for a, b in op.ranges():
+            Js, ks = op.slab(a, b)
+            want = torch.cat([ref[:, p * nn + a:p * nn + b] for p in range(len(whats))], 1)
+            assert ks == want.shape[1] and torch.equal(Js[:, :ks], want), (a, b)
+    assert rows == J.shape[0]
