@@ -566,7 +566,8 @@ int rb_split_tf32(float* J, float* lo, int64_t M, int64_t K, int64_t ldj, void* 
 int rb_reginv_prepare(double* H, int64_t M, int64_t ldh, double lambda, double* di, void* stream);
 size_t rb_cholesky_work_bytes(void);
 int rb_cholesky(double* H, int64_t M, int64_t ldh, void* work, size_t work_bytes, void* stream);
-/* rb_chol_solve's workspace: M doubles (the forward solution) */
+/* rb_chol_solve's workspace: both solutions in 64-word segments (a workspace
+ * of M doubles is taken too; the segments are then allocated on the stream) */
 size_t rb_chol_solve_work_bytes(int64_t M);
 int rb_chol_solve(const double* L, int64_t M, int64_t ldh, double* x, void* work, size_t work_bytes, void* stream);
 size_t rb_gemv_t_work_bytes(int64_t K);

@@ -344,97 +344,182 @@ __global__ void __launch_bounds__(kSyrkThreads) syrk_update_kernel(double* __res
       }
 }
 
-// The triangular solves of rb_chol_solve apply the diagonal blocks' inverses
-// X (kept by rb_cholesky in each block's strict upper triangle):
-// mode 0: y = X v (solves L_kk y = v), mode 1: y = X^T v (solves L_kk^T y = v).
-// y = X v (mode 0) or X^T v (mode 1) of diagonal block k0 into shared memory,
-// by all 256 threads of the block: the block's 64 x 64 entries are staged in
-// shared memory first (whole rows, coalesced), then a quad sums each output
-// from there in a fixed order; v is read from src[k0 ..]
-__device__ __forceinline__ void tri_block_apply(const double* __restrict__ L, int64_t ldh, int64_t k0, int nb,
-                                                const double* __restrict__ src, int mode, double* v, double* y,
-                                                double (*Xs)[kNB + 1]) {
+// L L^T x = b in one launch: a block of threads per 64-row block row (block
+// rows dealt round robin when there are more than resident blocks), forward in
+// ascending and then backward in descending order, so that every block only
+// waits for block rows that come earlier in its own order.  A solved segment
+// is handed on through global memory: its words start as kEmpty and a reader
+// polls the values themselves (one round trip through L2 instead of a flag and
+// then the data; a computed NaN is stored with another payload).  A thread
+// loads the next tile of L before it waits for the segment that multiplies it,
+// so per 64 rows the chain is one hand-over, a 64-term product, a quad
+// reduction and the product with the block's inverse.  One launch per block
+// row and direction before: 1024 launches of 8-11 us for the four solves of a
+// refined M = 8192 step, 2.36 ms per solve, now 0.43 ms (M = 8192).  Waits are bounded;
+// one that gives up ends its block with NaN in its segment.
+constexpr unsigned long long kEmpty = ~0ull;
+constexpr int kTrsvSpins = 1 << 20;  // about a second
+
+__device__ __forceinline__ double2 ld_seg(const double* p) {
+  double2 v;
+  asm volatile("ld.relaxed.gpu.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_seg(double* p, double v) {
+  if (isnan(v)) v = __longlong_as_double(0x7ff8000000000000LL);
+  asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
+}
+__device__ __forceinline__ bool seg_empty(double v) { return (unsigned long long)__double_as_longlong(v) == kEmpty; }
+
+// 8 pairs of a segment at p + stride u; false when they do not arrive
+template <int STRIDE>
+__device__ __forceinline__ bool wait_seg(const double* p, double2 (&v)[8], const volatile int& bad) {
+  for (int spin = 0; spin < kTrsvSpins; ++spin) {
+    bool ok = true;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      v[u] = ld_seg(p + STRIDE * u);
+      ok = ok && !seg_empty(v[u].x) && !seg_empty(v[u].y);
+    }
+    if (ok) return true;
+    if (spin > 256) {
+      if (bad) return false;  // (the block has given up already)
+      __nanosleep(64);
+    }
+  }
+  return false;
+}
+
+// y, x: segments of ceil(M / 64) x 64 words, all kEmpty at launch; xio: b on
+// entry, the solution on return
+__global__ void __launch_bounds__(256, 1) chol_solve_kernel(const double* __restrict__ L, int64_t ldh, int64_t M,
+                                                            double* __restrict__ xio, double* __restrict__ y,
+                                                            double* __restrict__ x) {
+  __shared__ double t[kNB], part[4][kNB];
+  __shared__ int bad;
   const int tid = threadIdx.x;
-#pragma unroll 4
-  for (int e = tid; e < kNB * kNB; e += 256) {
-    const int r = e / kNB, c = e % kNB;
-    Xs[r][c] = (r < nb && c < nb) ? L[(k0 + r) * ldh + k0 + c] : 0.0;
-  }
-  if (tid < nb) v[tid] = src[k0 + tid];
+  const int64_t nblk = (M + kNB - 1) / kNB;
+  if (tid == 0) bad = 0;
   __syncthreads();
-  const int i = tid >> 2, q = tid & 3;
-  double s = 0.0;
-  if (i < nb) {
-    if (mode == 0) {  // X[i][t], t < i, sits at (t, i)
-      for (int t = q; t <= i; t += 4) s = fma(t == i ? 1.0 / Xs[i][i] : Xs[t][i], v[t], s);
-    } else {  // X[t][i], t > i, sits at (i, t)
-      for (int t = i + q; t < nb; t += 4) s = fma(t == i ? 1.0 / Xs[i][i] : Xs[i][t], v[t], s);
+  // ---- L y = b: thread (r, q) sums columns 8 u + 2 q, + 1 of row r
+  {
+    const int r = tid >> 2, q = tid & 3;
+    for (int64_t j = blockIdx.x; j < nblk; j += gridDim.x) {
+      const int64_t j0 = j * kNB, row = j0 + r;
+      const int nb = (int)min((int64_t)kNB, M - j0);
+      const bool on = r < nb;
+      // the inverse's row r: X[r][c] at (c, r), c < r; 1 / L[r][r]
+      double xi[16];
+#pragma unroll
+      for (int u = 0; u < 16; ++u) {
+        const int c = 8 * (u >> 1) + 2 * q + (u & 1);
+        xi[u] = !on || c > r ? 0.0 : c == r ? 1.0 / L[row * ldh + row] : L[(j0 + c) * ldh + row];
+      }
+      const double* Lr = L + (on ? row : j0) * ldh + 2 * q;
+      double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0, lt[16];
+      auto tile = [&](int64_t i) {
+#pragma unroll
+        for (int u = 0; u < 16; ++u) lt[u] = Lr[i * kNB + 8 * (u >> 1) + (u & 1)];
+      };
+      if (j > 0) tile(0);
+      for (int64_t i = 0; i < j; ++i) {
+        double c[16];
+#pragma unroll
+        for (int u = 0; u < 16; ++u) c[u] = lt[u];
+        if (i + 1 < j) tile(i + 1);
+        double2 v[8];
+        if (!wait_seg<8>(y + i * kNB + 2 * q, v, bad)) bad = 1;
+#pragma unroll
+        for (int u = 0; u < 8; u += 2) {
+          a0 = fma(c[2 * u], v[u].x, a0);
+          a1 = fma(c[2 * u + 1], v[u].y, a1);
+          a2 = fma(c[2 * u + 2], v[u + 1].x, a2);
+          a3 = fma(c[2 * u + 3], v[u + 1].y, a3);
+        }
+      }
+      double s = (a0 + a1) + (a2 + a3);
+      s += __shfl_xor_sync(0xffffffffu, s, 1);
+      s += __shfl_xor_sync(0xffffffffu, s, 2);
+      if (q == 0) t[r] = on ? xio[row] - s : 0.0;
+      __syncthreads();
+      double z0 = 0.0, z1 = 0.0;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        z0 = fma(xi[2 * u], t[8 * u + 2 * q], z0);
+        z1 = fma(xi[2 * u + 1], t[8 * u + 2 * q + 1], z1);
+      }
+      double z = z0 + z1;
+      z += __shfl_xor_sync(0xffffffffu, z, 1);
+      z += __shfl_xor_sync(0xffffffffu, z, 2);
+      if (q == 0) st_seg(y + j0 + r, bad ? __longlong_as_double(0x7ff8000000000000LL) : z);
+      __syncthreads();
     }
   }
-  s += __shfl_xor_sync(0xffffffffu, s, 1);
-  s += __shfl_xor_sync(0xffffffffu, s, 2);
-  if (i < nb && q == 0) y[i] = s;
-  __syncthreads();
-}
-
-// One forward step of L y = b, fused: every block solves diagonal block k0
-// (y = X v, v = x[k0 ..]) itself, block 0 stores y in w, and each block
-// subtracts L[r][k0 ..] y from its kSolveRows rows r below the block (rows
-// split over the 8 warps; lane c sums columns c and c + 32, then a warp sum
-// per row).
-constexpr int kSolveRows = 32;
-__global__ void __launch_bounds__(256) fwd_solve_kernel(const double* __restrict__ L, int64_t ldh, int64_t M,
-                                                        int64_t k0, int nb, double* __restrict__ x,
-                                                        double* __restrict__ w) {
-  __shared__ double v[kNB], y[kNB];
-  __shared__ double Xs[kNB][kNB + 1];
-  tri_block_apply(L, ldh, k0, nb, x, 0, v, y, Xs);
-  if (blockIdx.x == 0 && threadIdx.x < nb) w[k0 + threadIdx.x] = y[threadIdx.x];
-  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-  constexpr int RW = kSolveRows / 8;  // rows per warp
-  const int64_t rb = k0 + nb + blockIdx.x * (int64_t)kSolveRows + wp * RW;
-  const double y0 = lane < nb ? y[lane] : 0.0, y1 = lane + 32 < nb ? y[lane + 32] : 0.0;
-  double s[RW];
+  // ---- L^T x = y: thread (c, g) sums rows 16 g .. + 15 of column c
+  {
+    const int c = tid & 63, g = tid >> 6;
+    const int64_t last = (nblk - 1 - blockIdx.x) / gridDim.x * gridDim.x + blockIdx.x;  // the block's last block row
+    for (int64_t j = blockIdx.x < nblk ? last : -1; j >= 0; j -= gridDim.x) {
+      const int64_t j0 = j * kNB;
+      const int nb = (int)min((int64_t)kNB, M - j0);
+      const bool on = c < nb;
+      // column c of the inverse: X[r][c] at (c, r), r > c; 1 / L[c][c]
+      double xi[16];
 #pragma unroll
-  for (int u = 0; u < RW; ++u) {
-    const int64_t r = rb + u;
-    s[u] = 0.0;
-    if (r < M) {
-      const double* Lr = L + r * ldh + k0;
-      if (lane < nb) s[u] = Lr[lane] * y0;
-      if (lane + 32 < nb) s[u] = fma(Lr[lane + 32], y1, s[u]);
+      for (int u = 0; u < 16; ++u) {
+        const int r = 16 * g + u;
+        xi[u] = !on || r < c || r >= nb ? 0.0 : r == c ? 1.0 / L[(j0 + c) * ldh + j0 + c] : L[(j0 + c) * ldh + j0 + r];
+      }
+      const double* Lc = L + j0 + (on ? c : 0);
+      double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0, lt[16];
+      auto tile = [&](int64_t i) {
+#pragma unroll
+        for (int u = 0; u < 16; ++u) {
+          const int64_t r = i * kNB + 16 * g + u;
+          lt[u] = r < M ? Lc[r * ldh] : 0.0;
+        }
+      };
+      if (j + 1 < nblk) tile(nblk - 1);
+      for (int64_t i = nblk - 1; i > j; --i) {
+        double l[16];
+#pragma unroll
+        for (int u = 0; u < 16; ++u) l[u] = lt[u];
+        if (i - 1 > j) tile(i - 1);
+        double2 v[8];
+        if (!wait_seg<2>(x + i * kNB + 16 * g, v, bad)) bad = 1;
+#pragma unroll
+        for (int u = 0; u < 8; u += 2) {
+          a0 = fma(l[2 * u], v[u].x, a0);
+          a1 = fma(l[2 * u + 1], v[u].y, a1);
+          a2 = fma(l[2 * u + 2], v[u + 1].x, a2);
+          a3 = fma(l[2 * u + 3], v[u + 1].y, a3);
+        }
+      }
+      part[g][c] = (a0 + a1) + (a2 + a3);
+      __syncthreads();
+      if (tid < kNB) {
+        // this block row's own y (the same block solved it)
+        const double yv = ld_seg(y + j0 + (tid & ~1)).x, yw = ld_seg(y + j0 + (tid & ~1)).y;
+        const double s = (part[0][tid] + part[1][tid]) + (part[2][tid] + part[3][tid]);
+        t[tid] = tid < nb ? ((tid & 1) ? yw : yv) - s : 0.0;
+      }
+      __syncthreads();
+      double z0 = 0.0, z1 = 0.0;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        z0 = fma(xi[2 * u], t[16 * g + 2 * u], z0);
+        z1 = fma(xi[2 * u + 1], t[16 * g + 2 * u + 1], z1);
+      }
+      part[g][c] = z0 + z1;
+      __syncthreads();
+      if (tid < kNB) {
+        double z = (part[0][tid] + part[1][tid]) + (part[2][tid] + part[3][tid]);
+        if (bad) z = __longlong_as_double(0x7ff8000000000000LL);
+        st_seg(x + j0 + tid, z);
+        if (tid < nb) xio[j0 + tid] = z;
+      }
+      __syncthreads();
     }
-  }
-#pragma unroll
-  for (int u = 0; u < RW; ++u) {
-    const double t = warp_sum(s[u]);
-    if (lane == 0 && rb + u < M) x[rb + u] -= t;
-  }
-}
-
-// One backward step of L^T x = y, fused: every block solves diagonal block
-// k0 (v = w[k0 ..], the forward solution less the later blocks' terms),
-// block 0 stores the result in x, and each block subtracts L[k0 + r][j] y[r]
-// from its 32 columns j < k0 of w (8 warps over the block's rows, summed in
-// a fixed order).
-__global__ void __launch_bounds__(256) bwd_solve_kernel(const double* __restrict__ L, int64_t ldh, int64_t k0, int nb,
-                                                        double* __restrict__ w, double* __restrict__ x) {
-  __shared__ double v[kNB], y[kNB], part[8][32];
-  __shared__ double Xs[kNB][kNB + 1];
-  tri_block_apply(L, ldh, k0, nb, w, 1, v, y, Xs);
-  if (blockIdx.x == 0 && threadIdx.x < nb) x[k0 + threadIdx.x] = y[threadIdx.x];
-  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-  const int64_t j = blockIdx.x * 32 + lane;
-  double s = 0.0;
-  if (j < k0)
-    for (int r = wp; r < nb; r += 8) s = fma(L[(k0 + r) * ldh + j], y[r], s);
-  part[wp][lane] = s;
-  __syncthreads();
-  if (wp == 0 && j < k0) {
-    double t = 0.0;
-#pragma unroll
-    for (int q = 0; q < 8; ++q) t += part[q][lane];
-    w[j] -= t;
   }
 }
 
@@ -874,27 +959,39 @@ int rb_cholesky(double* H, int64_t M, int64_t ldh, void* work, size_t work_bytes
   return RB_OK;
 }
 
-size_t rb_chol_solve_work_bytes(int64_t M) { return (size_t)std::max<int64_t>(M, 1) * sizeof(double); }
+// the segments of y and x, whole blocks of 64
+size_t rb_chol_solve_work_bytes(int64_t M) {
+  return 2 * (size_t)ceil_div(std::max<int64_t>(M, 1), kNB) * kNB * sizeof(double) + 16;
+}
 
 int rb_chol_solve(const double* L, int64_t M, int64_t ldh, double* x, void* work, size_t work_bytes, void* stream) {
   if (!L || !x || !work || M < 1 || ldh < M) return fail(RB_EARG, "rb_chol_solve: bad arguments");
-  if (work_bytes < rb_chol_solve_work_bytes(M)) return fail(RB_EARG, "rb_chol_solve: workspace too small");
+  if (work_bytes < (size_t)M * sizeof(double)) return fail(RB_EARG, "rb_chol_solve: workspace too small");
   cudaStream_t st = as_stream(stream);
-  // one launch per diagonal block and direction: each block of a launch
-  // solves the 64 x 64 diagonal step itself and then its share of the update
-  double* w = reinterpret_cast<double*>(work);  // the forward solution, consumed by the backward steps
-  for (int64_t k0 = 0; k0 < M; k0 += kNB) {  // L y = b
-    const int nb = (int)std::min<int64_t>(kNB, M - k0);
-    const int64_t rest = M - k0 - nb;
-    fwd_solve_kernel<<<(unsigned)std::max<int64_t>(1, ceil_div(rest, kSolveRows)), 256, 0, st>>>(L, ldh, M, k0, nb,
-                                                                                                 x, w);
-    RB_LAUNCH_CHECK();
+  const int64_t nblk = ceil_div(M, kNB);
+  // a workspace of M doubles is taken as well: the segments come from the pool
+  void* own = nullptr;
+  if (work_bytes < rb_chol_solve_work_bytes(M)) {
+    RB_CUDA_TRY(cudaMallocAsync(&own, rb_chol_solve_work_bytes(M), st));
+    work = own;
   }
-  for (int64_t k0 = ((M - 1) / kNB) * kNB; k0 >= 0; k0 -= kNB) {  // L^T x = y
-    const int nb = (int)std::min<int64_t>(kNB, M - k0);
-    bwd_solve_kernel<<<(unsigned)std::max<int64_t>(1, ceil_div(k0, 32)), 256, 0, st>>>(L, ldh, k0, nb, w, x);
-    RB_LAUNCH_CHECK();
+  double* ys = reinterpret_cast<double*>((reinterpret_cast<uintptr_t>(work) + 15) & ~uintptr_t(15));
+  double* xs = ys + nblk * kNB;
+  cudaError_t e = cudaMemsetAsync(ys, 0xff, 2 * (size_t)nblk * kNB * sizeof(double), st);
+  // the blocks wait for one another: a cooperative launch, at most one per SM
+  int dev = 0, sms = 1;
+  if (e == cudaSuccess) e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e == cudaSuccess) {
+    void* args[] = {(void*)&L, (void*)&ldh, (void*)&M, (void*)&x, (void*)&ys, (void*)&xs};
+    e = cudaLaunchCooperativeKernel((const void*)chol_solve_kernel, dim3((unsigned)std::min<int64_t>(nblk, sms)),
+                                    dim3(256), args, 0, st);
   }
+  if (own) {
+    const cudaError_t f = cudaFreeAsync(own, st);
+    if (e == cudaSuccess) e = f;
+  }
+  RB_CUDA_TRY(e);
   return RB_OK;
 }
 

@@ -248,3 +248,50 @@ def test_grid_jacobian_rows_equal_the_general_kernels(ns, nd, mesh_kind, cplx):
             want = torch.cat([ref[:, p * nn + a:p * nn + b] for p in range(len(whats))], 1)
             assert ks == want.shape[1] and torch.equal(Js[:, :ks], want), (a, b)
     assert rows == J.shape[0]
+
+
+@pytest.mark.parametrize("M,pad", [(1, 0), (2, 3), (63, 1), (64, 0), (65, 0), (128, 5), (1000, 0), (9473, 0), (9535, 1)])
+def test_chol_solve_segments(M, pad):
+    """L L^T x = b over block rows handed on between thread blocks: one block
+    row, ragged last rows, strided factors, and more block rows than SMs (9473
+    = 148 x 64 + 1).  L is unit-diagonal plus a small lower part, so that
+    ||L^-1||_inf <= 1 / (1 - 0.5) and the error bound M eps cond is below
+    M x 2.2e-16 x 16; with the short workspace and in a captured launch the
+    bits are the same."""
+    g = torch.Generator("cuda").manual_seed(M)
+    ld = M + pad
+    L = torch.rand((M, ld), generator=g, device="cuda", dtype=torch.float64).sub_(0.5).mul_(1.0 / M)
+    Lt = torch.tril(L[:, :M], -1) + torch.eye(M, device="cuda", dtype=torch.float64)
+    H = torch.full((M, ld), float("nan"), device="cuda", dtype=torch.float64)
+    H[:, :M] = Lt
+    # rb_cholesky leaves each diagonal block's inverse in its strict upper triangle
+    for k in range(0, M, 64):
+        e = min(M, k + 64)
+        X = torch.linalg.inv(Lt[k:e, k:e])
+        H[k:e, k:e] = Lt[k:e, k:e] + torch.tril(X, -1).T
+    x0 = torch.randn(M, generator=g, device="cuda", dtype=torch.float64)
+    b = Lt @ (Lt.T @ x0)
+    tol = M * 2.2e-16 * 16 * float(x0.abs().max())
+    wb = engine._lib.lib().rb_chol_solve_work_bytes(M)
+
+    def solve(x, w, nbytes):
+        engine.call("rb_chol_solve", engine.ptr(H), M, ld, engine.ptr(x), engine.ptr(w), nbytes, engine.stream())
+
+    work = torch.empty(wb, dtype=torch.uint8, device="cuda")
+    x = b.clone()
+    solve(x, work, wb)
+    assert float((x - x0).abs().max()) <= tol
+    short = torch.empty(M * 8, dtype=torch.uint8, device="cuda")
+    xs = b.clone()
+    solve(xs, short, M * 8)
+    assert torch.equal(x, xs)
+    xc = b.clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        solve(xc, work, wb)
+    for _ in range(2):
+        xc.copy_(b)
+        graph.replay()
+        assert torch.equal(x, xc)
+    with pytest.raises(Exception, match="workspace too small"):
+        solve(xs, short, M * 8 - 1)
