@@ -34,130 +34,172 @@ __global__ void prep_scale_kernel(double* __restrict__ H, int64_t M, int64_t ldh
 }
 
 // Factor the nb x nb diagonal block at (j0, j0) (lower, L11) and form its
-// inverse X = L11^-1.  256 threads; the block's lower triangle sits in
-// shared memory.  Column c: every thread reads the pivot and forms its
-// reciprocal square root itself (no hand-off), 64 threads scale the column,
-// and after a barrier the rank-1 update of the columns right of c is spread
-// over all threads (each owns the same ~9 entries of the triangle in every
-// step).  X is then formed column by column by forward substitution (thread
-// (j = tid / 4, q = tid % 4) owns column j, rows q, q + 4, ...; the quad's
-// terms in four interleaved chains, added in fixed order) and stored
-// transposed in the block's strict upper triangle:
-// H[j0 + j][j0 + i] = X[i][j], i > j (the diagonal of X is 1 / L[i][i]).
-// The panel solve and rb_chol_solve then apply X as a product.
-constexpr int kTri = kNB * (kNB + 1) / 2;     // entries of the lower triangle
-constexpr int kTriOwn = (kTri + 255) / 256;  // per thread
+// inverse X = L11^-1, stored transposed in the block's strict upper triangle:
+// H[j0 + j][j0 + i] = X[i][j], i > j (the diagonal of X is 1 / L[i][i]).  The
+// panel solve and rb_chol_solve then apply X as a product.
+//
+// One block of 256 threads; the bound is the chain of 64 pivots.  It runs in
+// four steps of 16 columns, so that only a 16 x 16 block's pivots are serial:
+// one warp factors it in registers (lane = row; a pivot's reciprocal root and
+// one row exchange per column, no barrier) and inverts it, then all threads
+// apply that inverse to the rows below (16-term products) and update the rest
+// of the triangle (16-term products, 2 x 2 entries per thread).  X is put
+// together from the four 16 x 16 inverses by block products.  Rows beyond nb
+// are padded with the identity.  (Two columns per barrier pair over the whole
+// block, and the inverse by a chain of 64 substitution steps, took 63.6 us per
+// block in an M = 8192 factorisation, now 38, 24 where no update shares its SM;
+// 128 of them are on the critical path.)
+constexpr int kPB = 16;
 __global__ void __launch_bounds__(256) potrf_diag_kernel(double* __restrict__ H, int64_t ldh, int64_t j0, int nb,
                                                          int* __restrict__ err) {
-  __shared__ double Ls[kNB][kNB + 1];
-  __shared__ double rdiag[kNB];
-  const int tid = threadIdx.x;
-  for (int e = tid; e < kNB * kNB; e += 256) {
-    const int i = e / kNB, j = e % kNB;
-    Ls[i][j] = (i < nb && j <= i) ? H[(j0 + i) * ldh + j0 + j] : 0.0;
-  }
-  // owned entries e = tid + 256 v of the row-major lower triangle, (i, j)
-  // packed as i * 256 + j (-1: none)
-  int own[kTriOwn];
+  __shared__ double Ls[kNB][kNB + 1];  // the block, then L
+  extern __shared__ double psm[];
+  double(*Xs)[kNB + 1] = reinterpret_cast<double(*)[kNB + 1]>(psm);           // X (lower)
+  double(*Ts)[kPB + 1] = reinterpret_cast<double(*)[kPB + 1]>(psm + kNB * (kNB + 1));  // 3 x 16 x 16 products
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  double in[kNB * kNB / 256];  // every load under way before the first is used
 #pragma unroll
-  for (int v = 0; v < kTriOwn; ++v) {
-    const int e = tid + 256 * v;
-    if (e < kTri) {
-      int i = (int)((sqrtf(8.f * (float)e + 1.f) - 1.f) * 0.5f);
-      while (i * (i + 1) / 2 > e) --i;
-      while ((i + 1) * (i + 2) / 2 <= e) ++i;
-      own[v] = i * 256 + (e - i * (i + 1) / 2);
-    } else {
-      own[v] = -1;
-    }
+  for (int v = 0; v < kNB * kNB / 256; ++v) {
+    const int i = (tid + 256 * v) / kNB, j = tid % kNB;
+    in[v] = (i < nb && j <= i) ? H[(j0 + i) * ldh + j0 + j] : (i == j ? 1.0 : 0.0);
+  }
+#pragma unroll
+  for (int v = 0; v < kNB * kNB / 256; ++v) {
+    const int i = (tid + 256 * v) / kNB, j = tid % kNB;
+    Ls[i][j] = in[v];
+    Xs[i][j] = 0.0;
   }
   __syncthreads();
-  // Two columns per step (one barrier pair instead of two): with c and c + 1,
-  // every thread forms both pivots itself; thread i scales its entry of
-  // column c, takes column c's update of its entry of column c + 1 and
-  // scales that; then the owned entries right of c + 1 take both updates,
-  // column c's first.  Every entry sees the same operations in the same
-  // order as in one column per step, so the factor is the same bits.
-  // One reciprocal square root per column: the pivot is d / sqrt(d), and
-  // the column is scaled by 1 / sqrt(d) (as LAPACK's dpotf2 scales by the
-  // reciprocal).
-  for (int c = 0; c < nb; c += 2) {
-    if (c + 1 < nb) {
-      const double d0 = Ls[c][c], a10 = Ls[c + 1][c], a11 = Ls[c + 1][c + 1];
-      const bool ok0 = d0 > 0.0 && isfinite(d0);
-      const double rp0 = ok0 ? rsqrt(d0) : 1.0;
-      const double l10 = a10 * rp0;
-      const double d1 = fma(-l10, l10, a11);
-      const bool ok1 = d1 > 0.0 && isfinite(d1);
-      const double rp1 = ok1 ? rsqrt(d1) : 1.0;
-      if (tid == 0 && (!ok0 || !ok1)) atomicExch(err, (int)(j0 + c + (ok0 ? 1 : 0)) + 1);
-      if (tid > c + 1 && tid < nb) {
-        const double li0 = Ls[tid][c] * rp0;
-        Ls[tid][c] = li0;
-        Ls[tid][c + 1] = fma(-li0, l10, Ls[tid][c + 1]) * rp1;
-      }
-      __syncthreads();
-      // every thread has read the pivots: their entries take L now (the
-      // update below reads only the entries below them in columns c, c + 1)
-      if (tid == c) Ls[c][c] = ok0 ? d0 * rp0 : 1.0;
-      if (tid == c + 1) {
-        Ls[c + 1][c] = l10;
-        Ls[c + 1][c + 1] = ok1 ? d1 * rp1 : 1.0;
-      }
+#pragma unroll 1
+  for (int kb = 0; kb < kNB; kb += kPB) {
+    if (w == 0) {  // lanes 16..31 repeat lanes 0..15
+      const int l = lane & (kPB - 1);
+      double r[kPB], x[kPB], ri = 1.0;
 #pragma unroll
-      for (int v = 0; v < kTriOwn; ++v) {
-        const int i = own[v] >> 8, j = own[v] & 255;
-        if (own[v] >= 0 && j > c + 1 && i < nb)
-          Ls[i][j] = fma(-Ls[i][c + 1], Ls[j][c + 1], fma(-Ls[i][c], Ls[j][c], Ls[i][j]));
+      for (int c = 0; c < kPB; ++c) r[c] = Ls[kb + l][kb + c];
+#pragma unroll
+      for (int c = 0; c < kPB; ++c) {
+        const double d = __shfl_sync(0xffffffffu, r[c], c);
+        const bool ok = d > 0.0 && isfinite(d);
+        const double rp = ok ? rsqrt(d) : 1.0;
+        if (lane == 0 && !ok && kb + c < nb) atomicCAS(err, 0, (int)(j0 + kb + c) + 1);
+        const double lc = l == c ? (ok ? d * rp : 1.0) : r[c] * rp;
+        r[c] = lc;
+#pragma unroll
+        for (int j = c + 1; j < kPB; ++j) r[j] = fma(-lc, __shfl_sync(0xffffffffu, lc, j), r[j]);
       }
-      __syncthreads();
-    } else {  // the last column of an odd block
-      const double d = Ls[c][c];
-      const bool ok = d > 0.0 && isfinite(d);
-      const double rp = ok ? rsqrt(d) : 1.0;
-      if (tid == 0 && !ok) atomicExch(err, (int)(j0 + c) + 1);
-      __syncthreads();
-      if (tid == c) Ls[c][c] = ok ? d * rp : 1.0;
-      __syncthreads();
+      if (lane < kPB) {
+#pragma unroll
+        for (int c = 0; c < kPB; ++c)
+          if (c <= l) Ls[kb + l][kb + c] = r[c];
+      }
+      // column l of the inverse by substitution; 1 / L[i][i] = ri of lane i
+#pragma unroll
+      for (int c = 0; c < kPB; ++c)
+        if (c == l) ri = r[c];
+      ri = 1.0 / ri;
+#pragma unroll
+      for (int i = 0; i < kPB; ++i) {
+        double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+        for (int k = 0; k < i; ++k) {
+          const double lik = __shfl_sync(0xffffffffu, r[k], i);
+          if (k & 1) s1 = fma(lik, x[k], s1);
+          else s0 = fma(lik, x[k], s0);
+        }
+        const double rii = __shfl_sync(0xffffffffu, ri, i);
+        x[i] = i < l ? 0.0 : i == l ? rii : -(s0 + s1) * rii;
+      }
+      if (lane < kPB) {
+#pragma unroll
+        for (int i = 0; i < kPB; ++i) Xs[kb + i][kb + l] = x[i];
+      }
     }
+    __syncthreads();
+    const int m0 = kb + kPB, mr = kNB - m0;  // rows below
+    // L21 = A21 X11^T: thread = (row, 4 columns)
+    for (int e = tid; e < mr * 4; e += 256) {
+      const int i = m0 + (e >> 2), c0 = (e & 3) * 4;
+      double a[kPB], o[4];
+#pragma unroll
+      for (int t = 0; t < kPB; ++t) a[t] = Ls[i][kb + t];
+#pragma unroll
+      for (int v = 0; v < 4; ++v) {
+        double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+        for (int t = 0; t < kPB; t += 2) {
+          s0 = fma(a[t], Xs[kb + c0 + v][kb + t], s0);
+          s1 = fma(a[t + 1], Xs[kb + c0 + v][kb + t + 1], s1);
+        }
+        o[v] = s0 + s1;
+      }
+      __syncwarp();  // the four threads of a row have read it (whole warps: mr * 4 is a multiple of 32)
+#pragma unroll
+      for (int v = 0; v < 4; ++v) Ls[i][kb + c0 + v] = o[v];
+    }
+    __syncthreads();
+    // the rest of the triangle, 2 x 2 entries per thread
+    const int h = mr / 2;
+    for (int e = tid; e < h * (h + 1) / 2; e += 256) {
+      int bi = (int)((sqrtf(8.f * (float)e + 1.f) - 1.f) * 0.5f);
+      while (bi * (bi + 1) / 2 > e) --bi;
+      while ((bi + 1) * (bi + 2) / 2 <= e) ++bi;
+      const int i = m0 + 2 * bi, j = m0 + 2 * (e - bi * (bi + 1) / 2);
+      double s00 = Ls[i][j], s01 = Ls[i][j + 1], s10 = Ls[i + 1][j], s11 = Ls[i + 1][j + 1];
+#pragma unroll
+      for (int t = 0; t < kPB; ++t) {
+        const double a0 = Ls[i][kb + t], a1 = Ls[i + 1][kb + t], b0 = Ls[j][kb + t], b1 = Ls[j + 1][kb + t];
+        s00 = fma(-a0, b0, s00);
+        s01 = fma(-a0, b1, s01);
+        s10 = fma(-a1, b0, s10);
+        s11 = fma(-a1, b1, s11);
+      }
+      Ls[i][j] = s00;
+      if (j + 1 <= i) Ls[i][j + 1] = s01;
+      Ls[i + 1][j] = s10;
+      Ls[i + 1][j + 1] = s11;
+    }
+    __syncthreads();
   }
-  // L11 back to H (lower, whole rows)
   for (int e = tid; e < kNB * kNB; e += 256) {
     const int i = e / kNB, j = e % kNB;
     if (i < nb && j <= i) H[(j0 + i) * ldh + j0 + j] = Ls[i][j];
   }
-  if (tid < nb) rdiag[tid] = 1.0 / Ls[tid][tid];  // the 64 reciprocals at once, off the chain below
-  __syncthreads();
-  // X = L11^-1, column j by the quad of column j: X[j][j] = 1 / L[j][j],
-  // X[i][j] = -(sum_{k=j}^{i-1} L[i][k] X[k][j]) / L[i][i]
-  const int j = tid >> 2, q = tid & 3;
-  double x[kNB / 4];
+  // X below its diagonal blocks, one block diagonal after the other:
+  // X_pq = -X_pp sum_{q <= k < p} L_pk X_kq; thread = one entry of a block
+  const int bi = tid >> 4, bj = tid & 15;
+#pragma unroll 1
+  for (int dgl = 1; dgl < kNB / kPB; ++dgl) {
+    for (int q = 0; q + dgl < kNB / kPB; ++q) {
+      const int p = q + dgl;
+      double s0 = 0.0, s1 = 0.0;
+      for (int k = q; k < p; ++k)
 #pragma unroll
-  for (int u = 0; u < kNB / 4; ++u) x[u] = 0.0;
-  for (int i = 0; i < nb; ++i) {
-    double p[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll
-    for (int u = 0; u < kNB / 4; ++u) {
-      const int k = q + 4 * u;
-      if (k >= j && k < i) p[u & 3] = fma(Ls[i][k], x[u], p[u & 3]);
+        for (int t = 0; t < kPB; t += 2) {
+          s0 = fma(Ls[p * kPB + bi][k * kPB + t], Xs[k * kPB + t][q * kPB + bj], s0);
+          s1 = fma(Ls[p * kPB + bi][k * kPB + t + 1], Xs[k * kPB + t + 1][q * kPB + bj], s1);
+        }
+      Ts[q * kPB + bi][bj] = s0 + s1;
     }
-    double part = (p[0] + p[1]) + (p[2] + p[3]);
-    part += __shfl_xor_sync(0xffffffffu, part, 1);
-    part += __shfl_xor_sync(0xffffffffu, part, 2);
-    if (i >= j && j < nb) {
-      const double ri = rdiag[i];
-      const double xi = (i == j) ? ri : -part * ri;
+    __syncthreads();
+    for (int q = 0; q + dgl < kNB / kPB; ++q) {
+      const int p = q + dgl;
+      double s0 = 0.0, s1 = 0.0;
 #pragma unroll
-      for (int u = 0; u < kNB / 4; ++u)
-        if (q + 4 * u == i) x[u] = xi;
+      for (int t = 0; t < kPB; t += 2) {
+        s0 = fma(Xs[p * kPB + bi][p * kPB + t], Ts[q * kPB + t][bj], s0);
+        s1 = fma(Xs[p * kPB + bi][p * kPB + t + 1], Ts[q * kPB + t + 1][bj], s1);
+      }
+      Xs[p * kPB + bi][q * kPB + bj] = -(s0 + s1);
     }
+    __syncthreads();
   }
-#pragma unroll
-  for (int u = 0; u < kNB / 4; ++u) {
-    const int i = q + 4 * u;
-    if (i > j && i < nb && j < nb) H[(j0 + j) * ldh + j0 + i] = x[u];
+  for (int e = tid; e < kNB * kNB; e += 256) {
+    const int j = e / kNB, i = e % kNB;
+    if (i > j && i < nb) H[(j0 + j) * ldh + j0 + i] = Xs[i][j];
   }
 }
+constexpr int kPotrfSmem = (kNB * (kNB + 1) + 3 * kPB * (kPB + 1)) * (int)sizeof(double);
 
 // X^T of a factored diagonal block in shared memory: Xt[t][c] = X[c][t]
 // (t <= c; H's strict upper triangle of the block, 1 / L[c][c] on the
@@ -881,6 +923,7 @@ int rb_cholesky(double* H, int64_t M, int64_t ldh, void* work, size_t work_bytes
   if (work_bytes < rb_cholesky_work_bytes()) return fail(RB_EARG, "rb_cholesky: workspace too small");
   if (M > 65535 * 32) return fail(RB_ESIZE, "rb_cholesky: matrix too large");
   cudaStream_t st = as_stream(stream);
+  RB_CUDA_TRY(cudaFuncSetAttribute(potrf_diag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPotrfSmem));
   int* err = reinterpret_cast<int*>(work);
   RB_CUDA_TRY(cudaMemsetAsync(err, 0, sizeof(int), st));
   RB_CUDA_TRY(cudaFuncSetAttribute(trsm_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrsmSmem));
@@ -915,7 +958,7 @@ int rb_cholesky(double* H, int64_t M, int64_t ldh, void* work, size_t work_bytes
     const int64_t bend = std::min<int64_t>(J0 + kOuter, M);
     for (int64_t j0 = J0; j0 < bend; j0 += kNB) {
       const int nb = (int)std::min<int64_t>(kNB, M - j0);
-      potrf_diag_kernel<<<1, 256, 0, sp>>>(H, ldh, j0, nb, err);
+      potrf_diag_kernel<<<1, 256, kPotrfSmem, sp>>>(H, ldh, j0, nb, err);
       RB_LAUNCH_CHECK();
       const int64_t rest = M - j0 - nb;
       if (rest <= 0) break;

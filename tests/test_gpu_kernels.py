@@ -295,3 +295,35 @@ def test_chol_solve_segments(M, pad):
         assert torch.equal(x, xc)
     with pytest.raises(Exception, match="workspace too small"):
         solve(xs, short, M * 8 - 1)
+
+
+@pytest.mark.parametrize("M,pad", [(1, 0), (15, 1), (16, 0), (17, 0), (33, 0), (63, 0), (64, 2), (81, 0), (129, 0)])
+def test_cholesky_diagonal_block_and_its_inverse(M, pad):
+    """The 16-column steps of a diagonal block: factor and inverse (strict
+    upper triangle, transposed) at every remainder, a strided matrix, and the
+    first pivot that is not positive.  A = B B^T / M + I has condition at most
+    1 + 4 (M + 7) / M < 40, so M eps cond < M x 1e-14 bounds both."""
+    g = torch.Generator("cuda").manual_seed(M)
+    B = torch.randn((M, M + 7), generator=g, device="cuda", dtype=torch.float64)
+    A = B @ B.T / (M + 7) + torch.eye(M, device="cuda", dtype=torch.float64)
+    ld = M + pad
+
+    def factor(a):
+        H = torch.zeros((M, ld), device="cuda", dtype=torch.float64)
+        H[:, :M] = a
+        work = torch.empty(engine._lib.lib().rb_cholesky_work_bytes(), dtype=torch.uint8, device="cuda")
+        engine.call("rb_cholesky", engine.ptr(H), M, ld, engine.ptr(work), work.numel(), engine.stream())
+        return H[:, :M]
+
+    H = factor(A)
+    L = torch.linalg.cholesky(A)
+    assert float((torch.tril(H) - L).abs().max()) <= M * 1e-14 * float(L.abs().max())
+    for k in range(0, M, 64):
+        e = min(M, k + 64)
+        X = torch.linalg.inv(L[k:e, k:e])
+        assert float((torch.triu(H[k:e, k:e], 1).T - torch.tril(X, -1)).abs().max()) <= M * 1e-14 * 4
+    for p in sorted({0, M // 2, M - 1}):
+        bad = A.clone()
+        bad[p, p] = -1.0
+        with pytest.raises(Exception, match=f"at row {p}$"):
+            factor(bad)
