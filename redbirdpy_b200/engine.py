@@ -11,6 +11,7 @@ here computes on the CPU; every numerical step is a call into
 """
 
 import ctypes
+import threading
 import weakref
 import zlib
 
@@ -252,26 +253,79 @@ class PinnedPool:
     every view of that array) has been released, so an array returned to the
     caller is never overwritten.  Fresh pageable arrays cost a page fault per
     4 KB on first touch (~2 GB/s); a reused pinned buffer takes the copy at
-    PCIe speed."""
+    PCIe speed (the fields of a 3M-tet frequency-domain reconstruction, 1.07
+    GB: 460 -> 20 ms).  At most ``per_shape`` buffers of a shape and
+    ``max_bytes`` in all are kept: a new one takes the place of released ones
+    of other shapes, and a result that finds no room is copied the plain way.
+    Safe to use from several threads; ``trim`` gives released buffers back."""
 
-    def __init__(self, per_shape=3, min_bytes=1 << 20):
+    def __init__(self, per_shape=3, min_bytes=1 << 20, max_bytes=16 << 30):
         self.per_shape = per_shape
         self.min_bytes = min_bytes
-        self._slots = {}
+        self.max_bytes = max_bytes
+        self._slots = {}  # (shape, dtype) -> [[buffer, weak reference to its array, or None when free]]
+        self._lock = threading.Lock()
+
+    def trim(self, need=None):
+        """Drop released buffers: all, or until ``need`` more bytes fit."""
+        with self._lock:
+            return self._trim(need)
+
+    @staticmethod
+    def _size(nbytes):
+        """What the host allocator takes for a buffer: a power of two."""
+        return 1 << max(0, int(nbytes) - 1).bit_length()
+
+    def _bytes(self):
+        return sum(self._size(s[0].nbytes) for slots in self._slots.values() for s in slots)
+
+    def _trim(self, need):
+        used, dropped = self._bytes(), False
+        for key in list(self._slots):
+            slots = self._slots[key]
+            for slot in list(slots):
+                if need is not None and used + need <= self.max_bytes:
+                    break
+                if slot[1] is None or slot[1]() is None:
+                    used -= self._size(slot[0].nbytes)
+                    slots.remove(slot)
+                    dropped = True
+            slot = None
+            if not slots:
+                del self._slots[key]
+        if dropped and hasattr(torch._C, "_host_emptyCache"):
+            torch._C._host_emptyCache()  # the buffers go back to the system, not to the host allocator
+        return need is None or used + need <= self.max_bytes
+
+    def _take(self, t):
+        """A buffer of t's shape reserved for the caller, or None."""
+        key = (tuple(t.shape), t.dtype)
+        with self._lock:
+            slots = self._slots.get(key, [])
+            slot = next((s for s in slots if s[1] is None or s[1]() is None), None)
+            if slot is None:
+                if len(slots) >= self.per_shape or not self._trim(self._size(t.numel() * t.element_size())):
+                    return None
+                try:
+                    slot = [torch.empty(t.shape, dtype=t.dtype, pin_memory=True), None]
+                except RuntimeError:  # no page-locked memory to be had
+                    return None
+                self._slots.setdefault(key, []).append(slot)
+            slot[1] = object  # reserved until its array is known (a call gives a live object)
+            return slot
 
     def to_numpy(self, t):
-        if t.numel() * t.element_size() < self.min_bytes:
-            return t.cpu().numpy()
-        slots = self._slots.setdefault((tuple(t.shape), t.dtype), [])
-        slot = next((s for s in slots if s[1] is None or s[1]() is None), None)
+        big = t.numel() * t.element_size() >= self.min_bytes and not t.requires_grad
+        slot = self._take(t) if big else None
         if slot is None:
-            if len(slots) >= self.per_shape:  # every pooled buffer is still referenced
-                return t.cpu().numpy()
-            slot = [torch.empty(t.shape, dtype=t.dtype, pin_memory=True), None]
-            slots.append(slot)
-        slot[0].copy_(t, non_blocking=True)
-        torch.cuda.current_stream(t.device).synchronize()
-        arr = slot[0].numpy()
+            return t.cpu().numpy()
+        try:
+            slot[0].copy_(t, non_blocking=True)
+            torch.cuda.current_stream(t.device).synchronize()
+            arr = slot[0].numpy()
+        except BaseException:
+            slot[1] = None
+            raise
         slot[1] = weakref.ref(arr)
         return arr
 

@@ -530,10 +530,10 @@ def runrecon(cfg, recon, detphi0, sd=None, **kwargs):
     else:
         Jout = J[:, :K]
         if Jout.numel() * 4 < 2 ** 31:
-            Jout = Jout.float().cpu().numpy()
+            Jout = engine.host_pool.to_numpy(Jout.float())
     if len(wavelengths) == 1:
-        det_out, phi_out = dets[0].cpu().numpy(), phis[0].cpu().numpy()
+        det_out, phi_out = dets[0].cpu().numpy(), engine.host_pool.to_numpy(phis[0])
     else:
         det_out = {wv: d.cpu().numpy() for wv, d in zip(wavelengths, dets)}
-        phi_out = {wv: p.cpu().numpy() for wv, p in zip(wavelengths, phis)}
+        phi_out = {wv: engine.host_pool.to_numpy(p) for wv, p in zip(wavelengths, phis)}
     return recon, resid, cfg, updates, {"mua": Jout}, det_out, phi_out

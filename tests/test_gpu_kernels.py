@@ -327,3 +327,37 @@ def test_cholesky_diagonal_block_and_its_inverse(M, pad):
         bad[p, p] = -1.0
         with pytest.raises(Exception, match=f"at row {p}$"):
             factor(bad)
+
+
+def test_pinned_pool_is_bounded_and_thread_safe():
+    """A full pool falls back to plain copies, a released buffer makes room
+    for another shape, and threads never share a buffer."""
+    import threading
+
+    pool = engine.PinnedPool(per_shape=3, min_bytes=0, max_bytes=3 << 20)
+    ts = [torch.full((1 << 17,), float(i), device="cuda", dtype=torch.float64) for i in range(4)]
+    arrs = [pool.to_numpy(t) for t in ts]  # the fourth finds no room
+    assert pool._bytes() == 3 << 20 and all((a == i).all() for i, a in enumerate(arrs))
+    b = pool.to_numpy(torch.ones(1 << 18, device="cuda", dtype=torch.float64))
+    assert pool._bytes() == 3 << 20 and (b == 1).all()
+    del arrs[0], arrs[0]
+    c = pool.to_numpy(torch.full((1 << 18,), 7.0, device="cuda", dtype=torch.float64))
+    assert pool._bytes() == 3 << 20 and (c == 7).all() and (b == 1).all()
+    assert all((a == i + 2).all() for i, a in enumerate(arrs))
+    del arrs, c
+    pool.trim()
+    assert pool._bytes() == 0
+    bad = []
+
+    def work(k):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for i in range(20):
+                v = float(100 * k + i)
+                a = pool.to_numpy(torch.full((64, 64), v, device="cuda", dtype=torch.float64))
+                if not (a == v).all():
+                    bad.append(v)
+
+    th = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+    [t.start() for t in th]
+    [t.join() for t in th]
+    assert not bad
