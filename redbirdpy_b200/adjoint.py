@@ -86,7 +86,8 @@ class DeviceModel:
         hit = _BUDGETS.get(key)
         if hit is not None:
             return hit
-        kw = {k: v for k, v in self.solve_kw.items() if k != "budget"}
+        # Jacobi alone, as fixed-budget solves run
+        kw = dict({k: v for k, v in self.solve_kw.items() if k != "budget"}, coarse=False)
         mat = engine.assemble(self.mesh, self.optics(mua.detach(), dcoef.detach()))
         _, info = engine.solve(mat, self.B, **kw)
         if info["flag"] != 0:

@@ -2214,6 +2214,9 @@ static int solve_small(const rb_csr& A, const double* B, T64* X, int64_t k, cons
     info.outer = std::max(info.outer, c.outer);
     info.sweep_iters_max = std::max(info.sweep_iters_max, c.sweep_max);
   }
+  // in whole host checks, as the separate kernels count them: fixed budgets
+  // are made from this number
+  info.sweep_iters_max = std::min(o.maxiter, (int)ceil_div(info.sweep_iters_max, o.check_every) * o.check_every);
   info.iters += iters;
   info.flag = std::max(info.flag, flag);
   info.launches += 2;

@@ -361,3 +361,25 @@ def test_pinned_pool_is_bounded_and_thread_safe():
     [t.start() for t in th]
     [t.join() for t in th]
     assert not bad
+
+
+def test_captured_step_budget_covers_its_jacobi_solves():
+    """A captured step on a mesh whose checked solves take the V-cycle (24
+    iterations where Jacobi alone takes 130): its budget is for the solves it
+    runs, so it converges; also a batch of such instances."""
+    from redbirdpy_b200.adjoint import BatchModel, CapturedStep, DeviceModel, detector_values
+
+    cfg = _box_cfg((34, 30, 18), 2.0, 0.0, 5, 4)
+    cfgs = [_box_cfg(c, 2.0, 0.0, 4, 3) for c in ((24, 20, 12), (20, 24, 14), (28, 20, 10))]
+    for model, cs in ((DeviceModel(cfg), [cfg]), (BatchModel(cfgs), cfgs)):
+        assert model.mesh.nn >= engine.COARSE_MIN_NODES
+        prop = np.vstack([c["prop"] for c in cs])
+        mua = torch.as_tensor(prop[:, 0].copy(), device="cuda")
+        dco = torch.as_tensor(1.0 / (3.0 * (prop[:, 0] + prop[:, 1])), device="cuda")
+        with torch.no_grad():
+            ref = detector_values(model, mua, dco)
+        step = CapturedStep(model, lambda det: det.square().sum(), mua, dco)
+        det = step(mua, dco)[1].detach()
+        assert int(torch.as_tensor(step.status).max()) == 0
+        assert float((det - ref).abs().max()) <= 1e-10 * float(ref.abs().max())
+        step.release()
