@@ -382,8 +382,9 @@ int rb_femsolve(const rb_csr* A, const double* B, void* X, int64_t nrhs,
                 const rb_solve_opts* opts, rb_solve_info* info /* host */, void* work,
                 size_t work_bytes, void* stream);
 /* rb_femsolve (mixed precision) with the three-level V-cycle preconditioner:
- * opts->coarse, groups and instances must be NULL, check_every >= 1, and
- * n x (nrhs rounded up to 4) < 2^31.  work: rb_femsolve_mid_work_bytes. */
+ * opts->coarse and groups must be NULL, check_every >= 1, and n x (nrhs
+ * rounded up to 4) < 2^31.  work: rb_femsolve_mid_work_bytes, with instances
+ * plus rb_instances_work_bytes for nrhs rounded up to 4. */
 size_t rb_femsolve_mid_work_bytes(const rb_csr* A, const rb_midlevel* mid, int64_t nrhs);
 int rb_femsolve_mid(const rb_csr* A, const rb_midlevel* mid, const double* B, void* X, int64_t nrhs,
                     const rb_solve_opts* opts, rb_solve_info* info, void* work, size_t work_bytes, void* stream);

@@ -1723,10 +1723,12 @@ struct SegBufs {
   int64_t ncol = 0;        // the caller's columns (relres layout)
   double* s2 = nullptr;    // ninst x seg_parts x k partial squared norms
   OuterState* seg = nullptr;  // ninst x k
+  double* fac = nullptr;      // 2 x ninst x k: scales and reciprocals (vc_seg_factor_kernel)
 };
 static size_t seg_carve(Carver& cv, SegBufs& sb, int64_t ninst, int64_t k) {
   sb.s2 = cv.take<double>(ninst * seg_parts(ninst) * k);
   sb.seg = cv.take<OuterState>(ninst * k);
+  sb.fac = cv.take<double>(2 * ninst * k);
   return cv.used;
 }
 
@@ -2086,7 +2088,8 @@ static int solve_block(const rb_csr& A, const double* B, T64* X, int64_t ldx, in
     RB_CUDA_TRY(cudaMemsetAsync(b.counter + 1, 0, sizeof(int32_t), st));
     const double itol_min = sizeof(T) == sizeof(T64) ? o.inner_tol : std::min(o.inner_tol, 1e-6);
     if (segm) {
-      seg_norm_kernel<T64><<<sgg, kSegWarps * 32, 0, st>>>(ninst, snp, k, sb.in->row_ptr, b.R64, sb.s2);
+      if (from_b) seg_norm_kernel<double><<<sgg, kSegWarps * 32, 0, st>>>(ninst, snp, k, sb.in->row_ptr, B, sb.s2);
+      else seg_norm_kernel<T64><<<sgg, kSegWarps * 32, 0, st>>>(ninst, snp, k, sb.in->row_ptr, b.R64, sb.s2);
       seg_outer_kernel<<<sgm, 256, 0, st>>>(nseg, snp, k, sb.s2, sb.seg, o.tol, stall, o.inner_tol, itol_min);
       seg_summary_kernel<<<(unsigned)ceil_div(k, 128), 128, 0, st>>>(ninst, k, sb.seg, b.os, b.counter + 1);
       launches += 2;
@@ -2108,8 +2111,11 @@ static int solve_block(const rb_csr& A, const double* B, T64* X, int64_t ldx, in
     }
     if constexpr (sizeof(T) != sizeof(T64)) {
       if (vc) {
-        if (from_b) vc_cast_kernel<T64, double, T><<<eg, 256, 0, st>>>(n, k, B, vc->s64, b.os, b.R, b.P, b.Xs);
-        else vc_cast_kernel<T64, T64, T><<<eg, 256, 0, st>>>(n, k, b.R64, vc->s64, b.os, b.R, b.P, b.Xs);
+        if (segm) vc_seg_factor_kernel<<<sgm, 256, 0, st>>>(nseg, sb.seg, sb.fac);
+        if (from_b)
+          vc_cast_kernel<T64, double, T><<<eg, 256, 0, st>>>(n, k, B, vc->s64, b.os, rinst, sb.fac, b.R, b.P, b.Xs);
+        else
+          vc_cast_kernel<T64, T64, T><<<eg, 256, 0, st>>>(n, k, b.R64, vc->s64, b.os, rinst, sb.fac, b.R, b.P, b.Xs);
         RB_LAUNCH_CHECK();
         int it = 0;
         RB_TRY((vc_inner<T64, T>(A, vc->op, k, b.part_a, b.part_b, b.Xs, b.R, b.P, b.Q, b.cs, b.os, b.counter,
@@ -2117,7 +2123,8 @@ static int solve_block(const rb_csr& A, const double* B, T64* X, int64_t ldx, in
         total_iters += it;
         info.sweep_iters_max = std::max(info.sweep_iters_max, it);
         if (it >= o.maxiter) sweep_flag = 1;
-        vc_correct_kernel<T64, T><<<eg, 256, 0, st>>>(n, k, b.Xs, vc->s64, b.os, X);
+        vc_correct_kernel<T64, T><<<eg, 256, 0, st>>>(n, k, b.Xs, vc->s64, b.os, rinst,
+                                                      segm ? sb.fac + nseg : nullptr, X);
         RB_LAUNCH_CHECK();
         launches += 2;
         continue;
@@ -2268,7 +2275,7 @@ static int femsolve_t(const rb_csr& A, const double* B, T64* X, int64_t nrhs, co
     sb.in = o.instances;
     sb.ncol = nrhs;
     seg_carve(cv, sb, o.instances->ninst, kb);
-    if (!sb.s2 || !sb.seg) return fail(RB_EARG, "rb_femsolve: workspace too small for the instances");
+    if (!sb.s2 || !sb.seg || !sb.fac) return fail(RB_EARG, "rb_femsolve: workspace too small for the instances");
   }
   RB_CUDA_TRY(cudaMemsetAsync(b.counter, 0, 8 * sizeof(int32_t), st));
   if (o.coarse) {
@@ -2457,7 +2464,7 @@ int rb_femsolve_mid(const rb_csr* A, const rb_midlevel* mid, const double* B, vo
   if (nrhs < 1 || A->n < 1) return fail(RB_EARG, "rb_femsolve_mid: empty system");
   if (nrhs > kMaxCols) return fail(RB_ESIZE, "rb_femsolve_mid: at most %lld right-hand sides per call", (long long)kMaxCols);
   const rb_solve_opts& o = *opts;
-  if (o.precision != RB_MIXED || o.coarse || o.groups || o.instances || o.check_every < 1 || o.maxiter < 1 ||
+  if (o.precision != RB_MIXED || o.coarse || o.groups || o.check_every < 1 || o.maxiter < 1 ||
       o.max_outer < 1 || !(o.tol > 0) || !(o.inner_tol > 0))
     return fail(RB_EARG, "rb_femsolve_mid: bad options");
   if (!A->val64 || !A->dinv64 || !A->val32 || !A->dinv32 || !A->indptr || !A->indices)
@@ -2468,7 +2475,14 @@ int rb_femsolve_mid(const rb_csr* A, const rb_midlevel* mid, const double* B, vo
       mid->nnz1 < 1 || !c || c->nc < 1 || c->nc > kCoarseMax || c->nc > g->ng || !c->agg || !c->agg_ptr || !c->agg_rows)
     return fail(RB_EARG, "rb_femsolve_mid: incomplete level");
   if (A->n * vc_cols(nrhs) >= (int64_t(1) << 31)) return fail(RB_ESIZE, "rb_femsolve_mid: n x columns above 2^31");
-  if (work_bytes < rb_femsolve_mid_work_bytes(A, mid, nrhs)) return fail(RB_EARG, "rb_femsolve_mid: workspace too small");
+  size_t need = rb_femsolve_mid_work_bytes(A, mid, nrhs);
+  if (o.instances) {
+    const rb_instances& in = *o.instances;
+    if (in.ninst < 1 || !in.row_ptr || !in.row_inst || !in.status)
+      return fail(RB_EARG, "rb_femsolve_mid: instances need ninst >= 1, row_ptr, row_inst and status");
+    need += rb_instances_work_bytes(in.ninst, vc_cols(nrhs));
+  }
+  if (work_bytes < need) return fail(RB_EARG, "rb_femsolve_mid: workspace too small");
   *info = rb_solve_info{};
   cudaStream_t st = as_stream(stream);
   if (A->is_complex)

@@ -737,34 +737,48 @@ vc_beta_kernel(int64_t k, int nbt, const A* part_t, int nbe, const A* part_e, co
 }
 
 // ------------------------------------------------ scaled residual, correction
-// the columns' factors in shared memory: scale, or its reciprocal (one
-// division per block and column instead of one per entry), 0 when not active
+// Column factors: scale or its reciprocal, 0 where not active (one division
+// per block and column instead of one per entry).  With stacked instances
+// they are per (instance, column), read from a table made for the sweep.
+template <bool INV>
+__device__ __forceinline__ double vc_factor(const OuterState& o) { return o.active ? (INV ? 1.0 / o.scale : o.scale) : 0.0; }
 template <bool INV>
 __device__ __forceinline__ void vc_factors(int64_t k, const OuterState* __restrict__ os, double* f) {
-  for (int c = threadIdx.x; c < k; c += blockDim.x)
-    f[c] = os[c].active ? (INV ? 1.0 / os[c].scale : os[c].scale) : 0.0;
+  for (int c = threadIdx.x; c < k; c += blockDim.x) f[c] = vc_factor<INV>(os[c]);
   __syncthreads();
 }
 
+// factors of every (instance, column): fac[j] the scale, fac[m + j] its reciprocal
+__global__ void vc_seg_factor_kernel(int64_t m, const OuterState* __restrict__ seg, double* __restrict__ fac) {
+  const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (j >= m) return;
+  fac[j] = vc_factor<false>(seg[j]);
+  fac[m + j] = vc_factor<true>(seg[j]);
+}
+
 // r^ = T(S R64 scale) for active columns, 0 elsewhere; x = p = 0.  RT: the
-// residual's type (double for the right-hand side of a first sweep from 0)
+// residual's type (double for the right-hand side of a first sweep from 0);
+// rinst / segf: the rows' instances and their factors, or NULL
 template <typename T64, typename RT, typename T>
 __global__ void __launch_bounds__(256)
 vc_cast_kernel(int64_t n, int64_t k, const RT* __restrict__ R64, const T64* __restrict__ s64,
-               const OuterState* __restrict__ os, T* __restrict__ R, T* __restrict__ P, T* __restrict__ Xs) {
+               const OuterState* __restrict__ os, const int32_t* __restrict__ rinst, const double* __restrict__ segf,
+               T* __restrict__ R, T* __restrict__ P, T* __restrict__ Xs) {
   constexpr int V = 16 / (int)sizeof(T);
   __shared__ double fac[kMaxCols];
-  vc_factors<false>(k, os, fac);
+  if (!rinst) vc_factors<false>(k, os, fac);
   const int64_t kv = k / V;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n * kv; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t row = i / kv, c = (i - row * kv) * V;
+    const double* f = rinst ? segf + (int64_t)rinst[row] * k + c : fac + c;
     const T64 s = s64[row];
     alignas(16) RT v[V];
     alignas(16) T o[V], z[V];
     ldv<RT, V>(R64 + row * k + c, v);
 #pragma unroll
     for (int q = 0; q < V; ++q) {
-      o[q] = narrow_to<T>(r_mul(fac[c + q], cs_mul(s, v[q])));
+      const double fq = f[q];  // (a done column's residual may be non-finite: 0, not 0 x it)
+      o[q] = fq != 0.0 ? narrow_to<T>(r_mul(fq, cs_mul(s, v[q]))) : s_zero(T());
       z[q] = s_zero(T());
     }
     stv<T, V>(R + row * k + c, o);
@@ -773,17 +787,19 @@ vc_cast_kernel(int64_t n, int64_t k, const RT* __restrict__ R64, const T64* __re
   }
 }
 
-// X64 += S x^ / scale for active columns (an inactive one's x^ is 0)
+// X64 += S x^ / scale for active columns
 template <typename T64, typename T>
 __global__ void __launch_bounds__(256)
 vc_correct_kernel(int64_t n, int64_t k, const T* __restrict__ D, const T64* __restrict__ s64,
-                  const OuterState* __restrict__ os, T64* __restrict__ X) {
+                  const OuterState* __restrict__ os, const int32_t* __restrict__ rinst,
+                  const double* __restrict__ segf, T64* __restrict__ X) {
   constexpr int V = 16 / (int)sizeof(T);
   __shared__ double fac[kMaxCols];
-  vc_factors<true>(k, os, fac);
+  if (!rinst) vc_factors<true>(k, os, fac);
   const int64_t kv = k / V;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n * kv; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t row = i / kv, c = (i - row * kv) * V;
+    const double* f = rinst ? segf + (int64_t)rinst[row] * k + c : fac + c;
     const T64 s = s64[row];
     alignas(16) T64 x[V];
     alignas(16) T d[V];
@@ -792,8 +808,10 @@ vc_correct_kernel(int64_t n, int64_t k, const T* __restrict__ D, const T64* __re
     for (int q = 0; q < V; ++q) x[q] = xp[q];
     ldv<T, V>(D + row * k + c, d);
 #pragma unroll
-    for (int q = 0; q < V; ++q)
-      if (fac[c + q] != 0.0) x[q] = s_add(x[q], r_mul(fac[c + q], s_mul(s, widen(d[q]))));
+    for (int q = 0; q < V; ++q) {
+      const double fq = f[q];
+      if (fq != 0.0) x[q] = s_add(x[q], r_mul(fq, s_mul(s, widen(d[q]))));
+    }
     stv<T64, V>(xp, x);
   }
 }

@@ -51,6 +51,7 @@ class DeviceMesh:
         self._coarse = {}
         self._groups = None
         self._mid = False  # not built yet
+        self.layout = None  # (positions, bbox, edge) for the groups, where not the nodes' own
         self._edge = None
         if self.ne:
             sel = np.arange(0, self.ne, max(1, self.ne // 65536))
@@ -157,9 +158,10 @@ class DeviceMesh:
         """The RowGroups of the blocked SpMM (built once), or None when the
         mesh has no usable edge length (e.g. a topology-only mesh)."""
         if self._groups is None:
-            if not self._edge or not np.isfinite(self._edge) or self._edge <= 0:
+            edge = self._edge if self.layout is None else self.layout[2]
+            if not edge or not np.isfinite(edge) or edge <= 0:
                 return None
-            self._groups = RowGroups(self, self._edge)
+            self._groups = RowGroups(self, edge)
         return self._groups
 
     def mid_level(self):
@@ -651,7 +653,7 @@ class RowGroups:
     def __init__(self, mesh, edge):
         dev = mesh.device
         nn = mesh.nn
-        lo, hi = mesh.bbox
+        node, (lo, hi) = (mesh.node, mesh.bbox) if mesh.layout is None else mesh.layout[:2]
         if not (np.isfinite(edge) and edge > 0 and np.all(np.isfinite(lo)) and np.all(np.isfinite(hi))):
             raise ValueError("row groups: degenerate mesh geometry")
         h = 2.0 * edge
@@ -665,7 +667,7 @@ class RowGroups:
         ng = ctypes.c_int64(0)
         wb = _lib.lib().rb_rowgroups_work_bytes(nn, int(np.prod(nb)))
         work = torch.empty(wb, dtype=torch.uint8, device=dev)
-        call("rb_rowgroups_bin", ptr(mesh.node), nn, float(x0[0]), float(x0[1]), float(x0[2]), h, int(nb[0]),
+        call("rb_rowgroups_bin", ptr(node), nn, float(x0[0]), float(x0[1]), float(x0[2]), h, int(nb[0]),
              int(nb[1]), int(nb[2]), ptr(self.rows), ctypes.byref(ng), ptr(work), wb, stream())
         self.ng = int(ng.value)
         csr = _lib.RbCsr(nn, mesh.nnz, mesh.indptr.data_ptr(), mesh.indices.data_ptr(), None, None, None, None, 0)
@@ -702,8 +704,9 @@ class _GroupNodes:
     per group (its first node's)."""
 
     def __init__(self, mesh, rg):
-        self.device, self.bbox, self.nn = mesh.device, mesh.bbox, rg.ng
-        self.node = mesh.node[rg.rows[: 8 * rg.ng].view(rg.ng, 8)[:, 0].long()].contiguous()
+        node, self.bbox = (mesh.node, mesh.bbox) if mesh.layout is None else mesh.layout[:2]
+        self.device, self.nn = mesh.device, rg.ng
+        self.node = node[rg.rows[: 8 * rg.ng].view(rg.ng, 8)[:, 0].long()].contiguous()
 
 
 class MidLevel:
@@ -724,21 +727,27 @@ class MidLevel:
         self.nnz1 = int(nnz1.value)
         self.mcol = torch.empty(max(self.nnz1, 1), dtype=torch.int32, device=dev)
         call("rb_midlevel_fill", ctypes.byref(rg.struct), ptr(self.grp), ptr(self.mptr), ptr(self.mcol), stream())
-        self.coarse = CoarseSpace(_GroupNodes(mesh, rg), mid_coarse_target(rg.ng))
+        # (a layout of instances side by side leaves about half the cells empty)
+        target = mid_coarse_target(rg.ng) * (1 if mesh.layout is None else 2)
+        self.coarse = CoarseSpace(_GroupNodes(mesh, rg), target)
         self.struct = _lib.RbMidlevel(ctypes.pointer(rg.struct), self.grp.data_ptr(), self.mptr.data_ptr(),
                                       self.mcol.data_ptr(), self.nnz1, ctypes.pointer(self.coarse.struct))
 
 
 def _resolve_mid(mat, n, k, prec, coarse, groups, instances, budget):
-    """The MidLevel a solve takes, or None: with every choice left to the
-    engine ('auto'), a mixed-precision solve of one system assembled on a
-    mesh of at least COARSE_MIN_NODES nodes."""
-    if coarse != "auto" or groups != "auto" or prec != _lib.RB_MIXED or instances is not None or budget is not None:
+    """The MidLevel a solve takes, or None: a mixed-precision solve on a mesh
+    of at least COARSE_MIN_NODES nodes with every choice left to the engine
+    ('auto'), or of stacked instances ('blocks') whose mesh has a layout that
+    keeps their groups apart."""
+    if groups != "auto" or prec != _lib.RB_MIXED or budget is not None:
         return None
     mesh = getattr(mat, "mesh", None)
     if not hasattr(mesh, "mid_level") or n < COARSE_MIN_NODES or n * (min(k, 128) + 4) >= 2 ** 31:
         return None
-    return mesh.mid_level()
+    if (coarse == "auto" and instances is None) or (coarse == "blocks" and instances is not None
+                                                    and mesh.layout is not None):
+        return mesh.mid_level()
+    return None
 
 
 def _resolve_groups(mat, groups):
@@ -760,7 +769,7 @@ def _resolve_coarse(mat, coarse):
     """CoarseSpace for solve(coarse=...): 'auto' (meshes of at least
     COARSE_MIN_NODES nodes), True, an aggregate count, a CoarseSpace, or
     None/False for Jacobi only."""
-    if coarse is None or coarse is False:
+    if coarse is None or coarse is False or (isinstance(coarse, str) and coarse == "blocks"):
         return None
     if isinstance(coarse, CoarseSpace):
         return coarse
@@ -831,6 +840,8 @@ class SolveTuner:
         if hit is not None:
             return hit
         kw = {k: v for k, v in kw.items() if k not in ("spmm_lanes", "check_every", "profile", "budget")}
+        if kw.get("coarse") == "blocks":
+            kw["coarse"] = False  # (the shapes are the separate kernels', which fixed budgets run)
         cands = [dict(spmm_lanes=lanes, check_every=c) for lanes in self.LANES for c in self.CHECKS]
         solve(mat, B, **kw, **cands[0])  # warm-up: first launches, plans, caches
         best, times = None, {}
@@ -881,7 +892,8 @@ def solve(mat, B, precision="mixed", tol=DEFAULT_TOL, inner_tol=None, maxiter=20
     With ``coarse`` and ``groups`` left at 'auto', a mixed-precision solve on a
     mesh of 20000 nodes or more takes the three-level V-cycle preconditioner
     (MidLevel; a solve that it does not bring to convergence is redone with
-    the two-level form).  ``coarse`` otherwise adds the aggregation coarse
+    the two-level form); ``coarse='blocks'`` with ``instances`` asks the same of
+    a batch (Jacobi alone where it does not apply).  ``coarse`` otherwise adds the aggregation coarse
     space to the Jacobi preconditioner (see _resolve_coarse).
     ``inner_tol`` (relative residual of each FP32 correction sweep) defaults to
     1e-5 with a coarse space and 1e-4 without: on the 520k-node box at 128
@@ -942,6 +954,8 @@ def solve(mat, B, precision="mixed", tol=DEFAULT_TOL, inner_tol=None, maxiter=20
         inf = _lib.RbSolveInfo()
         if mid is not None:
             wb = _lib.lib().rb_femsolve_mid_work_bytes(ctypes.byref(mat.struct), ctypes.byref(mid.struct), kb)
+            if instances is not None:
+                wb += _lib.lib().rb_instances_work_bytes(instances.ninst, (kb + 3) // 4 * 4)
             try:
                 work = torch.empty(wb, dtype=torch.uint8, device=B.device)
             except torch.cuda.OutOfMemoryError:
@@ -963,6 +977,9 @@ def solve(mat, B, precision="mixed", tol=DEFAULT_TOL, inner_tol=None, maxiter=20
             if Xb is not X:
                 X[:, c0:c0 + kb] = Xb
             _add_info(info, inf)
+            if instances is not None:
+                inst_status.append(instances.status.cpu().numpy())
+                inst_relres.append(rel)
             continue
         wb = _lib.lib().rb_femsolve_work_bytes(n, mat.struct.nnz, kb, int(mat.is_complex), prec)
         if cs is not None:

@@ -383,3 +383,35 @@ def test_captured_step_budget_covers_its_jacobi_solves():
         assert int(torch.as_tensor(step.status).max()) == 0
         assert float((det - ref).abs().max()) <= 1e-10 * float(ref.abs().max())
         step.release()
+
+
+@pytest.mark.parametrize("omega", [0.0, 2 * np.pi * 1e8])
+def test_batch_vcycle_equals_jacobi(omega):
+    """Stacked instances of unequal spacing and scale (one with D 1000 times
+    smaller, one with fewer optodes, so zero columns): the V-cycle's fields
+    against Jacobi's, per instance; statuses; a solve cut short reports every
+    instance; a batch of small instances keeps Jacobi alone."""
+    from redbirdpy_b200.adjoint import BatchModel
+
+    cfgs = [_box_cfg(c, h, omega, ns, 2) for c, h, ns in
+            (((24, 20, 12), 1.0, 3), ((20, 24, 14), 3.0, 5), ((28, 20, 10), 2.0, 1), ((19, 21, 11), 0.5, 5))]
+    bm = BatchModel(cfgs)
+    assert bm.solve_kw["coarse"] == "blocks" and bm.mesh.layout is not None
+    prop = np.vstack([c["prop"] for c in cfgs])
+    mua = torch.as_tensor(prop[:, 0].copy(), device="cuda")
+    dco = torch.as_tensor(1.0 / (3.0 * (prop[:, 0] + prop[:, 1])), device="cuda")
+    dco[int(bm.node_off[1]):int(bm.node_off[2])] *= 1e-3
+    mat = engine.assemble(bm.mesh, bm.optics(mua, dco))
+    X, info = engine.solve(mat, bm.B, **bm.solve_kw)
+    assert info["spmm_kernel"] == "vc_spmm_kernel" and info["flag"] == 0 and not info["inst_status"].any()
+    Y, inf2 = engine.solve(mat, bm.B, **dict(bm.solve_kw, coarse=False))
+    assert inf2["spmm_kernel"] != "vc_spmm_kernel" and not inf2["inst_status"].any()
+    assert info["inst_relres"].shape == (4, bm.B.shape[1]) and info["inst_relres"].max() <= 1e-14
+    for a, b in zip(bm.node_slices(X), bm.node_slices(Y)):
+        assert float((a - b).abs().max()) <= 1e-10 * float(b.abs().max())
+    assert float(X[int(bm.node_off[2]):int(bm.node_off[3]), 1:5].abs().max()) == 0.0
+    _, short = engine.solve(mat, bm.B, **dict(bm.solve_kw, maxiter=2, max_outer=1))
+    assert short["flag"] == 1 and (short["inst_status"] == 1).all()
+    small = BatchModel([_box_cfg((14, 12, 8), 2.0, omega, 3, 2) for _ in range(12)])
+    assert small.mesh.nn >= engine.COARSE_MIN_NODES and small.solve_kw["coarse"] is False
+    assert small.mesh.layout is None
