@@ -5,7 +5,7 @@
 // (up to 8 neighbouring nodes each, P1 their 0/1 membership); aggregates of
 // the groups (P2, at most kCoarseMax), whose operator is inverted densely.
 // Every level is scaled to a unit diagonal, A^ = S A S with S = D^-1/2, so the
-// Jacobi smoother is a number: with w = 1.6 / (Gershgorin bound of D^-1 A),
+// Jacobi smoother is a number: with w = 1.7 / (Gershgorin bound of D^-1 A),
 // below 2 / lambda_max, so that the cycle stays positive definite (real) or
 // symmetric (complex), one application of the symmetric cycle to r^ is
 //   t = A^ r^,  f = P1^T S^-1 (r^ - w t),  e = M1 f,
@@ -183,16 +183,19 @@ vc_values_kernel(int64_t n, const int32_t* __restrict__ indptr, const int32_t* _
   if ((threadIdx.x & 31) == 0) atomicMax(bound, m);
 }
 
-// smoother parameters from the bounds g: fine w = 1.6 / g; group level the
-// degree-2 Chebyshev polynomial of [g / 8, g] (Saad, Iterative Methods for
-// Sparse Linear Systems, section 12.3) written as a - b A^
+// smoother parameters from the bounds g: fine w = 1.7 / g; group level the
+// degree-2 Chebyshev polynomial of [g / 16, g] (Saad, Iterative Methods for
+// Sparse Linear Systems, section 12.3) written as a - b A^.  Iterations at
+// w g / (bound over lower end) 1.6 / 8, 1.7 / 16, 1.9 / 16: regular boxes, whose
+// bound is tight, 24, 22, 36 (43k nodes) and 32, 30, 39 (520k); displaced
+// nodes, whose bound is a fifth too large, 26, 25, 24 and 41, 38, 38.
 __global__ void vc_param_kernel(VcPar* __restrict__ p) {
   const float g0 = __uint_as_float(p->g[0]), g1 = __uint_as_float(p->g[1]);
-  p->w = 1.6f / g0;
+  p->w = 1.7f / g0;
   p->w2 = p->w * p->w;
   p->one = 1.f;
   p->mone = -1.f;
-  const double hi = g1, lo = hi / 8.0, th = 0.5 * (hi + lo), de = 0.5 * (hi - lo), sg = th / de;
+  const double hi = g1, lo = hi / 16.0, th = 0.5 * (hi + lo), de = 0.5 * (hi - lo), sg = th / de;
   const double r0 = 1.0 / sg, r1 = 1.0 / (2.0 * sg - r0);
   p->a = (float)((1.0 + r1 * r0) / th + 2.0 * r1 / de);
   p->b = (float)(2.0 * r1 / (de * th));
