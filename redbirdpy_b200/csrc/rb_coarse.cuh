@@ -156,53 +156,64 @@ __device__ __forceinline__ double s_neg(double a) { return -a; }
 __device__ __forceinline__ cdouble s_neg(cdouble a) { return make_double2(-a.x, -a.y); }
 
 // ------------------------------------------- Gauss-Jordan on one 64-block
-// Dinv = (A[b0.., b0..])^-1 for the nb x nb diagonal block.  Two copies of
-// the block in shared memory: pivot step c reads one and writes the other
-// (one barrier per pivot).  Thread t owns column t % 64 of rows t / 64 + 4 u.
-constexpr int kGjLd = kGjB + 1;
-template <typename T>
-constexpr size_t gj_smem_bytes() { return sizeof(T) * 2 * kGjB * kGjLd; }
-
+// Dinv = (A[b0.., b0..])^-1 for the nb x nb diagonal block.  Bound: the chain
+// of 64 pivots (a read, a reciprocal, a product, an update each).  A thread
+// keeps column t % 64 of rows t / 64 + 4 u in registers; only the next pivot's
+// row and column pass through shared memory, one barrier per pivot.  With two
+// copies of the block in shared memory, each entry read and written per pivot,
+// it took 56 us (complex 88), now 27 (63).
 template <typename T>
 __global__ void __launch_bounds__(256) gj_diag_kernel(const T* __restrict__ A, int64_t lda, int64_t b0, int nb,
                                                       T* __restrict__ Dinv, int* __restrict__ err) {
-  extern __shared__ __align__(16) unsigned char gsm[];
-  T* cur = reinterpret_cast<T*>(gsm);
-  T* nxt = cur + kGjB * kGjLd;
+  constexpr int R = kGjB / 4;  // rows of a thread
+  __shared__ __align__(16) T row[2][kGjB], col[2][4][R];
   const int tid = threadIdx.x;
   const int j = tid & (kGjB - 1), ib = tid / kGjB;
+  T a[R];
 #pragma unroll
-  for (int u = 0; u < kGjB / 4; ++u) {
+  for (int u = 0; u < R; ++u) {
     const int i = ib + 4 * u;
-    cur[i * kGjLd + j] = (i < nb && j < nb) ? A[(b0 + i) * lda + b0 + j] : s_zero(T());
+    a[u] = (i < nb && j < nb) ? A[(b0 + i) * lda + b0 + j] : s_zero(T());
+  }
+  if (ib == 0) row[0][j] = a[0];
+  if (j == 0) {
+#pragma unroll
+    for (int u = 0; u < R; ++u) col[0][ib][u] = a[u];
   }
   __syncthreads();
-  for (int c = 0; c < nb; ++c) {
-    const T piv = cur[c * kGjLd + c];
-    if (s_bad(piv)) {  // uniform: every thread reads the same pivot
-      if (tid == 0) atomicExch(err, 1);
-      return;
-    }
-    const T ip = s_inv(piv);
-    const T rcj = s_mul(cur[c * kGjLd + j], ip);  // scaled pivot row
 #pragma unroll
-    for (int u = 0; u < kGjB / 4; ++u) {
-      const int i = ib + 4 * u;
-      const T mic = cur[i * kGjLd + c];
-      T v;
-      if (i == c) v = (j == c) ? ip : rcj;
-      else v = (j == c) ? s_neg(s_mul(mic, ip)) : s_sub(cur[i * kGjLd + j], s_mul(mic, rcj));
-      nxt[i * kGjLd + j] = v;
+  for (int u0 = 0; u0 < R; ++u0) {
+#pragma unroll 1
+    for (int r = 0; r < 4; ++r) {
+      const int c = 4 * u0 + r, buf = c & 1;
+      if (c >= nb) break;
+      const T piv = row[buf][c];
+      if (s_bad(piv)) {  // uniform: every thread reads the same pivot
+        if (tid == 0) atomicExch(err, 1);
+        return;
+      }
+      const T ip = s_inv(piv);
+      const T rcj = s_mul(row[buf][j], ip);  // scaled pivot row
+#pragma unroll
+      for (int u = 0; u < R; ++u) {
+        const T mic = col[buf][ib][u];
+        if (u == u0 && ib == r) a[u] = (j == c) ? ip : rcj;
+        else a[u] = (j == c) ? s_neg(s_mul(mic, ip)) : s_sub(a[u], s_mul(mic, rcj));
+      }
+      if (c + 1 < nb) {  // the next pivot's row and column
+        if (ib == ((r + 1) & 3)) row[buf ^ 1][j] = r == 3 ? a[u0 + 1 < R ? u0 + 1 : u0] : a[u0];
+        if (j == c + 1) {
+#pragma unroll
+          for (int u = 0; u < R; ++u) col[buf ^ 1][ib][u] = a[u];
+        }
+      }
+      __syncthreads();
     }
-    __syncthreads();
-    T* t = cur;
-    cur = nxt;
-    nxt = t;
   }
 #pragma unroll
-  for (int u = 0; u < kGjB / 4; ++u) {
+  for (int u = 0; u < R; ++u) {
     const int i = ib + 4 * u;
-    Dinv[i * kGjB + j] = (i < nb && j < nb) ? cur[i * kGjLd + j] : s_zero(T());
+    Dinv[i * kGjB + j] = (i < nb && j < nb) ? a[u] : s_zero(T());
   }
 }
 
@@ -435,11 +446,9 @@ static int coarse_setup(const rb_csr& A, CoarseBufs<T64, T>& c, cudaStream_t st)
   RB_CUDA_TRY(cudaMemsetAsync(c.err, 0, sizeof(int), st));
   const T64 one = h_real<T64>(1.0), mone = h_real<T64>(-1.0), zero = h_real<T64>(0.0);
   const unsigned eg = (unsigned)std::min<int64_t>(ceil_div(nc * kGjB, 256), 148 * 8);
-  constexpr size_t gj_smem = gj_smem_bytes<T64>();
-  RB_CUDA_TRY(cudaFuncSetAttribute(gj_diag_kernel<T64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gj_smem));
   for (int64_t b0 = 0; b0 < nc; b0 += kGjB) {
     const int nb = (int)std::min<int64_t>(kGjB, nc - b0);
-    gj_diag_kernel<T64><<<1, 256, gj_smem, st>>>(c.A64, nc, b0, nb, c.Dinv, c.err);
+    gj_diag_kernel<T64><<<1, 256, 0, st>>>(c.A64, nc, b0, nb, c.Dinv, c.err);
     RB_LAUNCH_CHECK();
     // R = Dinv A[b, :]  (Dinv is symmetric: the inverse of a diagonal block
     // of the symmetric Schur complement, so it serves as its own transpose)
@@ -476,10 +485,12 @@ static int coarse_apply(const CoarseOp<T>& c, const T* R, int64_t k, cudaStream_
     RB_LAUNCH_CHECK();
   }
   // enough blocks for two per SM: split the nc-long sums (fixed order, no atomics)
+  // in pieces of 64 or more (at nc = 250, k = 37 an unsplit product took 9.8 us
+  // in 4 blocks, 4 pieces take 4.4; complex at nc = 1183, k = 128 50 -> 37)
   const T one = h_real<T>(1.0), zero = h_real<T>(0.0);
   const int64_t tiles = ceil_div(nc, 64) * ceil_div(k, gemm_bn<T>());
   const int splits = (int)std::max<int64_t>(1, std::min<int64_t>({kCoarseSplits, ceil_div(2 * 148, tiles),
-                                                                   ceil_div(nc, 256)}));
+                                                                   ceil_div(nc, 64)}));
   RB_TRY(gemm_tn<T>(nc, k, nc, one, c.X, nc, c.rc, k, zero, true, c.es, k, st, splits, nc * k, live));
   coarse_dot_kernel<T><<<kCdotGrid, 256, 0, st>>>(nc, k, c.rc, c.es, splits, c.ec, (typename Scalar<T>::acc*)c.part,
                                                   live);

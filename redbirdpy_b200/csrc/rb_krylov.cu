@@ -2299,7 +2299,7 @@ static int femsolve_t(const rb_csr& A, const double* B, T64* X, int64_t nrhs, co
       vb.cb.op.agg = mid->coarse->agg;
       vb.cb.op.agg_ptr = mid->coarse->agg_ptr;
       vb.cb.op.agg_rows = mid->coarse->agg_rows;
-      RB_TRY((vc_setup<T64, T>(A, *mid, vb, st)));
+      RB_TRY((vc_setup<T64, T>(A, *mid, vb, vc_groups<T>(vc_grids<T>(n, g.ng, kb)), st)));
       info.launches += 12 + 5 * (int)ceil_div(vb.cb.op.nc, kGjB);
     }
   }

@@ -842,7 +842,7 @@ static VcGrids vc_grids(int64_t n, int64_t ng, int64_t k) {
 
 // the matrix-dependent part: scaled values, group-level matrix, its dense inverse
 template <typename T64, typename T>
-static int vc_setup(const rb_csr& A, const rb_midlevel& mid, VcBufs<T64, T>& b, cudaStream_t st) {
+static int vc_setup(const rb_csr& A, const rb_midlevel& mid, VcBufs<T64, T>& b, bool groups, cudaStream_t st) {
   VcOp<T>& o = b.op;
   const T64* val = (const T64*)A.val64;
   const T64* dinv = (const T64*)A.dinv64;
@@ -853,7 +853,7 @@ static int vc_setup(const rb_csr& A, const rb_midlevel& mid, VcBufs<T64, T>& b, 
   vc_values_kernel<T64, T><<<(unsigned)std::min<int64_t>(ceil_div(A.n, 16), 148 * 32), 256, 0, st>>>(
       A.n, A.indptr, A.indices, val, dinv, b.s64, o.vs, &o.par->g[0]);
   RB_LAUNCH_CHECK();
-  RB_TRY(rg_fill_coef<T>(A, o.vs, o.rg, st));
+  if (groups) RB_TRY(rg_fill_coef<T>(A, o.vs, o.rg, st));  // (read by vc_spmm_kernel alone)
   vc_mid_kernel<T64, T><<<(unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(o.ng, kMidWarps), 148 * 64)),
                           kMidWarps * 32, 0, st>>>(o.ng, o.rg.rows, A.indptr, A.indices, val, mid.grp, o.mptr, o.mcol,
                                                    b.s64, b.val1, o.cm);
