@@ -33,6 +33,35 @@ int fail(int code, const char* fmt, ...);
     if (s_ != RB_OK) return s_;      \
   } while (0)
 
+// Chains of short kernels: a kernel launched with launch_early may be scheduled
+// while its predecessor in the stream still runs (programmatic stream
+// serialization), which hides the gap of a microsecond or two between them.
+// Such a kernel calls chain_wait() before it touches memory: it returns once
+// the predecessor has ended and its writes are visible, and since that one
+// waited too, so have all before it.  The call also lets the next kernel be
+// scheduled.  Without the launch attribute it does nothing.
+__device__ __forceinline__ void chain_wait() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+// the live-column count of an iteration's kernels (written by an earlier one)
+__device__ __forceinline__ bool chain_dead(const int32_t* live) {
+  return live && *reinterpret_cast<const volatile int32_t*>(live) == 0;
+}
+template <typename... P, typename... A>
+inline cudaError_t launch_early(bool early, void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t st, A... a) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = early ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(a)...);
+}
+
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
 constexpr int kWarp = 32;

@@ -151,7 +151,8 @@ __global__ void __launch_bounds__(kBlk, BpsSpmm<T>::value)
 spmm_kernel(int64_t n, int64_t k, const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices,
             const T* __restrict__ val, const T* __restrict__ X, T* __restrict__ Y,
             const double* __restrict__ B, void* __restrict__ part_, const int32_t* __restrict__ live) {
-  if (live && *live == 0) return;  // every column converged: a no-op iteration
+  chain_wait();
+  if (chain_dead(live)) return;  // every column converged: a no-op iteration
   // residual norms accumulate |r|^2 in double; dot products in the acc type
   typedef std::conditional_t<EPI == EPI_RESID, double, typename Scalar<T>::acc> A;
   A* part = reinterpret_cast<A*>(part_);
@@ -640,7 +641,8 @@ __global__ void __launch_bounds__(kBlk, BpsSpmm<T>::value)
 spmm_pair_kernel(int64_t n, int64_t k, const int32_t* __restrict__ indptr, const T* __restrict__ val, GroupPlan gp,
                  const T* __restrict__ X, T* __restrict__ Y, void* __restrict__ part_,
                  const int32_t* __restrict__ live) {
-  if (live && *live == 0) return;  // every column converged: a no-op iteration
+  chain_wait();
+  if (chain_dead(live)) return;  // every column converged: a no-op iteration
   constexpr int V = PairCfg<T>::V, S = PairCfg<T>::S, U = 8;
   typedef typename Scalar<T>::acc A;
   static_assert(EPI == EPI_PQDOT, "row-pair SpMM: p.Ap epilogue only");
@@ -1137,6 +1139,7 @@ __device__ __forceinline__ cdouble block_sum_part(const A* __restrict__ part, in
 template <typename A>
 __global__ void __launch_bounds__(kFinThreads) fin_alpha_kernel(int64_t k, int nb, const A* part_pq, ColState* cs,
                                                                int32_t* __restrict__ clear) {
+  chain_wait();
   if (clear && blockIdx.x == 0 && threadIdx.x == 0) *clear = 0;
   const int64_t c = blockIdx.x;
   if (c >= k) return;
@@ -1591,30 +1594,31 @@ static Shape pick_spmm_shape(int64_t n, int64_t k) {
 // Krylov loop)
 template <typename T, int EPI>
 int spmm_t(const rb_csr& A, const T* val, const T* X, T* Y, const double* B, void* part, int64_t k,
-           const Shape& sh, cudaStream_t st, const int32_t* live = nullptr) {
+           const Shape& sh, cudaStream_t st, const int32_t* live = nullptr, bool early = false) {
   const bool o32 = (uint64_t)A.n * (uint64_t)k < (1ull << 31);
   if (sh.S == 2) {
     if (sh.L != 32 || sh.V != 2 || k != 128) return fail(RB_EARG, "bad sliced SpMM shape");
     if (o32)
-      spmm_kernel<T, 32, 2, EPI, 2, true><<<sh.grid, kBlk, 0, st>>>(A.n, k, A.indptr, A.indices, val, X, Y, B, part, live);
+      RB_CUDA_TRY(launch_early(early, spmm_kernel<T, 32, 2, EPI, 2, true>, dim3(sh.grid), dim3(kBlk), st, A.n, k,
+                               A.indptr, A.indices, val, X, Y, B, part, live));
     else
-      spmm_kernel<T, 32, 2, EPI, 2, false><<<sh.grid, kBlk, 0, st>>>(A.n, k, A.indptr, A.indices, val, X, Y, B, part, live);
-    RB_LAUNCH_CHECK();
+      RB_CUDA_TRY(launch_early(early, spmm_kernel<T, 32, 2, EPI, 2, false>, dim3(sh.grid), dim3(kBlk), st, A.n, k,
+                               A.indptr, A.indices, val, X, Y, B, part, live));
     return RB_OK;
   }
   if (sh.L == 32 && !o32) {  // offsets beyond int32: the 64-bit index arithmetic
 #define RB_SPMM(L_, V_) \
-  spmm_kernel<T, L_, V_, EPI, 1, false><<<sh.grid, kBlk, 0, st>>>(A.n, k, A.indptr, A.indices, val, X, Y, B, part, live)
+  RB_CUDA_TRY(launch_early(early, spmm_kernel<T, L_, V_, EPI, 1, false>, dim3(sh.grid), dim3(kBlk), st, A.n, k, \
+                           A.indptr, A.indices, val, X, Y, B, part, live))
     RB_DISPATCH_LV(sh, RB_SPMM);
 #undef RB_SPMM
-    RB_LAUNCH_CHECK();
     return RB_OK;
   }
 #define RB_SPMM(L_, V_) \
-  spmm_kernel<T, L_, V_, EPI><<<sh.grid, kBlk, 0, st>>>(A.n, k, A.indptr, A.indices, val, X, Y, B, part, live)
+  RB_CUDA_TRY(launch_early(early, spmm_kernel<T, L_, V_, EPI>, dim3(sh.grid), dim3(kBlk), st, A.n, k, \
+                           A.indptr, A.indices, val, X, Y, B, part, live))
   RB_DISPATCH_LV(sh, RB_SPMM);
 #undef RB_SPMM
-  RB_LAUNCH_CHECK();
   return RB_OK;
 }
 
@@ -1657,13 +1661,13 @@ static int spmm_grp(const rb_csr& A, const T* val, const GroupPlan& gp, const T*
 
 template <typename T, int EPI>
 static int spmm_pair(const rb_csr& A, const T* val, const GroupPlan& gp, const T* X, T* Y, void* part,
-                     int64_t k, unsigned* grid_out, cudaStream_t st, const int32_t* live) {
+                     int64_t k, unsigned* grid_out, cudaStream_t st, const int32_t* live, bool early = false) {
   if (!pair_cols_ok<T>(k) || A.n * k >= (int64_t(1) << 31))
     return fail(RB_EARG, "row-pair SpMM: %lld columns", (long long)k);
   const unsigned grid = (unsigned)std::max<int64_t>(
       1, std::min<int64_t>(num_sms() * BpsSpmm<T>::value, ceil_div(gp.ng * PairCfg<T>::S, kBlk / 32)));
-  spmm_pair_kernel<T, EPI><<<grid, kBlk, 0, st>>>(A.n, k, A.indptr, val, gp, X, Y, part, live);
-  RB_LAUNCH_CHECK();
+  RB_CUDA_TRY(launch_early(early, spmm_pair_kernel<T, EPI>, dim3(grid), dim3(kBlk), st, A.n, k, A.indptr, val, gp, X, Y,
+                           part, live));
   *grid_out = grid;
   return RB_OK;
 }

@@ -357,7 +357,8 @@ template <bool MID>
 __global__ void __launch_bounds__(kBlk, 3)
 vc_spmm_kernel(int64_t k, VcOp<float> o, const float* __restrict__ X, float* __restrict__ Y,
                double* __restrict__ part, const int32_t* __restrict__ live) {
-  if (live && *live == 0) return;
+  chain_wait();
+  if (chain_dead(live)) return;
   constexpr int V = 4, L = 32;
   __shared__ double sm[kBlk * V];
   RB_G_TASK(float, L, V, 1);
@@ -405,7 +406,8 @@ vc_spmm_kernel(int64_t k, VcOp<float> o, const float* __restrict__ X, float* __r
 template <typename T, int L, int S>
 __global__ void __launch_bounds__(kBlk)
 vc_restrict_kernel(int64_t k, VcOp<T> o, const T* __restrict__ R, const int32_t* __restrict__ live) {
-  if (live && *live == 0) return;
+  chain_wait();
+  if (chain_dead(live)) return;
   constexpr int V = 16 / (int)sizeof(T);
   const int li = threadIdx.x % L;
   const int64_t task0 = blockIdx.x * (int64_t)(kBlk / L) + threadIdx.x / L, tasks = (int64_t)gridDim.x * (kBlk / L);
@@ -457,6 +459,7 @@ template <typename T, int L, int S>
 __global__ void __launch_bounds__(kBlk, 2)
 vc_pupdate_kernel(int64_t k, VcOp<T> o, const ColState* __restrict__ cs, const T* __restrict__ R, T* __restrict__ P,
                   T* __restrict__ Xs) {
+  chain_wait();
   constexpr int V = 16 / (int)sizeof(T), NR = kPupRows, H = kRG / NR;
   RB_G_TASK(T, L, V, S);
   T al[V], be[V];
@@ -531,7 +534,8 @@ template <typename T, int L, int S, bool INIT>
 __global__ void __launch_bounds__(kBlk, 4)
 vc_update_kernel(int64_t n, int64_t k, const ColState* __restrict__ cs, T* __restrict__ R, const T* __restrict__ Q,
                  double* __restrict__ part, cdouble* __restrict__ part_u, const int32_t* __restrict__ live) {
-  if (live && *live == 0) return;
+  chain_wait();
+  if (chain_dead(live)) return;
   constexpr int V = 16 / (int)sizeof(T);
   constexpr bool CX = Scalar<T>::is_complex;
   __shared__ double sm[kBlk * V];
@@ -587,7 +591,8 @@ vc_mid_spmm_kernel(int64_t k, VcOp<T> o, const T* __restrict__ U, const float* _
                    const T* __restrict__ W, const float* __restrict__ cw, const T* __restrict__ G,
                    const float* __restrict__ cg, const T* __restrict__ rowscale, T* __restrict__ out,
                    typename Scalar<T>::acc* __restrict__ part, const int32_t* __restrict__ live) {
-  if (live && *live == 0) return;
+  chain_wait();
+  if (chain_dead(live)) return;
   constexpr int V = 16 / (int)sizeof(T);
   typedef typename Scalar<T>::acc A;
   __shared__ A sm[DOT ? kBlk * V : 1];
@@ -644,7 +649,8 @@ vc_mid_spmm_kernel(int64_t k, VcOp<T> o, const T* __restrict__ U, const float* _
 template <typename T>
 __global__ void vc_prolong_kernel(int64_t ng, int64_t k, const int32_t* __restrict__ agg, const T* __restrict__ ec,
                                   const T* __restrict__ is1, T* __restrict__ x2, const int32_t* __restrict__ live) {
-  if (live && *live == 0) return;
+  chain_wait();
+  if (chain_dead(live)) return;
   constexpr int V = 16 / (int)sizeof(T);
   const int64_t kv = k / V;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < ng * kv; i += (int64_t)gridDim.x * blockDim.x) {
@@ -674,6 +680,7 @@ template <bool CX>
 __global__ void __launch_bounds__(kFinThreads)
 vc_rr_kernel(int64_t k, int nb, const double* part, const cdouble* part_u, ColState* cs, double tol2,
              int32_t* nactive) {
+  chain_wait();
   const int64_t c = blockIdx.x;
   if (c >= k || !cs[c].active) return;  // uniform over the block
   double rr;
@@ -698,6 +705,7 @@ template <bool CX>
 __global__ void __launch_bounds__(kFinThreads)
 vc_start_kernel(int64_t k, int nb, const double* part, const cdouble* part_u, ColState* cs,
                 const OuterState* __restrict__ os, int32_t* nactive) {
+  chain_wait();
   const int64_t c = blockIdx.x;
   if (c >= k) return;
   double rr;
@@ -721,6 +729,7 @@ template <typename A>
 __global__ void __launch_bounds__(kFinThreads)
 vc_beta_kernel(int64_t k, int nbt, const A* part_t, int nbe, const A* part_e, const VcPar* __restrict__ par,
                ColState* cs, int first, int32_t* nactive) {
+  chain_wait();
   const int64_t c = blockIdx.x;
   if (c >= k || !cs[c].active) return;  // uniform over the block
   const cdouble rt = block_sum_part<A>(part_t, nbt, k, c), ef = block_sum_part<A>(part_e, nbe, k, c);
@@ -890,16 +899,15 @@ static int vc_spmm(const rb_csr& A, const VcOp<T>& o, const VcGrids& g, const Gr
   if constexpr (std::is_same<T, float>::value) {
     if (vc_groups<T>(g)) {
       *nb = g.grp;
-      if (mid) vc_spmm_kernel<true><<<g.grp, kBlk, 0, st>>>(k, o, X, Y, (double*)part, live);
-      else vc_spmm_kernel<false><<<g.grp, kBlk, 0, st>>>(k, o, X, Y, (double*)part, live);
-      RB_LAUNCH_CHECK();
+      if (mid) RB_CUDA_TRY(launch_early(true, vc_spmm_kernel<true>, dim3(g.grp), dim3(kBlk), st, k, o, X, Y, (double*)part, live));
+      else RB_CUDA_TRY(launch_early(true, vc_spmm_kernel<false>, dim3(g.grp), dim3(kBlk), st, k, o, X, Y, (double*)part, live));
       return RB_OK;
     }
   }
-  if (gp) return spmm_pair<T, EPI_PQDOT>(A, o.vs, *gp, X, Y, part, k, nb, st, live);
+  if (gp) return spmm_pair<T, EPI_PQDOT>(A, o.vs, *gp, X, Y, part, k, nb, st, live, true);
   const Shape sh = pick_spmm_shape<T>(A.n, k);
   *nb = sh.grid;
-  return spmm_t<T, EPI_PQDOT>(A, o.vs, X, Y, nullptr, part, k, sh, st, live);
+  return spmm_t<T, EPI_PQDOT>(A, o.vs, X, Y, nullptr, part, k, sh, st, live, true);
 }
 
 // t = A^ r, f, then e = M1 f with (e, f): all but the p-update of one cycle
@@ -910,21 +918,28 @@ static int vc_apply(const rb_csr& A, const VcOp<T>& o, const VcGrids& g, const G
   const VcPar* p = o.par;
   RB_TRY(vc_spmm<T>(A, o, g, gp, true, R, o.t, part_t, k, nbt, st, live));
   if (!vc_groups<T>(g)) {
-#define RB_VR(L_, S_) vc_restrict_kernel<T, L_, S_><<<g.mid, kBlk, 0, st>>>(k, o, R, live)
+#define RB_VR(L_, S_) \
+  RB_CUDA_TRY(launch_early(true, vc_restrict_kernel<T, L_, S_>, dim3(g.mid), dim3(kBlk), st, k, o, R, live))
     RB_DISPATCH_G(g.sh, RB_VR);
 #undef RB_VR
     *launches += 1;
   }
-#define RB_VM(L_, S_)                                                                                                   vc_mid_spmm_kernel<T, L_, S_, false><<<g.mid, kBlk, 0, st>>>(k, o, o.f, &p->a, nullptr, nullptr, o.f, &p->nb, nullptr,                                                               o.x2, nullptr, live);                                     vc_mid_spmm_kernel<T, L_, S_, false><<<g.mid, kBlk, 0, st>>>(k, o, o.f, &p->one, nullptr, nullptr, o.x2, &p->mone,                                                                   o.is1, o.w, nullptr, live)
+#define RB_VM1(L_, S_, DOT_, ...) \
+  RB_CUDA_TRY(launch_early(true, vc_mid_spmm_kernel<T, L_, S_, DOT_>, dim3(g.mid), dim3(kBlk), st, k, o, __VA_ARGS__, live))
+#define RB_VM(L_, S_)                                                                                              \
+  RB_VM1(L_, S_, false, o.f, &p->a, nullptr, nullptr, o.f, &p->nb, nullptr, o.x2, nullptr);                        \
+  RB_VM1(L_, S_, false, o.f, &p->one, nullptr, nullptr, o.x2, &p->mone, o.is1, o.w, nullptr)
   RB_DISPATCH_G(g.sh, RB_VM);
 #undef RB_VM
-  RB_LAUNCH_CHECK();
-  RB_TRY(coarse_apply<T>(o.co, o.w, k, st, live));
-  vc_prolong_kernel<T><<<g.pro, 256, 0, st>>>(o.ng, k, o.co.agg, o.co.ec, o.is1, o.x2, live);
-#define RB_VM(L_, S_)                                                                                                   vc_mid_spmm_kernel<T, L_, S_, false><<<g.mid, kBlk, 0, st>>>(k, o, o.f, &p->one, nullptr, nullptr, o.x2, &p->mone,                                                                   nullptr, o.w, nullptr, live);                             vc_mid_spmm_kernel<T, L_, S_, true><<<g.mid, kBlk, 0, st>>>(k, o, o.x2, &p->one, o.w, &p->a, o.w, &p->nb, o.s1, o.e,                                                              (Acc*)o.part_c, live)
+  RB_TRY(coarse_apply<T>(o.co, o.w, k, st, live, true));
+  RB_CUDA_TRY(launch_early(true, vc_prolong_kernel<T>, dim3(g.pro), dim3(256), st, o.ng, k, o.co.agg, o.co.ec, o.is1,
+                           o.x2, live));
+#define RB_VM(L_, S_)                                                                                              \
+  RB_VM1(L_, S_, false, o.f, &p->one, nullptr, nullptr, o.x2, &p->mone, nullptr, o.w, nullptr);                    \
+  RB_VM1(L_, S_, true, o.x2, &p->one, o.w, &p->a, o.w, &p->nb, o.s1, o.e, (Acc*)o.part_c)
   RB_DISPATCH_G(g.sh, RB_VM);
 #undef RB_VM
-  RB_LAUNCH_CHECK();
+#undef RB_VM1
   *launches += 9;
   return RB_OK;
 }
@@ -949,12 +964,12 @@ static int vc_inner(const rb_csr& A, const VcOp<T>& o, int64_t k, void* part_a, 
   auto precondition = [&](int first, int32_t* live) -> int {
     unsigned nbt = 0;
     RB_TRY(vc_apply<T>(A, o, g, gp, R, part_a, k, &nbt, st, live, launches));
-    vc_beta_kernel<Acc><<<(unsigned)k, kFinThreads, 0, st>>>(k, (int)nbt, (const Acc*)part_a, (int)g.mid,
-                                                             (const Acc*)o.part_c, o.par, cs, first, live);
-#define RB_VP(L_, S_) vc_pupdate_kernel<T, L_, S_><<<g.half, kBlk, 0, st>>>(k, o, cs, R, P, Xs)
+    RB_CUDA_TRY(launch_early(true, vc_beta_kernel<Acc>, dim3((unsigned)k), dim3(kFinThreads), st, k, (int)nbt,
+                             (const Acc*)part_a, (int)g.mid, (const Acc*)o.part_c, o.par, cs, first, live));
+#define RB_VP(L_, S_) \
+  RB_CUDA_TRY(launch_early(true, vc_pupdate_kernel<T, L_, S_>, dim3(g.half), dim3(kBlk), st, k, o, cs, R, P, Xs))
     RB_DISPATCH_G(g.sh, RB_VP);
 #undef RB_VP
-    RB_LAUNCH_CHECK();
     *launches += 2;
     return RB_OK;
   };
@@ -972,13 +987,16 @@ static int vc_inner(const rb_csr& A, const VcOp<T>& o, int64_t k, void* part_a, 
     unsigned nb = 0;
     RB_TRY(vc_spmm<T>(A, o, g, gp, false, P, Q, part_a, k, &nb, st, live));
     RB_TRY(tm.record(st));
-    fin_alpha_kernel<Acc><<<(unsigned)k, kFinThreads, 0, st>>>(k, (int)nb, (const Acc*)part_a, cs, next);
-#define RB_VU(L_, S_)                                                                                                vc_update_kernel<T, L_, S_, false><<<g.row, kBlk, 0, st>>>(A.n, k, cs, R, Q, part_b, (cdouble*)part_a, live)
+    RB_CUDA_TRY(launch_early(true, fin_alpha_kernel<Acc>, dim3((unsigned)k), dim3(kFinThreads), st, k, (int)nb,
+                             (const Acc*)part_a, cs, next));
+#define RB_VU(L_, S_)                                                                                        \
+  RB_CUDA_TRY(launch_early(true, vc_update_kernel<T, L_, S_, false>, dim3(g.row), dim3(kBlk), st, A.n, k, cs, R, Q, \
+                           part_b, (cdouble*)part_a, live))
     RB_DISPATCH_G(g.sh, RB_VU);
 #undef RB_VU
     RB_TRY(tm.record(st));
-    vc_rr_kernel<CX><<<(unsigned)k, kFinThreads, 0, st>>>(k, (int)g.row, part_b, (cdouble*)part_a, cs, tol * tol, next);
-    RB_LAUNCH_CHECK();
+    RB_CUDA_TRY(launch_early(true, vc_rr_kernel<CX>, dim3((unsigned)k), dim3(kFinThreads), st, k, (int)g.row,
+                             (const double*)part_b, (const cdouble*)part_a, cs, tol * tol, next));
     RB_TRY(precondition(0, next));
     RB_TRY(tm.record(st));
     *launches += 4;
