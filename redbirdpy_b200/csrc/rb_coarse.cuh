@@ -165,6 +165,7 @@ __global__ void __launch_bounds__(256) gj_diag_kernel(const T* __restrict__ A, i
   __shared__ __align__(16) T row[2][kGjB], col[2][4][R];
   const int tid = threadIdx.x;
   const int j = tid & (kGjB - 1), ib = tid / kGjB;
+  chain_wait();
   T a[R];
 #pragma unroll
   for (int u = 0; u < R; ++u) {
@@ -217,6 +218,7 @@ __global__ void __launch_bounds__(256) gj_diag_kernel(const T* __restrict__ A, i
 // itself zero); kGjB x nc, ld nc
 template <typename T>
 __global__ void gj_cols_kernel(const T* __restrict__ A, int64_t nc, int64_t b0, int nb, T* __restrict__ CbT) {
+  chain_wait();
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nc * kGjB;
        e += (int64_t)gridDim.x * blockDim.x) {
     const int j = (int)(e / nc);
@@ -229,6 +231,7 @@ __global__ void gj_cols_kernel(const T* __restrict__ A, int64_t nc, int64_t b0, 
 template <typename T>
 __global__ void gj_rows_kernel(T* __restrict__ A, int64_t nc, int64_t b0, int nb, const T* __restrict__ R,
                                const T* __restrict__ Dinv) {
+  chain_wait();
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < (int64_t)nb * nc;
        e += (int64_t)gridDim.x * blockDim.x) {
     const int64_t i = e / nc, j = e % nc;
@@ -446,20 +449,19 @@ static int coarse_setup(const rb_csr& A, CoarseBufs<T64, T>& c, cudaStream_t st)
   const unsigned eg = (unsigned)std::min<int64_t>(ceil_div(nc * kGjB, 256), 148 * 8);
   for (int64_t b0 = 0; b0 < nc; b0 += kGjB) {
     const int nb = (int)std::min<int64_t>(kGjB, nc - b0);
-    gj_diag_kernel<T64><<<1, 256, 0, st>>>(c.A64, nc, b0, nb, c.Dinv, c.err);
-    RB_LAUNCH_CHECK();
+    RB_CUDA_TRY(launch_early(true, gj_diag_kernel<T64>, dim3(1), dim3(256), st, c.A64, nc, b0, nb, c.Dinv, c.err));
     // R = Dinv A[b, :]  (Dinv is symmetric: the inverse of a diagonal block
     // of the symmetric Schur complement, so it serves as its own transpose)
-    RB_TRY(gemm_tn<T64>(nb, nc, nb, one, c.Dinv, kGjB, c.A64 + b0 * nc, nc, zero, true, c.Rb, nc, st));
+    RB_TRY(gemm_tn<T64>(nb, nc, nb, one, c.Dinv, kGjB, c.A64 + b0 * nc, nc, zero, true, c.Rb, nc, st, 1, 0,
+                        nullptr, true));
     // CbT = (A[:, b])^T with the block's own rows zeroed
-    gj_cols_kernel<T64><<<eg, 256, 0, st>>>(c.A64, nc, b0, nb, c.Cb);
-    RB_LAUNCH_CHECK();
+    RB_CUDA_TRY(launch_early(true, gj_cols_kernel<T64>, dim3(eg), dim3(256), st, c.A64, nc, b0, nb, c.Cb));
     // A -= Cb R (rank-nb update of every row outside the block)
-    RB_TRY(gemm_tn<T64>(nc, nc, nb, mone, c.Cb, nc, c.Rb, nc, one, false, c.A64, nc, st));
+    RB_TRY(gemm_tn<T64>(nc, nc, nb, mone, c.Cb, nc, c.Rb, nc, one, false, c.A64, nc, st, 1, 0, nullptr, true));
     // A[:, b] = -Cb Dinv outside the block; A[b, :] = R; A[b, b] = Dinv
-    RB_TRY(gemm_tn<T64>(nc, nb, nb, mone, c.Cb, nc, c.Dinv, kGjB, zero, true, c.A64 + b0, nc, st));
-    gj_rows_kernel<T64><<<eg, 256, 0, st>>>(c.A64, nc, b0, nb, c.Rb, c.Dinv);
-    RB_LAUNCH_CHECK();
+    RB_TRY(gemm_tn<T64>(nc, nb, nb, mone, c.Cb, nc, c.Dinv, kGjB, zero, true, c.A64 + b0, nc, st, 1, 0,
+                        nullptr, true));
+    RB_CUDA_TRY(launch_early(true, gj_rows_kernel<T64>, dim3(eg), dim3(256), st, c.A64, nc, b0, nb, c.Rb, c.Dinv));
   }
   cast_kernel<T64, T><<<(unsigned)std::min<int64_t>(ceil_div(nc * nc, 256), 148 * 16), 256, 0, st>>>(nc * nc, c.A64,
                                                                                                      c.op.X);

@@ -952,14 +952,14 @@ static int vc_inner(const rb_csr& A, const VcOp<T>& o, int64_t k, void* part_a, 
   typedef typename Scalar<T>::acc Acc;
   constexpr bool CX = Scalar<T>::is_complex;
   const VcGrids g = vc_grids<T>(A.n, o.ng, k);
-  int32_t* slot[2] = {counter + 4, counter + 5};
-  int32_t* snap = counter + 6;
-  int rd = 1;
-  RB_CUDA_TRY(cudaMemsetAsync(slot[rd], 0, sizeof(int32_t), st));
+  // live counts, one of four words per iteration: iteration i fills word i % 4,
+  // which iteration i + 1 reads and iteration i + 4 clears
+  int32_t* const slot = counter + 4;
+  RB_CUDA_TRY(cudaMemsetAsync(slot + 3, 0, sizeof(int32_t), st));
 #define RB_VU(L_, S_)                                                                                                vc_update_kernel<T, L_, S_, true><<<g.row, kBlk, 0, st>>>(A.n, k, cs, R, Q, part_b, (cdouble*)part_a, nullptr)
   RB_DISPATCH_G(g.sh, RB_VU);
 #undef RB_VU
-  vc_start_kernel<CX><<<(unsigned)k, kFinThreads, 0, st>>>(k, (int)g.row, part_b, (cdouble*)part_a, cs, os, slot[rd]);
+  vc_start_kernel<CX><<<(unsigned)k, kFinThreads, 0, st>>>(k, (int)g.row, part_b, (cdouble*)part_a, cs, os, slot + 3);
   RB_LAUNCH_CHECK();
   auto precondition = [&](int first, int32_t* live) -> int {
     unsigned nbt = 0;
@@ -973,16 +973,16 @@ static int vc_inner(const rb_csr& A, const VcOp<T>& o, int64_t k, void* part_a, 
     *launches += 2;
     return RB_OK;
   };
-  RB_TRY(precondition(1, slot[rd]));
+  RB_TRY(precondition(1, slot + 3));
   *launches += 2;
   // Every iteration is a handful of launches, so the host looks at the live
   // count of each, one iteration behind the one it has queued (BurstSync).
   BurstSync bs;
   RB_TRY(bs.init());
-  int it = 0, pend = -1, next_snap = 0;
+  int it = 0;
   while (it < maxiter) {
-    const int32_t* live = slot[rd];
-    int32_t* next = slot[rd ^ 1];
+    const int32_t* live = slot + ((it + 3) & 3);
+    int32_t* next = slot + (it & 3);
     RB_TRY(tm.record(st));
     unsigned nb = 0;
     RB_TRY(vc_spmm<T>(A, o, g, gp, false, P, Q, part_a, k, &nb, st, live));
@@ -1000,26 +1000,24 @@ static int vc_inner(const rb_csr& A, const VcOp<T>& o, int64_t k, void* part_a, 
     RB_TRY(precondition(0, next));
     RB_TRY(tm.record(st));
     *launches += 4;
-    rd ^= 1;
-    ++it;
-    RB_CUDA_TRY(cudaMemcpyAsync(snap + next_snap, slot[rd], sizeof(int32_t), cudaMemcpyDeviceToDevice, st));
-    RB_CUDA_TRY(cudaEventRecord(bs.ev[next_snap], st));
+    RB_CUDA_TRY(cudaEventRecord(bs.ev[it & 1], st));
+    // (BurstSync::read takes a base that its event's number is added to)
+    auto count = [&](int i, int32_t* v) { return bs.read(i & 1, slot + (i & 3) - (i & 1), v); };
     int32_t v = 1;
+    ++it;
     if (tm.on) {
-      RB_TRY(bs.read(next_snap, snap, &v));
+      RB_TRY(count(it - 1, &v));
       RB_TRY(tm.harvest());
       if (v == 0) break;
       continue;
     }
-    if (pend >= 0) {
-      RB_TRY(bs.read(pend, snap, &v));
+    if (it > 1) {
+      RB_TRY(count(it - 2, &v));
       if (v == 0) {
         --it;  // the iteration queued after the last one was a no-op
         break;
       }
     }
-    pend = next_snap;
-    next_snap ^= 1;
   }
   *iters_out = it;
   return RB_OK;
