@@ -734,20 +734,41 @@ class MidLevel:
                                       self.mcol.data_ptr(), self.nnz1, ctypes.pointer(self.coarse.struct))
 
 
+# Where the V-cycle takes over from the one-launch Jacobi solve (clusters of
+# thread blocks, up to 32768 rows): at 450,000 entries of the right-hand side (a
+# complex one counts 1.65 times), times 16000 / nodes on smaller meshes, whose
+# Jacobi solves need fewer iterations.  One launch / V-cycle in ms: 5814 nodes
+# x 128 columns 1.8 / 2.6; 9261 x 48 1.7 / 2.3, x 96 3.2 / 2.7; 12150 x 32 2.2 /
+# 2.3, x 64 3.4 / 2.5; 17081 x 16 2.0 / 2.4, x 32 3.0 / 2.4; 24255 x 8 1.2 / 2.4,
+# x 16 2.4 / 2.5, x 32 3.6 / 2.6; 32292 x 8 1.5 / 2.6, x 16 3.3 / 2.7; complex
+# 7245 x 64 2.0 / 2.9, x 128 3.8 / 3.4; 12150 x 16 1.9 / 2.6, x 32 3.1 / 2.7;
+# 17081 x 16 3.5 / 2.9; 24255 x 8 2.2 / 2.9, x 16 4.2 / 3.0; 32292 x 8 2.7 / 3.1.
+VCYCLE_ENTRIES = 450000
+VCYCLE_NODES = 16000
+ONE_LAUNCH_ROWS = 32768
+
+
+def _one_launch(n, k, cplx):
+    """Whether a system of n rows and k columns goes faster in one launch."""
+    entries = n * min(k, 128) * (1.65 if cplx else 1.0)
+    return n <= ONE_LAUNCH_ROWS and entries * min(1.0, n / VCYCLE_NODES) < VCYCLE_ENTRIES
+
+
 def _resolve_mid(mat, n, k, prec, coarse, groups, instances, budget):
-    """The MidLevel a solve takes, or None: a mixed-precision solve on a mesh
-    of at least COARSE_MIN_NODES nodes with every choice left to the engine
-    ('auto'), or of stacked instances ('blocks') whose mesh has a layout that
-    keeps their groups apart."""
+    """The MidLevel a solve takes, or None: a mixed-precision solve with every
+    choice left to the engine ('auto') that is too large for one launch, or of
+    stacked instances ('blocks') whose mesh has a layout that keeps their
+    groups apart."""
     if groups != "auto" or prec != _lib.RB_MIXED or budget is not None:
         return None
     mesh = getattr(mat, "mesh", None)
-    if not hasattr(mesh, "mid_level") or n < COARSE_MIN_NODES or n * (min(k, 128) + 4) >= 2 ** 31:
+    if not hasattr(mesh, "mid_level") or n * (min(k, 128) + 4) >= 2 ** 31:
         return None
-    if (coarse == "auto" and instances is None) or (coarse == "blocks" and instances is not None
-                                                    and mesh.layout is not None):
-        return mesh.mid_level()
-    return None
+    if instances is None:
+        take = coarse == "auto" and not _one_launch(n, k, mat.is_complex)
+    else:
+        take = coarse == "blocks" and n >= COARSE_MIN_NODES and mesh.layout is not None
+    return mesh.mid_level() if take else None
 
 
 def _resolve_groups(mat, groups):
@@ -889,10 +910,10 @@ def solve(mat, B, precision="mixed", tol=DEFAULT_TOL, inner_tol=None, maxiter=20
     entirely in FP64.  Up to 128 columns per library call; wider B is solved
     in column blocks.  ``x0`` (nn x k, the solution's dtype) is an initial
     guess: the refinement starts from its FP64 residual instead of from zero.
-    With ``coarse`` and ``groups`` left at 'auto', a mixed-precision solve on a
-    mesh of 20000 nodes or more takes the three-level V-cycle preconditioner
-    (MidLevel; a solve that it does not bring to convergence is redone with
-    the two-level form); ``coarse='blocks'`` with ``instances`` asks the same of
+    With ``coarse`` and ``groups`` left at 'auto', a mixed-precision solve that
+    is too large for one launch (see _one_launch) takes the three-level V-cycle
+    preconditioner (MidLevel; a solve that it does not bring to convergence is
+    redone with the two-level form, on less than 20000 nodes with Jacobi alone); ``coarse='blocks'`` with ``instances`` asks the same of
     a batch (Jacobi alone where it does not apply).  ``coarse`` otherwise adds the aggregation coarse
     space to the Jacobi preconditioner (see _resolve_coarse).
     ``inner_tol`` (relative residual of each FP32 correction sweep) defaults to
@@ -926,6 +947,9 @@ def solve(mat, B, precision="mixed", tol=DEFAULT_TOL, inner_tol=None, maxiter=20
         coarse = False
         if instances is None:
             instances = Instances([0, n], B.device)
+    if (coarse == "auto" and groups == "auto" and prec == _lib.RB_MIXED and instances is None and not profile
+            and not spmm_lanes and _one_launch(n, k, mat.is_complex)):
+        coarse = None  # (no coarse space: the library then solves it in one launch)
     mid = _resolve_mid(mat, n, k, prec, coarse, groups, instances, budget) if k else None
     cs = _resolve_coarse(mat, coarse) if mid is None else None
     if inner_tol is None:

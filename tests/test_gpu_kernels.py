@@ -415,3 +415,24 @@ def test_batch_vcycle_equals_jacobi(omega):
     small = BatchModel([_box_cfg((14, 12, 8), 2.0, omega, 3, 2) for _ in range(12)])
     assert small.mesh.nn >= engine.COARSE_MIN_NODES and small.solve_kw["coarse"] is False
     assert small.mesh.layout is None
+
+
+@pytest.mark.parametrize("cells,ns,nd,cplx,one", [
+    ((21, 20, 20), 3, 4, False, True), ((20, 20, 20), 42, 41, False, True), ((20, 20, 20), 43, 42, False, False),
+    ((20, 20, 20), 25, 25, True, True), ((20, 20, 20), 26, 26, True, False), ((30, 28, 26), 9, 9, False, True),
+    ((30, 28, 26), 9, 10, False, False), ((20, 20, 20), 64, 64, True, False), ((32, 31, 31), 2, 1, True, False)])
+def test_solve_routes_between_one_launch_and_vcycle(cells, ns, nd, cplx, one):
+    """Both sides of the lines between the one-launch solve and the V-cycle
+    (entries, node factor, complex weight, rows of one launch): the route, and the
+    fields against the FP64 solve.  Both are refined to a relative residual of
+    1e-15, times a condition number below 1e4 times 10."""
+    cfg = _box_cfg(cells, 2.0, 2 * np.pi * 1e8 if cplx else 0.0, ns, nd)
+    model = rbb.adjoint.DeviceModel(cfg)
+    mua = torch.as_tensor(cfg["prop"][:, 0].copy(), device="cuda")
+    dco = torch.as_tensor(1.0 / (3.0 * (cfg["prop"][:, 0] + cfg["prop"][:, 1])), device="cuda")
+    mat = engine.assemble(model.mesh, model.optics(mua, dco))
+    X, info = engine.solve(mat, model.B)
+    assert info["flag"] == 0 and (info["launches"] == 2) == one
+    assert (info["coarse_nc"] > 0) == (not one)
+    Y, _ = engine.solve(mat, model.B, precision="fp64")
+    assert float((X - Y).abs().max()) <= 1e-10 * float(Y.abs().max())
