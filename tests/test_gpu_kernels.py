@@ -155,7 +155,7 @@ def _box_cfg(cells, h, omega, ns, nd, seed=0, hole=False):
 @pytest.mark.parametrize("cells,cols,hole", [((28, 27, 25), (1, 2), True), ((28, 27, 25), (17, 20), True),
                                              ((40, 24, 20), (31, 33), False), ((28, 27, 25), (33, 34), False),
                                              ((27, 28, 26), (64, 64), True), ((28, 27, 25), (70, 61), False)])
-def test_vcycle_solve_matches_the_two_level_form(cells, cols, hole, omega):
+def test_vcycle_solve_matches_the_two_level_form(cells, cols, hole, omega, monkeypatch):
     """The three-level cycle at lane layouts from 4 to 128 columns (padded
     counts, both column slices of complex solves, more than one block of 128)
     on meshes with partly empty groups: the solution of the two-level and
@@ -164,6 +164,7 @@ def test_vcycle_solve_matches_the_two_level_form(cells, cols, hole, omega):
     iterations, and again from a perturbed start."""
     from redbirdpy_b200.forward import forward_device
 
+    monkeypatch.setattr(engine, "VCYCLE_ENTRIES", 0)  # few columns too
     cfg = _box_cfg(cells, 1.5, omega, *cols, hole=hole)
     d1, p1, _, mat, i1 = forward_device(cfg)
     assert mat.n >= engine.COARSE_MIN_NODES and engine.mesh_of(cfg).mid_level() is not None
@@ -176,9 +177,10 @@ def test_vcycle_solve_matches_the_two_level_form(cells, cols, hole, omega):
     assert i2["flag"] == 0 and (p2 - p0).abs().max() <= 1e-9 * p0.abs().max()
 
 
-def test_vcycle_zero_and_non_finite_columns():
+def test_vcycle_zero_and_non_finite_columns(monkeypatch):
     """A zero column stays exactly zero; a non-finite one is flagged and the
     others still solve (through the two-level form)."""
+    monkeypatch.setattr(engine, "VCYCLE_ENTRIES", 0)
     cfg = _box_cfg((28, 27, 25), 1.5, 0.0, 3, 2)
     mesh = engine.mesh_of(cfg)
     mat = engine.assemble(mesh, engine.Optics.from_cfg(mesh, cfg))
@@ -363,12 +365,13 @@ def test_pinned_pool_is_bounded_and_thread_safe():
     assert not bad
 
 
-def test_captured_step_budget_covers_its_jacobi_solves():
+def test_captured_step_budget_covers_its_jacobi_solves(monkeypatch):
     """A captured step on a mesh whose checked solves take the V-cycle (24
     iterations where Jacobi alone takes 130): its budget is for the solves it
     runs, so it converges; also a batch of such instances."""
     from redbirdpy_b200.adjoint import BatchModel, CapturedStep, DeviceModel, detector_values
 
+    monkeypatch.setattr(engine, "VCYCLE_ENTRIES", 0)
     cfg = _box_cfg((34, 30, 18), 2.0, 0.0, 5, 4)
     cfgs = [_box_cfg(c, 2.0, 0.0, 4, 3) for c in ((24, 20, 12), (20, 24, 14), (28, 20, 10))]
     for model, cs in ((DeviceModel(cfg), [cfg]), (BatchModel(cfgs), cfgs)):
