@@ -602,6 +602,11 @@ jac_tc_kernel(JacArgs a, const In* __restrict__ phi, float* __restrict__ Jout, u
 // switch that lets a caller take the SIMT products instead
 __device__ int g_jac_tc_err;
 static bool g_jac_tc_on = false;
+// (rb_jacgrid.cu reports its own waits there too)
+int* jac_err_word() {
+  int* p = nullptr;
+  return cudaGetSymbolAddress(reinterpret_cast<void**>(&p), g_jac_tc_err) == cudaSuccess ? p : nullptr;
+}
 
 // launches the tensor-core form when the pairs are the full grid with FP32
 // output and the sizes fit it; returns 1 when it did not apply
@@ -805,7 +810,7 @@ int rb_jac_status(void* stream) {
   if (h) {
     const int zero = 0;
     RB_CUDA_TRY(cudaMemcpyToSymbol(g_jac_tc_err, &zero, sizeof(int)));
-    return fail(RB_ECUDA, "rb_jac: a tensor-core wait gave up (code %d); the rows are not valid", h);
+    return fail(RB_ECUDA, "rb_jac: a wait for a copy or the tensor cores gave up (code %d); the rows are not valid", h);
   }
   return RB_OK;
 }

@@ -17,10 +17,12 @@
 //  - jac_b_kernel builds the B matrices of a chunk of nodes, a warp per node,
 //    into a workspace that stays in L2;
 //  - jac_grid_kernel is persistent: 4 warps bring the next item's fields and B
-//    by cp.async into the other half of the shared memory while 8 warps form
-//    the products (with the computing warps fetching as well the two did not
-//    overlap: 6.9 ms against 6.1; with 2 fetching warps 8.9); the neighbour
-//    lists that this needs are loaded two items ahead;
+//    into the other half of the shared memory while 8 warps form the products:
+//    by bulk copies of a row's column range where sources and detectors are two
+//    ranges on 16 bytes (5.6 ms at the size below), else by cp.async (6.1; with
+//    the computing warps fetching as well the two did not overlap: 6.9; with 2
+//    fetching warps 8.9); the neighbour lists that this needs are loaded two
+//    items ahead;
 //  - a thread takes 4 sources x 4 detectors of one node; 8 neighbouring lanes
 //    take 8 neighbouring nodes whose J columns are one aligned sector (blocks
 //    of nodes start where the quantity's J column is a multiple of 8), and a
@@ -29,15 +31,19 @@
 //  - C replaces phi_d in place (a thread owns half of a column, the lane next
 //    to it the other half), which is what lets two buffers of 8 nodes fit.
 // Measured at 67,626 nodes, 64 x 64 complex pairs, two quantities (4.4 GB of
-// rows): 9.9 ms before, 6.7 now, of which 0.6 the B matrices.  FP64 products
-// (2.1 ms at the full rate) and their latency with two warps per scheduler
-// bound it now: 1.2 ms of a quantity are products, 0.5 the C matrices, 1.6 the
-// fetch of 8 GB out of L2, half of which hides.
+// rows): 9.9 ms before, 6.2 now, of which 0.6 the B matrices.  Shared memory
+// bounds it now: the products' reads take about as long as their FP64 work (2.1
+// ms at the full rate), the C matrices' two thirds of that again, with two warps
+// per scheduler to overlap them.  (The fetching warps forming C as well: 5.61
+// ms against 5.56.)
 #include <algorithm>
 
 #include "rb_common.cuh"
+#include "rb_tc.cuh"
 
 namespace rb {
+
+int* jac_err_word();  // rb_jac.cu: what rb_jac_status reads
 
 enum { JG_MUA_REF = 0, JG_MUA_NODAL = 1, JG_D = 2 };
 constexpr int kJgThreads = 256;    // threads that compute
@@ -144,6 +150,13 @@ __device__ __forceinline__ void b_fma(cdouble& acc, double b, cdouble v) {
   acc.y = fma(b, v.y, acc.y);
 }
 
+// a copy of the asynchronous engine, completed on a barrier (16-byte aligned, whole 16 bytes)
+__device__ __forceinline__ void jg_bulk(void* dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(jg_u32(dst)),
+               "l"(src), "r"(bytes), "r"(bar)
+               : "memory");
+}
+
 // shared memory, per buffer: phi_s [TN][SP], phi_d (then C) [TN][SD], B
 // [TN][rmax RM]; then the neighbour lists of three items and the column map
 struct JgLayout {
@@ -181,8 +194,10 @@ __host__ __device__ inline JgLayout jg_layout(int rmax, int nsu, int nd, int nbu
 template <typename C, bool SPLIT, int RM, int TN, int NBUF>
 __global__ void __launch_bounds__(kJgThreads + kJgProducers, 1)
 jac_grid_kernel(JgArgs a, const C* __restrict__ phi, const double* __restrict__ Bg, float* __restrict__ J,
-                int32_t items) {
+                int32_t items, int* __restrict__ err) {
   extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ __align__(8) uint64_t full[2];
+  __shared__ int s_bad;
   constexpr int NT = kJgThreads;
   static_assert(TN * RM <= NT, "a thread loads one neighbour at most");
   const int rmax = a.rmax, nsu = a.nsu, nd = a.nd;
@@ -242,9 +257,41 @@ jac_grid_kernel(JgArgs a, const C* __restrict__ phi, const double* __restrict__ 
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
 
+  // the same by bulk copies, a row and column range each: where the sources'
+  // and the detectors' columns are two ranges that start on 16 bytes
+  auto fetch_bulk = [&](int32_t item, int slot, int buf) {
+    const int32_t nb = item / ntile, tile = item - nb * ntile;
+    const int s0 = tile / L.ndt * ST, d0 = tile % L.ndt * DT;
+    const int64_t n0 = a.blk0 + (int64_t)nb * TN;
+    unsigned char* const base = smem + (size_t)buf * L.buf;
+    const uint32_t bar = smem_u32(&full[buf]);
+    const int r = tid - NT, t = r / rmax, q = r - t * rmax;
+    const int32_t m = r < TN * rmax ? snb[(slot * TN + t) * (RM + 1) + 1 + q] : -1;
+    const uint32_t sbytes = (uint32_t)(min(ST, nsu - s0) * (int)sizeof(C));
+    const uint32_t dbytes = (uint32_t)(min(DT, nd - d0) * (int)sizeof(C));
+    uint32_t bytes = m >= 0 ? sbytes + dbytes : 0u, bbytes = 0u;
+    const int t0 = (int)max((int64_t)0, a.chunk0 - n0), t1 = (int)min((int64_t)TN, a.chunk1 - n0);
+    if (r == 0 && t1 > t0) bbytes = (uint32_t)((t1 - t0) * rmax * RM * (int)sizeof(double));
+    mbar_expect_tx(bar, bytes + bbytes);  // (arrives for this thread)
+    if (m >= 0) {
+      const C* src = phi + (int64_t)m * a.ld;
+      jg_bulk(reinterpret_cast<C*>(base + L.phis) + t * L.SP + q * ST, src + scol[s0], sbytes, bar);
+      jg_bulk(reinterpret_cast<C*>(base + L.phid) + t * L.SD + q * DT, src + scol[nsu + d0], dbytes, bar);
+    }
+    if (bbytes)
+      jg_bulk(reinterpret_cast<double*>(base + L.b) + (size_t)t0 * rmax * RM,
+              Bg + (n0 + t0 - a.chunk0) * (int64_t)(rmax * RM), bbytes, bar);
+  };
+
   const int32_t step = gridDim.x;
   int32_t item = blockIdx.x;
   if (item >= items) return;
+  if (tid == 0) {
+    s_bad = 0;
+    mbar_init(smem_u32(&full[0]), kJgProducers);
+    mbar_init(smem_u32(&full[1]), kJgProducers);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
   int32_t lb, le, mb, me, mm;  // row bounds of the item three ahead; bounds and neighbour of the one two ahead
   bounds(item, lb, le);
   keep(0, le - lb, neighbour(lb, le));
@@ -252,20 +299,39 @@ jac_grid_kernel(JgArgs a, const C* __restrict__ phi, const double* __restrict__ 
   keep(1, le - lb, neighbour(lb, le));
   bounds(item + 2 * step, lb, le);
   __syncthreads();
+  bool range = ((reinterpret_cast<uintptr_t>(phi + scol[0]) | reinterpret_cast<uintptr_t>(phi + scol[nsu])) & 15) == 0 &&
+               (a.ld * (int64_t)sizeof(C)) % 16 == 0;
+  if (tid < nsu) range = range && scol[tid] == scol[0] + tid;
+  if (tid < nd) range = range && scol[nsu + tid] == scol[nsu] + tid;
+  const bool bulk = __syncthreads_and(range);
   const bool producer = tid >= NT;
-  if (producer) fetch(item, 0, 0);
+  if (producer) {
+    if (bulk) fetch_bulk(item, 0, 0);
+    else fetch(item, 0, 0);
+  }
   const int t = tid % TN, g = tid / TN, sb = g % NSB, db = g / NSB;
   int slot = 0;
   for (int it = 0; item < items; item += step, ++it) {
     const int buf = NBUF == 2 ? it & 1 : 0;
     const int next = slot == 2 ? 0 : slot + 1, after = next == 2 ? 0 : next + 1;
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    if (bulk) {
+      if (!producer && !mbar_wait(smem_u32(&full[buf]), (NBUF == 2 ? it >> 1 : it) & 1, err, 64)) s_bad = 1;
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
     __syncthreads();
+    if (bulk && *reinterpret_cast<volatile int*>(&s_bad)) {  // (reported by rb_jac_status)
+      mbar_wait(smem_u32(&full[buf]), (NBUF == 2 ? it >> 1 : it) & 1, err, 64);  // its own copies, again with a limit
+      return;
+    }
     mb = lb;
     me = le;
     mm = neighbour(mb, me);
     bounds(item + 3 * step, lb, le);
-    if (NBUF == 2 && producer && item + step < items) fetch(item + step, next, buf ^ 1);
+    if (NBUF == 2 && producer && item + step < items) {
+      if (bulk) fetch_bulk(item + step, next, buf ^ 1);
+      else fetch(item + step, next, buf ^ 1);
+    }
     unsigned char* const base = smem + (size_t)buf * L.buf;
     const C* const ps = reinterpret_cast<const C*>(base + L.phis);
     C* const pd = reinterpret_cast<C*>(base + L.phid);
@@ -347,9 +413,14 @@ jac_grid_kernel(JgArgs a, const C* __restrict__ phi, const double* __restrict__ 
       }
     }
     keep(after, me - mb, mm);  // (that slot's item is done with)
+    // the buffer's reads and writes come before the copies that refill it
+    if (bulk) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     if (NBUF == 1 && item + step < items) {
       __syncthreads();
-      if (producer) fetch(item + step, next, 0);
+      if (producer) {
+        if (bulk) fetch_bulk(item + step, next, 0);
+        else fetch(item + step, next, 0);
+      }
     }
     slot = next;
   }
@@ -364,6 +435,8 @@ static int jg_rm(int rmax) { return rmax <= 16 ? 16 : 32; }
 
 template <typename C, bool SPLIT, int RM, int TN>
 static int jg_run(JgArgs a, int64_t node1, const C* phi, float* J, double* work, bool* done, cudaStream_t st) {
+  int* const err = jac_err_word();
+  if (!err) return fail(RB_ECUDA, "rb_jac_multi: no error word");
   int nbuf = 2;
   JgLayout L = jg_layout<C, TN, RM>(a.rmax, a.nsu, a.nd, 2);
   if (L.total > kJgSmem) {
@@ -386,7 +459,7 @@ static int jg_run(JgArgs a, int64_t node1, const C* phi, float* J, double* work,
     jac_b_kernel<RM><<<(unsigned)std::min<int64_t>(ceil_div(a.chunk1 - c, bw), 148 * 64), bw * 32, 0, st>>>(a, work);
     RB_LAUNCH_CHECK();
     const int64_t items = ceil_div(a.chunk1 - a.blk0, TN) * ntile;
-    kern<<<(unsigned)std::min<int64_t>(items, 148), kJgThreads + kJgProducers, L.total, st>>>(a, phi, work, J, (int32_t)items);
+    kern<<<(unsigned)std::min<int64_t>(items, 148), kJgThreads + kJgProducers, L.total, st>>>(a, phi, work, J, (int32_t)items, err);
     RB_LAUNCH_CHECK();
   }
   *done = true;

@@ -439,3 +439,34 @@ def test_solve_routes_between_one_launch_and_vcycle(cells, ns, nd, cplx, one):
     assert (info["coarse_nc"] > 0) == (not one)
     Y, _ = engine.solve(mat, model.B, precision="fp64")
     assert float((X - Y).abs().max()) <= 1e-10 * float(Y.abs().max())
+
+
+@pytest.mark.parametrize("mesh_kind", ["box", "delaunay"])
+@pytest.mark.parametrize("cplx,ld,s0,sstep,d0", [
+    (False, 40, 0, 1, 12),   # two ranges on 16 bytes: bulk copies
+    (False, 40, 1, 1, 14),   # sources start off 16 bytes
+    (False, 40, 0, 1, 13),   # detectors start off 16 bytes
+    (False, 41, 0, 1, 12),   # rows start off 16 bytes
+    (False, 40, 0, 2, 26),   # every other column
+    (True, 41, 1, 1, 15),    # complex entries are 16 bytes each
+    (True, 41, 0, 2, 26)])
+def test_grid_jacobian_rows_by_either_copy(mesh_kind, cplx, ld, s0, sstep, d0):
+    """The fetch by bulk copies and the one by 16- or 8-byte copies, along the
+    line between them: rb_jac's rows bit for bit."""
+    mesh = engine.mesh_of(_mesh((6, 5, 4)) if mesh_kind == "box" else _delaunay_cfg())
+    ns, nd = 12, 8
+    g = torch.Generator("cuda").manual_seed(ld + d0)
+    dt = torch.complex128 if cplx else torch.float64
+    phi = torch.randn((mesh.nn, ld), generator=g, device="cuda", dtype=dt)
+    s, d = np.meshgrid(s0 + sstep * np.arange(ns), d0 + np.arange(nd))
+    sd = np.column_stack([s.ravel(), d.ravel(), np.ones(ns * nd)])
+    J, K = engine.jacobian_matrix(mesh, phi, sd, ("mua",), "exact", acc64=True)
+    cols, det0, ndet, psrc, pdet, colsd, ps, pd, gnsd = engine._pair_dev(sd, phi.device)
+    assert gnsd < 0
+    kind = engine._lib.RB_JAC_SPLIT_F32_ACC64 if cplx else engine._lib.RB_JAC_F32_ACC64
+    ref = torch.full_like(J, float("nan"))
+    engine.call("rb_jac", engine.ctypes.byref(mesh.struct), engine._lib.RB_JAC_MUA_NODAL, engine.ptr(phi),
+                engine._lib.RB_C128 if cplx else engine._lib.RB_F64, ld, engine.ptr(colsd), len(cols), det0, ndet,
+                engine.ptr(ps), engine.ptr(pd), gnsd, engine.ptr(ref), ref.shape[1], kind, mesh.rmax, mesh.emax,
+                engine.ptr(mesh.evol), None, engine.stream())
+    assert torch.equal(J[:, :K], ref[:, :K])
