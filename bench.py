@@ -777,7 +777,7 @@ def run_adjoint(world, args):
     out["jacobian"] = {"rows": int(J.shape[0]), "cols": int(K), "ms": round(jms, 3),
                        "write_gbs": round(jbytes / (jms * 1e-3) / 1e9, 1),
                        "frac_of_hbm": round(jbytes / (jms * 1e-3) / 1e9 / peak, 4),
-                       "note": "both parameter launches (rb_jac: mua_nodal, D) and the clear of the row padding"}
+                       "note": "both quantities (rb_jac_multi: mua_nodal, D) and the clear of the row padding"}
     return out
 
 

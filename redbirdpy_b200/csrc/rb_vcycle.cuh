@@ -24,8 +24,11 @@
 // over the row groups: each x row is gathered once per group, and P1^T of a
 // product is the sum of the rows the same warp has in registers.
 // Measured (whole forward, two-level -> this): 520k nodes x 128 columns 96.3 ->
-// 53.0 ms (130 -> 34 iterations), complex 224.6 -> 118.0 (160 -> 34); 43k x 37
-// 9.9 -> 6.0 (100 -> 27); gradient at 68k x 64 11.9 -> 6.7 (90 -> 26).
+// 49.9 ms (130 -> 34 iterations), complex 224.6 -> 116.3 (160 -> 34); 43k x 37
+// 9.9 -> 4.7 (100 -> 25); gradient at 68k x 64 11.9 -> 5.4 (90 -> 25); batch of 64
+// boxes 48.6 (Jacobi) -> 23.8.  The kernels of an iteration are launched early
+// (launch_early): a gap of a microsecond before each of 16 kernels was an eighth
+// of the middle sizes' time (43k x 37 5.42 -> 4.75).
 #pragma once
 
 namespace rb {

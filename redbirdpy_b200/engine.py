@@ -913,9 +913,10 @@ def solve(mat, B, precision="mixed", tol=DEFAULT_TOL, inner_tol=None, maxiter=20
     With ``coarse`` and ``groups`` left at 'auto', a mixed-precision solve that
     is too large for one launch (see _one_launch) takes the three-level V-cycle
     preconditioner (MidLevel; a solve that it does not bring to convergence is
-    redone with the two-level form, on less than 20000 nodes with Jacobi alone); ``coarse='blocks'`` with ``instances`` asks the same of
-    a batch (Jacobi alone where it does not apply).  ``coarse`` otherwise adds the aggregation coarse
-    space to the Jacobi preconditioner (see _resolve_coarse).
+    redone with the two-level form, on less than 20000 nodes with Jacobi alone);
+    ``coarse='blocks'`` with ``instances`` asks the same of a batch (Jacobi
+    alone where it does not apply).  ``coarse`` otherwise adds the aggregation
+    coarse space to the Jacobi preconditioner (see _resolve_coarse).
     ``inner_tol`` (relative residual of each FP32 correction sweep) defaults to
     1e-5 with a coarse space and 1e-4 without: on the 520k-node box at 128
     columns, 1e-5 took 3 sweeps / 130 iterations / 113.5 ms against 4 / 150 /
