@@ -467,12 +467,13 @@ int rb_jac_remap(const void* J, int32_t kind, int64_t rows, int64_t ldj, const i
                  void* stream);
 /* rb_jac_range for nparam quantities at once: quantity what[p] (host array)
  * goes to the columns col0[p] .. of J (host array, elements).  The full
- * source x detector grid (nsd < 0) of FP64 fields into FP32 rows formed in
- * FP64 takes a pipelined kernel (bit-identical to rb_jac; fastest with J
- * 32-byte aligned and ldj % 8 == 0); the rest runs rb_jac_range.  work:
- * rb_jac_multi_work_bytes (0 when the kernel does not apply; may then be
- * NULL), 16-byte aligned. */
-size_t rb_jac_multi_work_bytes(int32_t rmax);
+ * source x detector grid (nsd < 0; any counts) of FP64 fields into FP32 rows
+ * formed in FP64 takes a pipelined kernel when work is given (bit-identical to
+ * rb_jac; fastest with J 32-byte aligned and ldj % 8 == 0; worth it from about
+ * 8000 nodes); the rest runs rb_jac_range.  work: rb_jac_multi_work_bytes
+ * bytes, 16-byte aligned, or NULL (the bytes are 0 when the kernel does not
+ * apply or its tiles would be mostly empty). */
+size_t rb_jac_multi_work_bytes(int32_t rmax, int32_t nsu, int32_t ndet, int32_t is_complex);
 int rb_jac_multi(const rb_mesh* mesh, int32_t nparam, const int32_t* what, const int64_t* col0, const void* phi,
                  int32_t phi_kind, int64_t ld, const int32_t* cols, int32_t nc, int32_t det0, int32_t ndet,
                  const int32_t* pair_src, const int32_t* pair_det, int64_t nsd, void* J, int64_t ldj,

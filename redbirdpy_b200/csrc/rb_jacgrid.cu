@@ -300,7 +300,7 @@ jac_grid_kernel(JgArgs a, const C* __restrict__ phi, const double* __restrict__ 
   bounds(item + 2 * step, lb, le);
   __syncthreads();
   bool range = ((reinterpret_cast<uintptr_t>(phi + scol[0]) | reinterpret_cast<uintptr_t>(phi + scol[nsu])) & 15) == 0 &&
-               (a.ld * (int64_t)sizeof(C)) % 16 == 0;
+               (a.ld * (int64_t)sizeof(C)) % 16 == 0 && (nsu * sizeof(C)) % 16 == 0 && (nd * sizeof(C)) % 16 == 0;
   if (tid < nsu) range = range && scol[tid] == scol[0] + tid;
   if (tid < nd) range = range && scol[nsu + tid] == scol[nsu] + tid;
   const bool bulk = __syncthreads_and(range);
@@ -432,6 +432,12 @@ static int64_t jg_chunk(int rmax, int RM) {
   return std::max<int64_t>(1024, (int64_t(48) << 20) / per / 8 * 8);
 }
 static int jg_rm(int rmax) { return rmax <= 16 ? 16 : 32; }
+// the fraction of the tiles' pairs that exist
+template <typename C>
+static double jg_fill(int rmax, int nsu, int nd) {
+  const JgLayout L = rmax <= 16 ? jg_layout<C, 8, 16>(rmax, nsu, nd, 2) : jg_layout<C, 4, 32>(rmax, nsu, nd, 2);
+  return (double)nsu * nd / ((double)L.nst * L.ST * L.ndt * L.DT);
+}
 
 template <typename C, bool SPLIT, int RM, int TN>
 static int jg_run(JgArgs a, int64_t node1, const C* phi, float* J, double* work, bool* done, cudaStream_t st) {
@@ -478,8 +484,16 @@ using namespace rb;
 
 extern "C" {
 
-size_t rb_jac_multi_work_bytes(int32_t rmax) {
-  if (rmax < 1 || rmax > 32) return 0;
+size_t rb_jac_multi_work_bytes(int32_t rmax, int32_t nsu, int32_t ndet, int32_t is_complex) {
+  if (rmax < 1 || rmax > 32 || nsu < 1 || ndet < 1) return 0;
+  // the tiles must be filled: seven tenths of them with real fields, four with
+  // complex ones.  16,926 nodes x 2 quantities, jac_kernel / this, ms: real
+  // 1 x 1 pairs (1/16 filled) 0.37 / 0.43, 2 x 3 (3/8) 0.37 / 0.43, 33 x 17 (0.44)
+  // 0.83 / 0.90, 5 x 7 (0.55) 0.43 / 0.43, 11 x 13 (0.74) 0.57 / 0.44; complex 1 x 1
+  // 0.38 / 0.40, 2 x 3 0.44 / 0.41, 33 x 17 1.12 / 1.01, 11 x 13 0.61 / 0.45, 61 x 64
+  // 3.80 / 1.82
+  const double fill = is_complex ? jg_fill<cdouble>(rmax, nsu, ndet) : jg_fill<double>(rmax, nsu, ndet);
+  if (fill < (is_complex ? 0.4 : 0.7)) return 0;
   const int RM = jg_rm(rmax);
   return (size_t)jg_chunk(rmax, RM) * rmax * RM * sizeof(double) + 256;
 }
@@ -495,11 +509,10 @@ int rb_jac_multi(const rb_mesh* mesh, int32_t nparam, const int32_t* what, const
   // the staging fits; everything else through rb_jac_range
   const bool cx = phi_kind == RB_C128 && out_kind == RB_JAC_SPLIT_F32_ACC64;
   const bool re = phi_kind == RB_F64 && out_kind == RB_JAC_F32_ACC64;
-  const size_t need = rb_jac_multi_work_bytes(rmax);
+  const size_t need = rb_jac_multi_work_bytes(rmax, det0, ndet, cx);
   if (nsd < 0 && (cx || re) && need && work && work_bytes >= need && (reinterpret_cast<uintptr_t>(work) & 15) == 0 &&
       emax <= kJgMaxE && phi && cols && pair_src && pair_det && J && evol && nc >= 1 && ndet >= 1 && det0 >= 1 &&
-      det0 + ndet <= nc && det0 + ndet <= 128 && det0 <= 64 && -nsd == (int64_t)det0 * ndet && det0 % 4 == 0 &&
-      ndet % 4 == 0 && node0 >= 0 && count > 0 && node0 + count <= mesh->nn && ldj >= count) {
+      det0 + ndet <= nc && det0 + ndet <= 128 && det0 <= 64 && -nsd == (int64_t)det0 * ndet && node0 >= 0 && count > 0 && node0 + count <= mesh->nn && ldj >= count) {
     bool ok = (reinterpret_cast<uintptr_t>(phi) & (cx ? 15 : 7)) == 0;
     for (int p = 0; p < nparam; ++p) ok = ok && what[p] >= JG_MUA_REF && what[p] <= JG_D && (what[p] != JG_D || ddd);
     if (ok) {
@@ -532,6 +545,7 @@ int rb_jac_multi(const rb_mesh* mesh, int32_t nparam, const int32_t* what, const
     }
   }
   if (done) return RB_OK;
+  if (nsd < 0 && (det0 % 4 || ndet % 4)) nsd = -nsd;  // (rb_jac's grid form takes multiples of 4)
   const int esz = out_kind == RB_JAC_SPLIT_BF16 || out_kind == RB_JAC_BF16 ? 2
                   : out_kind == RB_F64 || out_kind == RB_C64 || out_kind == RB_JAC_SPLIT_F64 ? 8
                   : out_kind == RB_C128 ? 16 : 4;

@@ -1053,12 +1053,13 @@ def pair_map(sd, nsrc_cols=None):
     return cols, len(s_u), len(d_u), psrc, pdet, act[:, 0], act[:, 1]
 
 
-def _grid_nsd(psrc, pdet, nsu, ndet):
+def _grid_nsd(psrc, pdet, nsu, ndet, mult=4):
     """nsd as rb_jac expects it: negative when the pairs are every (source,
     detector) combination in detector-major order (sdmap's layout) with both
-    counts multiples of 4, which selects the register-blocked kernel path."""
+    counts multiples of 4, which selects the register-blocked kernel path;
+    mult=1 for rb_jac_multi, which takes any counts."""
     nsd = len(psrc)
-    if (nsd == nsu * ndet and nsu % 4 == 0 and ndet % 4 == 0
+    if (nsd == nsu * ndet and nsu % mult == 0 and ndet % mult == 0
             and np.array_equal(psrc, np.tile(np.arange(nsu), ndet))
             and np.array_equal(pdet, np.repeat(np.arange(ndet), nsu))):
         return -nsd
@@ -1173,12 +1174,19 @@ def _jac_what(name, mode):
     raise ValueError(f"unknown parameter {name}")
 
 
+# Nodes from which the full grid's rows take the pipelined kernel (and its
+# workspace): 16 x 16 pairs, one quantity, general kernel / this, ms: 2002 nodes
+# 0.181 / 0.179 (64 x 64 0.350 / 0.394), 16,926 nodes 0.352 / 0.279 (0.917 / 0.782),
+# 58,609 nodes 0.869 / 0.593 (2.291 / 1.986)
+JAC_GRID_NODES = 8192
+
+
 def _jac_params(mesh, whats, phi, phi_kind, colsd, nc, det0, ndet, ps, pd, gnsd, J, ldj, out_kind, stride, node0, count):
     """The rows of every parameter (rb_jac_multi), parameter p's columns from
     p * stride."""
     npar = len(whats)
-    wb = _lib.lib().rb_jac_multi_work_bytes(mesh.rmax)
-    if gnsd >= 0 or out_kind not in (_lib.RB_JAC_SPLIT_F32_ACC64, _lib.RB_JAC_F32_ACC64):
+    wb = _lib.lib().rb_jac_multi_work_bytes(mesh.rmax, det0, ndet, int(phi.is_complex()))
+    if gnsd >= 0 or count < JAC_GRID_NODES or out_kind not in (_lib.RB_JAC_SPLIT_F32_ACC64, _lib.RB_JAC_F32_ACC64):
         wb = 0  # not the pipelined kernel's: no workspace
     work = torch.empty(wb, dtype=torch.uint8, device=phi.device) if wb else None
     need_ddd = _lib.RB_JAC_D in whats
@@ -1219,7 +1227,7 @@ def jacobian_matrix(mesh, phi, sd, params=("mua",), mode="reference", dtype=torc
                 torch.complex64: _lib.RB_C64}[phi.dtype]
     colsd, ps, pd = _i32(cols, phi.device), _i32(psrc, phi.device), _i32(pdet, phi.device)
     _jac_params(mesh, [_jac_what(name, mode) for name in params], phi, phi_kind, colsd, len(cols), det0, ndet, ps, pd,
-                _grid_nsd(psrc, pdet, det0, ndet), J, ldj, out_kind, nn, 0, nn)
+                _grid_nsd(psrc, pdet, det0, ndet, 1), J, ldj, out_kind, nn, 0, nn)
     _jac_checked()
     return J, len(params) * nn
 
@@ -1364,7 +1372,8 @@ class SlabJacobian:
     def __init__(self, mesh, phi, sd, params=("mua",), mode="reference", width=4096, dtype=torch.float32,
                  acc64=False):
         self.mesh, self.phi, self.params, self.dtype = mesh, phi, tuple(params), dtype
-        self.cols, self.det0, self.ndet, psrc, pdet, self.colsd, self.ps, self.pd, self.gnsd = _pair_dev(sd, phi.device)
+        self.cols, self.det0, self.ndet, psrc, pdet, self.colsd, self.ps, self.pd, _ = _pair_dev(sd, phi.device)
+        self.gnsd = _grid_nsd(psrc, pdet, self.det0, self.ndet, 1)
         if len(self.cols) > 128 or self.ndet > 64:
             raise ValueError("rb_jac stages at most 128 phi columns and 64 detectors per call")
         nsd = len(psrc)

@@ -216,10 +216,11 @@ def _delaunay_cfg(seed=0):
 @pytest.mark.parametrize("cplx", [False, True])
 @pytest.mark.parametrize("mesh_kind", ["box", "delaunay"])
 @pytest.mark.parametrize("ns,nd", [(4, 4), (12, 8), (4, 64), (64, 4), (28, 36), (64, 64)])
-def test_grid_jacobian_rows_equal_the_general_kernels(ns, nd, mesh_kind, cplx):
+def test_grid_jacobian_rows_equal_the_general_kernels(ns, nd, mesh_kind, cplx, monkeypatch):
     """The pipelined kernel of the FP64-formed FP32 rows (both parameters, and
     node slabs of odd widths) = rb_jac's rows per quantity, bit for bit: the
     same products in the same order."""
+    monkeypatch.setattr(engine, "JAC_GRID_NODES", 1)
     mesh = engine.mesh_of(_mesh((7, 5, 4)) if mesh_kind == "box" else _delaunay_cfg())
     assert (mesh.rmax <= 16) == (mesh_kind == "box") and mesh.rmax <= 32 and mesh.emax <= 64
     g = torch.Generator("cuda").manual_seed(ns * 100 + nd)
@@ -450,9 +451,10 @@ def test_solve_routes_between_one_launch_and_vcycle(cells, ns, nd, cplx, one):
     (False, 40, 0, 2, 26),   # every other column
     (True, 41, 1, 1, 15),    # complex entries are 16 bytes each
     (True, 41, 0, 2, 26)])
-def test_grid_jacobian_rows_by_either_copy(mesh_kind, cplx, ld, s0, sstep, d0):
+def test_grid_jacobian_rows_by_either_copy(mesh_kind, cplx, ld, s0, sstep, d0, monkeypatch):
     """The fetch by bulk copies and the one by 16- or 8-byte copies, along the
     line between them: rb_jac's rows bit for bit."""
+    monkeypatch.setattr(engine, "JAC_GRID_NODES", 1)
     mesh = engine.mesh_of(_mesh((6, 5, 4)) if mesh_kind == "box" else _delaunay_cfg())
     ns, nd = 12, 8
     g = torch.Generator("cuda").manual_seed(ld + d0)
@@ -470,3 +472,30 @@ def test_grid_jacobian_rows_by_either_copy(mesh_kind, cplx, ld, s0, sstep, d0):
                 engine.ptr(ps), engine.ptr(pd), gnsd, engine.ptr(ref), ref.shape[1], kind, mesh.rmax, mesh.emax,
                 engine.ptr(mesh.evol), None, engine.stream())
     assert torch.equal(J[:, :K], ref[:, :K])
+
+
+@pytest.mark.parametrize("mesh_kind", ["box", "delaunay"])
+@pytest.mark.parametrize("ns,nd,cplx", [(1, 1, False), (2, 3, True), (3, 4, False), (5, 7, False), (5, 7, True),
+                                        (11, 13, False), (11, 13, True), (33, 17, False), (33, 17, True),
+                                        (63, 61, False), (63, 61, True), (7, 64, False), (7, 64, True)])
+def test_grid_jacobian_rows_at_any_counts(ns, nd, cplx, mesh_kind, monkeypatch):
+    """Counts that are no multiples of 4 (and tiles too empty for the kernel):
+    rb_jac's rows, pair by pair, bit for bit, at an even and an odd row stride
+    of the fields."""
+    monkeypatch.setattr(engine, "JAC_GRID_NODES", 1)
+    mesh = engine.mesh_of(_mesh((6, 5, 4)) if mesh_kind == "box" else _delaunay_cfg())
+    dt = torch.complex128 if cplx else torch.float64
+    kind = engine._lib.RB_JAC_SPLIT_F32_ACC64 if cplx else engine._lib.RB_JAC_F32_ACC64
+    s, d = np.meshgrid(np.arange(ns), ns + np.arange(nd))
+    sd = np.column_stack([s.ravel(), d.ravel(), np.ones(ns * nd)])
+    for ld in (ns + nd + (ns + nd) % 2, ns + nd + 1 - (ns + nd) % 2):
+        g = torch.Generator("cuda").manual_seed(ld)
+        phi = torch.randn((mesh.nn, ld), generator=g, device="cuda", dtype=dt)
+        J, K = engine.jacobian_matrix(mesh, phi, sd, ("mua",), "exact", acc64=True)
+        cols, det0, ndet, psrc, pdet, colsd, ps, pd, _ = engine._pair_dev(sd, phi.device)
+        ref = torch.full_like(J, float("nan"))
+        engine.call("rb_jac", engine.ctypes.byref(mesh.struct), engine._lib.RB_JAC_MUA_NODAL, engine.ptr(phi),
+                    engine._lib.RB_C128 if cplx else engine._lib.RB_F64, ld, engine.ptr(colsd), len(cols), det0, ndet,
+                    engine.ptr(ps), engine.ptr(pd), ns * nd, engine.ptr(ref), ref.shape[1], kind, mesh.rmax, mesh.emax,
+                    engine.ptr(mesh.evol), None, engine.stream())
+        assert torch.equal(J[:, :K], ref[:, :K]), ld
