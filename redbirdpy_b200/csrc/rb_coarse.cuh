@@ -36,10 +36,9 @@ constexpr int kCoarseSplits = 8;  // most K splits of the X rc product
 // 0.0625 ms per iteration with the scaled epilogue).
 template <typename T, int BN, bool SCALE>
 __global__ void __launch_bounds__(256) gemm_tn_kernel(int64_t m, int64_t n, int64_t kk, T alpha,
-                                                      const T* __restrict__ AT, int64_t lda, const T* __restrict__ B,
-                                                      int64_t ldb, T beta, int beta_zero, T* __restrict__ C,
-                                                      int64_t ldc, int64_t kchunk, int64_t cstride,
-                                                      const int32_t* __restrict__ live) {
+                                                      const T* AT, int64_t lda, const T* B, int64_t ldb, T beta,
+                                                      int beta_zero, T* C, int64_t ldc, int64_t kchunk,
+                                                      int64_t cstride, const int32_t* live) {
   chain_wait();
   if (chain_dead(live)) return;  // inside the Krylov loop: every column converged
   constexpr int BM = 64, BK = 16, TM = 4, TN = BN / 16;
@@ -159,7 +158,7 @@ __device__ __forceinline__ cdouble s_neg(cdouble a) { return make_double2(-a.x, 
 // copies of the block in shared memory, each entry read and written per pivot,
 // it took 56 us (complex 88), now 27 (63).
 template <typename T>
-__global__ void __launch_bounds__(256) gj_diag_kernel(const T* __restrict__ A, int64_t lda, int64_t b0, int nb,
+__global__ void __launch_bounds__(256) gj_diag_kernel(const T* A, int64_t lda, int64_t b0, int nb,
                                                       T* __restrict__ Dinv, int* __restrict__ err) {
   constexpr int R = kGjB / 4;  // rows of a thread
   __shared__ __align__(16) T row[2][kGjB], col[2][4][R];
@@ -217,7 +216,7 @@ __global__ void __launch_bounds__(256) gj_diag_kernel(const T* __restrict__ A, i
 // CbT[j][i] = A[i][b0 + j], the block column transposed (rows of the block
 // itself zero); kGjB x nc, ld nc
 template <typename T>
-__global__ void gj_cols_kernel(const T* __restrict__ A, int64_t nc, int64_t b0, int nb, T* __restrict__ CbT) {
+__global__ void gj_cols_kernel(const T* A, int64_t nc, int64_t b0, int nb, T* __restrict__ CbT) {
   chain_wait();
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nc * kGjB;
        e += (int64_t)gridDim.x * blockDim.x) {
@@ -229,8 +228,7 @@ __global__ void gj_cols_kernel(const T* __restrict__ A, int64_t nc, int64_t b0, 
 
 // A[b0 + i][:] = R[i][:]  and  A[b0 + i][b0 + j] = Dinv[i][j]
 template <typename T>
-__global__ void gj_rows_kernel(T* __restrict__ A, int64_t nc, int64_t b0, int nb, const T* __restrict__ R,
-                               const T* __restrict__ Dinv) {
+__global__ void gj_rows_kernel(T* __restrict__ A, int64_t nc, int64_t b0, int nb, const T* R, const T* Dinv) {
   chain_wait();
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < (int64_t)nb * nc;
        e += (int64_t)gridDim.x * blockDim.x) {
@@ -307,10 +305,10 @@ __global__ void cast_kernel(int64_t count, const T64* __restrict__ a, T* __restr
 // most warps of a 40-row aggregate idle: 13 us per call at 126 aggregates of
 // 5,775 rows x 40 columns, 4 us now.)
 template <typename T>
-__global__ void __launch_bounds__(256) restrict_kernel(int64_t nc, int64_t k, const T* __restrict__ R,
+__global__ void __launch_bounds__(256) restrict_kernel(int64_t nc, int64_t k, const T* R,
                                                        const int32_t* __restrict__ agg_ptr,
                                                        const int32_t* __restrict__ agg_rows, T* __restrict__ rc,
-                                                       const int32_t* __restrict__ live) {
+                                                       const int32_t* live) {
   chain_wait();
   if (chain_dead(live)) return;  // inside the Krylov loop: every column converged
   typedef typename Scalar<T>::acc A;
@@ -359,11 +357,10 @@ __global__ void __launch_bounds__(256) restrict_kernel(int64_t nc, int64_t k, co
 // part[block][c] = sum over this block's aggregates of rc[I][c] ec[I][c] (unconjugated)
 constexpr int kCdotGrid = 256;  // one aggregate per warp at nc = 2048
 template <typename T>
-__global__ void __launch_bounds__(256) coarse_dot_kernel(int64_t nc, int64_t k, const T* __restrict__ rc,
-                                                         const T* __restrict__ es, int splits,
-                                                         T* __restrict__ ec,
+__global__ void __launch_bounds__(256) coarse_dot_kernel(int64_t nc, int64_t k, const T* rc, const T* es,
+                                                         int splits, T* __restrict__ ec,
                                                          typename Scalar<T>::acc* __restrict__ part,
-                                                         const int32_t* __restrict__ live) {
+                                                         const int32_t* live) {
   chain_wait();
   if (chain_dead(live)) return;  // inside the Krylov loop: every column converged
   typedef typename Scalar<T>::acc A;

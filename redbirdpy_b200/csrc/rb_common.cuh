@@ -39,7 +39,10 @@ int fail(int code, const char* fmt, ...);
 // Such a kernel calls chain_wait() before it touches memory: it returns once
 // the predecessor has ended and its writes are visible, and since that one
 // waited too, so have all before it.  The call also lets the next kernel be
-// scheduled.  Without the launch attribute it does nothing.
+// scheduled.  Without the launch attribute it does nothing.  What the chain's
+// kernels hand on is never read through the read-only path (__ldg, or const
+// pointers with __restrict__): that asks for memory that nothing writes while
+// the kernel is resident, and its loads need not stay behind the wait.
 __device__ __forceinline__ void chain_wait() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");

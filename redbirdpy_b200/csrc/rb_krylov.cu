@@ -37,6 +37,33 @@ template <> struct BpsSpmm<cdouble> { static constexpr int value = 3; };
 constexpr int kGridMax = 148 * 8;       // upper bound of any grid (partials arrays)
 
 // ----------------------------------------------------------- vector access
+// ldv: arrays that nothing writes while the kernel is resident (the read-only
+// path).  ldv_w: arrays that this kernel or the one before it writes; with
+// early launches (launch_early) the one before is still running when a kernel
+// becomes resident, so what the chain's kernels hand on is read this way, from
+// pointers without __restrict__ (whose loads a compiler may turn into
+// read-only ones).  Volatile: the loads stay behind chain_wait and are issued
+// together where they stand, not sunk to their uses (vc_restrict_kernel).
+template <typename T, int V>
+__device__ __forceinline__ void ldv_w(const T* p, T (&o)[V]) {
+  constexpr int B = V * (int)sizeof(T);
+  uint32_t* d = reinterpret_cast<uint32_t*>(o);
+  const char* q = reinterpret_cast<const char*>(p);
+  if constexpr (B % 16 == 0) {
+#pragma unroll
+    for (int j = 0; j < B / 16; ++j)
+      asm volatile("ld.global.v4.b32 {%0, %1, %2, %3}, [%4];"
+                   : "=r"(d[4 * j]), "=r"(d[4 * j + 1]), "=r"(d[4 * j + 2]), "=r"(d[4 * j + 3])
+                   : "l"(q + 16 * j));
+  } else if constexpr (B % 8 == 0) {
+#pragma unroll
+    for (int j = 0; j < B / 8; ++j)
+      asm volatile("ld.global.v2.b32 {%0, %1}, [%2];" : "=r"(d[2 * j]), "=r"(d[2 * j + 1]) : "l"(q + 8 * j));
+  } else {
+#pragma unroll
+    for (int j = 0; j < B / 4; ++j) asm volatile("ld.global.b32 %0, [%1];" : "=r"(d[j]) : "l"(q + 4 * j));
+  }
+}
 template <typename T, int V>
 __device__ __forceinline__ void ldv(const T* __restrict__ p, T (&o)[V]) {
   constexpr int B = V * (int)sizeof(T);
@@ -149,10 +176,16 @@ enum { EPI_STORE = 0, EPI_PQDOT = 1, EPI_RESID = 2 };
 template <typename T, int L, int V, int EPI, int S = 1, bool O32 = true>
 __global__ void __launch_bounds__(kBlk, BpsSpmm<T>::value)
 spmm_kernel(int64_t n, int64_t k, const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices,
-            const T* __restrict__ val, const T* __restrict__ X, T* __restrict__ Y,
-            const double* __restrict__ B, void* __restrict__ part_, const int32_t* __restrict__ live) {
+            const T* __restrict__ val, const T* X, T* __restrict__ Y, const double* __restrict__ B,
+            void* __restrict__ part_, const int32_t* live) {
   chain_wait();
   if (chain_dead(live)) return;  // every column converged: a no-op iteration
+  // x is another kernel's output where this one can be launched early: FP32
+  // products of a cycle solve (n k < 2^31)
+  auto ldx = [](const T* p, T(&o)[V]) {
+    if constexpr (EPI == EPI_PQDOT && O32 && std::is_same<typename Scalar<T>::real, float>::value) ldv_w<T, V>(p, o);
+    else ldv<T, V>(p, o);
+  };
   // residual norms accumulate |r|^2 in double; dot products in the acc type
   typedef std::conditional_t<EPI == EPI_RESID, double, typename Scalar<T>::acc> A;
   A* part = reinterpret_cast<A*>(part_);
@@ -262,7 +295,7 @@ spmm_kernel(int64_t n, int64_t k, const int32_t* __restrict__ indptr, const int3
 #pragma unroll
             for (int u = 0; u < U; ++u) {
               const T* src = O32 ? xl + (uint32_t)oo[u] : xl + (int64_t)oo[u] * k;
-              ldv<T, V>(src, xv[u]);
+              ldx(src, xv[u]);
             }
 #pragma unroll
             for (int u = 0; u < U; ++u)
@@ -285,7 +318,7 @@ spmm_kernel(int64_t n, int64_t k, const int32_t* __restrict__ indptr, const int3
       for (int32_t p = b; p < e; ++p) {
         const T a = val[p];
         alignas(16) T xv[V];
-        ldv<T, V>(X + (int64_t)indices[p] * k + c0, xv);
+        ldx(X + (int64_t)indices[p] * k + c0, xv);
 #pragma unroll
         for (int j = 0; j < V; ++j) y[j] = s_fma(a, xv[j], y[j]);
       }
@@ -310,7 +343,7 @@ spmm_kernel(int64_t n, int64_t k, const int32_t* __restrict__ indptr, const int3
       }
       if constexpr (EPI == EPI_PQDOT) {
         alignas(16) T xv[V];
-        ldv<T, V>(X + row * k + c0, xv);
+        ldx(X + row * k + c0, xv);
 #pragma unroll
         for (int j = 0; j < V; ++j) {
           if constexpr (EPI == EPI_PQDOT) acc[j] = acc_fma(xv[j], y[j], acc[j]);
@@ -639,8 +672,7 @@ constexpr size_t grp_smem_bytes() {
 template <typename T, int EPI>
 __global__ void __launch_bounds__(kBlk, BpsSpmm<T>::value)
 spmm_pair_kernel(int64_t n, int64_t k, const int32_t* __restrict__ indptr, const T* __restrict__ val, GroupPlan gp,
-                 const T* __restrict__ X, T* __restrict__ Y, void* __restrict__ part_,
-                 const int32_t* __restrict__ live) {
+                 const T* X, T* __restrict__ Y, void* __restrict__ part_, const int32_t* live) {
   chain_wait();
   if (chain_dead(live)) return;  // every column converged: a no-op iteration
   constexpr int V = PairCfg<T>::V, S = PairCfg<T>::S, U = 8;
@@ -697,7 +729,7 @@ spmm_pair_kernel(int64_t n, int64_t k, const int32_t* __restrict__ indptr, const
         if (on) {
           alignas(16) T xv[U][V];
 #pragma unroll
-          for (int u = 0; u < U; ++u) ldv<T, V>(xl + (uint32_t)oo[u], xv[u]);
+          for (int u = 0; u < U; ++u) ldv_w<T, V>(xl + (uint32_t)oo[u], xv[u]);
           alignas(16) T aa[U], bbv[U];
           ldv_s<T, U>(wa + j, aa);
           ldv_s<T, U>(wb + j, bbv);
@@ -714,12 +746,12 @@ spmm_pair_kernel(int64_t n, int64_t k, const int32_t* __restrict__ indptr, const
     }
     if (on) {
       alignas(16) T pv[V];
-      ldv<T, V>(X + r0 * k + c0, pv);
+      ldv_w<T, V>(X + r0 * k + c0, pv);
 #pragma unroll
       for (int j = 0; j < V; ++j) acc[j] = acc_fma(pv[j], ya[j], acc[j]);
       stv<T, V>(Y + r0 * k + c0, ya);
       if (has1) {
-        ldv<T, V>(X + (r0 + 1) * k + c0, pv);
+        ldv_w<T, V>(X + (r0 + 1) * k + c0, pv);
 #pragma unroll
         for (int j = 0; j < V; ++j) acc[j] = acc_fma(pv[j], yb[j], acc[j]);
         stv<T, V>(Y + (r0 + 1) * k + c0, yb);
@@ -1115,7 +1147,7 @@ __global__ void fin_init_kernel(int64_t k, int nb, const A* part_rz, const doubl
 // leaves 1184 partials per column).  The sum is valid in thread 0.
 constexpr int kFinThreads = 256;
 template <typename A>
-__device__ __forceinline__ cdouble block_sum_part(const A* __restrict__ part, int nb, int64_t k, int64_t c) {
+__device__ __forceinline__ cdouble block_sum_part(const A* part, int nb, int64_t k, int64_t c) {
   __shared__ cdouble red[kFinThreads / 32];
   A s0 = acc_zero<A>(), s1 = acc_zero<A>();
   int b = threadIdx.x;
@@ -1138,7 +1170,7 @@ __device__ __forceinline__ cdouble block_sum_part(const A* __restrict__ part, in
 // into (its previous readers, the kernels of the iteration before, are done)
 template <typename A>
 __global__ void __launch_bounds__(kFinThreads) fin_alpha_kernel(int64_t k, int nb, const A* part_pq, ColState* cs,
-                                                               int32_t* __restrict__ clear) {
+                                                               int32_t* clear) {
   chain_wait();
   if (clear && blockIdx.x == 0 && threadIdx.x == 0) *clear = 0;
   const int64_t c = blockIdx.x;

@@ -118,13 +118,6 @@ static size_t vc_carve(Carver& cv, VcBufs<T64, T>& b, int64_t n, int64_t nnz, in
   return coarse_carve(cv, b.cb, nc, k);
 }
 
-// a vector load of memory that the same kernel writes (no read-only path)
-template <typename T, int V>
-__device__ __forceinline__ void ldv_rw(const T* p, T (&o)[V]) {
-  static_assert(V * sizeof(T) == 16, "16 bytes per lane");
-  *reinterpret_cast<int4*>(o) = *reinterpret_cast<const int4*>(p);
-}
-
 // ----------------------------------------------------------------- setup
 __device__ __forceinline__ double c_abs(double v) { return fabs(v); }
 __device__ __forceinline__ double c_abs(cdouble v) { return sqrt(v.x * v.x + v.y * v.y); }
@@ -331,7 +324,7 @@ __device__ __forceinline__ void g_walk(GAcc<T, V, NR>& acc, int32_t ub, int32_t 
       if (on) {
         alignas(16) T xv[U][V];
 #pragma unroll
-        for (int u = 0; u < U; ++u) ldv<T, V>(xl + (uint32_t)oo[u], xv[u]);
+        for (int u = 0; u < U; ++u) ldv_w<T, V>(xl + (uint32_t)oo[u], xv[u]);
 #pragma unroll
         for (int u = 0; u < U; ++u) acc.add(s_cf + (j + u) * NR, xv[u], (m4 >> (8 * u)) & 0xffu);
       }
@@ -358,8 +351,8 @@ __device__ __forceinline__ void g_walk(GAcc<T, V, NR>& acc, int32_t ub, int32_t 
 // right-hand side f^ = S1 P1^T S^-1 (x - w y) from the rows in registers.
 template <bool MID>
 __global__ void __launch_bounds__(kBlk, 3)
-vc_spmm_kernel(int64_t k, VcOp<float> o, const float* __restrict__ X, float* __restrict__ Y,
-               double* __restrict__ part, const int32_t* __restrict__ live) {
+vc_spmm_kernel(int64_t k, VcOp<float> o, const float* X, float* __restrict__ Y,
+               double* __restrict__ part, const int32_t* live) {
   chain_wait();
   if (chain_dead(live)) return;
   constexpr int V = 4, L = 32;
@@ -384,7 +377,7 @@ vc_spmm_kernel(int64_t k, VcOp<float> o, const float* __restrict__ X, float* __r
       const int32_t row = o.rg.rows[g * kRG + r];
       if (row < 0) continue;
       alignas(16) float xv[V], yv[V];
-      ldv<float, V>(X + (int64_t)row * k + c0, xv);
+      ldv_w<float, V>(X + (int64_t)row * k + c0, xv);
       const float is = MID ? o.is[row] : 0.f;
 #pragma unroll
       for (int q = 0; q < V; ++q) {
@@ -408,7 +401,7 @@ vc_spmm_kernel(int64_t k, VcOp<float> o, const float* __restrict__ X, float* __r
 // f^ = S1 P1^T S^-1 (r - w t), a group per lane group (after a row-wise t)
 template <typename T, int L, int S>
 __global__ void __launch_bounds__(kBlk)
-vc_restrict_kernel(int64_t k, VcOp<T> o, const T* __restrict__ R, const int32_t* __restrict__ live) {
+vc_restrict_kernel(int64_t k, VcOp<T> o, const T* R, const int32_t* live) {
   chain_wait();
   if (chain_dead(live)) return;
   constexpr int V = 16 / (int)sizeof(T);
@@ -419,6 +412,7 @@ vc_restrict_kernel(int64_t k, VcOp<T> o, const T* __restrict__ R, const int32_t*
   const float w = o.par->w;
   for (int64_t task = task0; task < o.ng * S; task += tasks) {
     const int64_t g = task / S;
+    const int32_t row0 = max(o.rg.rows[g * kRG], 0);  // (a group has at least one row, and its rows come first)
     alignas(16) T f[V];
 #pragma unroll
     for (int q = 0; q < V; ++q) f[q] = s_zero(T());
@@ -429,14 +423,12 @@ vc_restrict_kernel(int64_t k, VcOp<T> o, const T* __restrict__ R, const int32_t*
 #pragma unroll
       for (int r = 0; r < 4; ++r) {
         const int32_t row = o.rg.rows[g * kRG + h + r];
-        const int64_t at = (int64_t)max(row, 0) * k + c0;
-        ldv<T, V>(R + at, rv[r]);
-        ldv<T, V>(o.t + at, tv[r]);
-        is[r] = row >= 0 ? o.is[row] : s_zero(T());
-        if (row < 0) {  // an empty slot adds exact zeros
-#pragma unroll
-          for (int q = 0; q < V; ++q) rv[r][q] = tv[r][q] = s_zero(T());
-        }
+        // an empty slot repeats the group's first row at coefficient 0
+        const int64_t at = (int64_t)(row >= 0 ? row : row0) * k + c0;
+        ldv_w<T, V>(R + at, rv[r]);
+        ldv_w<T, V>(o.t + at, tv[r]);
+        const T s = o.is[row >= 0 ? row : row0];
+        is[r] = row >= 0 ? s : s_zero(T());
       }
 #pragma unroll
       for (int r = 0; r < 4; ++r)
@@ -460,8 +452,7 @@ vc_restrict_kernel(int64_t k, VcOp<T> o, const T* __restrict__ R, const int32_t*
 constexpr int kPupRows = 4;
 template <typename T, int L, int S>
 __global__ void __launch_bounds__(kBlk, 2)
-vc_pupdate_kernel(int64_t k, VcOp<T> o, const ColState* __restrict__ cs, const T* __restrict__ R, T* __restrict__ P,
-                  T* __restrict__ Xs) {
+vc_pupdate_kernel(int64_t k, VcOp<T> o, const ColState* cs, const T* R, T* P, T* Xs) {
   chain_wait();
   constexpr int V = 16 / (int)sizeof(T), NR = kPupRows, H = kRG / NR;
   RB_G_TASK(T, L, V, S);
@@ -491,14 +482,14 @@ vc_pupdate_kernel(int64_t k, VcOp<T> o, const ColState* __restrict__ cs, const T
 #pragma unroll
       for (int r = 0; r < NR; ++r) {
         const int64_t at = (int64_t)max(row[r], 0) * k + c0;
-        ldv_rw<T, V>(P + at, p[r]);
-        if (any & 2) ldv_rw<T, V>(Xs + at, x[r]);
+        ldv_w<T, V>(P + at, p[r]);
+        if (any & 2) ldv_w<T, V>(Xs + at, x[r]);
         if (any & 1) {
-          ldv<T, V>(R + at, rv[r]);
-          ldv<T, V>(o.t + at, tv[r]);
+          ldv_w<T, V>(R + at, rv[r]);
+          ldv_w<T, V>(o.t + at, tv[r]);
         }
       }
-      if (any & 1) ldv<T, V>(o.e + g * k + c0, eg);
+      if (any & 1) ldv_w<T, V>(o.e + g * k + c0, eg);
     }
     GAcc<T, V, NR> a;
     a.clear();
@@ -535,8 +526,8 @@ vc_pupdate_kernel(int64_t k, VcOp<T> o, const ColState* __restrict__ cs, const T
 // (INIT: the sums alone); rows in order
 template <typename T, int L, int S, bool INIT>
 __global__ void __launch_bounds__(kBlk, 4)
-vc_update_kernel(int64_t n, int64_t k, const ColState* __restrict__ cs, T* __restrict__ R, const T* __restrict__ Q,
-                 double* __restrict__ part, cdouble* __restrict__ part_u, const int32_t* __restrict__ live) {
+vc_update_kernel(int64_t n, int64_t k, const ColState* cs, T* R, const T* Q, double* __restrict__ part,
+                 cdouble* __restrict__ part_u, const int32_t* live) {
   chain_wait();
   if (chain_dead(live)) return;
   constexpr int V = 16 / (int)sizeof(T);
@@ -562,23 +553,32 @@ vc_update_kernel(int64_t n, int64_t k, const ColState* __restrict__ cs, T* __res
     acu[q] = make_double2(0.0, 0.0);
   }
   if (on) {
-#pragma unroll 2
-    for (int64_t task = task0; task < n * S; task += tasks) {
-      const int64_t at = task / S * k + c0;
-      alignas(16) T r[V], q_[V];
-      ldv<T, V>(R + at, r);
-      if (!INIT) {
-        ldv<T, V>(Q + at, q_);
+    // two rows at a time, all their loads before the first store
+    for (int64_t task = task0; task < n * S; task += 2 * tasks) {
+      const bool two = task + tasks < n * S;
+      alignas(16) T r[2][V], q_[2][V];
 #pragma unroll
-        for (int q = 0; q < V; ++q)
-          if (act[q]) r[q] = s_sub(r[q], s_mul(al[q], q_[q]));
-        stv<T, V>(R + at, r);
-      }
+      for (int u = 0; u < 2; ++u)
+        if (u == 0 || two) {
+          const int64_t at = (task + u * tasks) / S * k + c0;
+          ldv_w<T, V>(R + at, r[u]);
+          if (!INIT) ldv_w<T, V>(Q + at, q_[u]);
+        }
 #pragma unroll
-      for (int q = 0; q < V; ++q) {
-        acc[q] += s_abs2(r[q]);
-        if constexpr (CX) acu[q] = acc_fma(r[q], r[q], acu[q]);
-      }
+      for (int u = 0; u < 2; ++u)
+        if (u == 0 || two) {
+          if (!INIT) {
+#pragma unroll
+            for (int q = 0; q < V; ++q)
+              if (act[q]) r[u][q] = s_sub(r[u][q], s_mul(al[q], q_[u][q]));
+            stv<T, V>(R + (task + u * tasks) / S * k + c0, r[u]);
+          }
+#pragma unroll
+          for (int q = 0; q < V; ++q) {
+            acc[q] += s_abs2(r[u][q]);
+            if constexpr (CX) acu[q] = acc_fma(r[u][q], r[u][q], acu[q]);
+          }
+        }
     }
   }
   block_colreduce<double, L, V, S>(acc, part, k, sm);
@@ -590,10 +590,10 @@ vc_update_kernel(int64_t n, int64_t k, const ColState* __restrict__ cs, T* __res
 // before the scale) . F
 template <typename T, int L, int S, bool DOT>
 __global__ void __launch_bounds__(kBlk, 4)
-vc_mid_spmm_kernel(int64_t k, VcOp<T> o, const T* __restrict__ U, const float* __restrict__ cu,
-                   const T* __restrict__ W, const float* __restrict__ cw, const T* __restrict__ G,
-                   const float* __restrict__ cg, const T* __restrict__ rowscale, T* __restrict__ out,
-                   typename Scalar<T>::acc* __restrict__ part, const int32_t* __restrict__ live) {
+vc_mid_spmm_kernel(int64_t k, VcOp<T> o, const T* U, const float* __restrict__ cu, const T* W,
+                   const float* __restrict__ cw, const T* G, const float* __restrict__ cg,
+                   const T* __restrict__ rowscale, T* __restrict__ out,
+                   typename Scalar<T>::acc* __restrict__ part, const int32_t* live) {
   chain_wait();
   if (chain_dead(live)) return;
   constexpr int V = 16 / (int)sizeof(T);
@@ -614,12 +614,12 @@ vc_mid_spmm_kernel(int64_t k, VcOp<T> o, const T* __restrict__ U, const float* _
       alignas(16) T y[V], u[V];
 #pragma unroll
       for (int q = 0; q < V; ++q) y[q] = s_zero(T());
-      ldv<T, V>(U + g * k + c0, u);
+      ldv_w<T, V>(U + g * k + c0, u);
 #pragma unroll 4
       for (int32_t p = b; p < e; ++p) {
         const T a = o.v1[p];
         alignas(16) T x[V];
-        ldv<T, V>(G + (int64_t)o.mcol[p] * k + c0, x);
+        ldv_w<T, V>(G + (int64_t)o.mcol[p] * k + c0, x);
 #pragma unroll
         for (int q = 0; q < V; ++q) y[q] = s_fma(a, x[q], y[q]);
       }
@@ -627,13 +627,13 @@ vc_mid_spmm_kernel(int64_t k, VcOp<T> o, const T* __restrict__ U, const float* _
       for (int q = 0; q < V; ++q) y[q] = s_add(r_mul(fg, y[q]), r_mul(fu, u[q]));
       if (W) {
         alignas(16) T v[V];
-        ldv<T, V>(W + g * k + c0, v);
+        ldv_w<T, V>(W + g * k + c0, v);
 #pragma unroll
         for (int q = 0; q < V; ++q) y[q] = s_add(y[q], r_mul(fw, v[q]));
       }
       if (DOT) {
         alignas(16) T f[V];
-        ldv<T, V>(o.f + g * k + c0, f);
+        ldv_w<T, V>(o.f + g * k + c0, f);
 #pragma unroll
         for (int q = 0; q < V; ++q) acc[q] = acc_fma(y[q], f[q], acc[q]);
       }
@@ -650,8 +650,8 @@ vc_mid_spmm_kernel(int64_t k, VcOp<T> o, const T* __restrict__ U, const float* _
 
 // x2 += S1^-1 P2 ec
 template <typename T>
-__global__ void vc_prolong_kernel(int64_t ng, int64_t k, const int32_t* __restrict__ agg, const T* __restrict__ ec,
-                                  const T* __restrict__ is1, T* __restrict__ x2, const int32_t* __restrict__ live) {
+__global__ void vc_prolong_kernel(int64_t ng, int64_t k, const int32_t* __restrict__ agg, const T* ec,
+                                  const T* __restrict__ is1, T* x2, const int32_t* live) {
   chain_wait();
   if (chain_dead(live)) return;
   constexpr int V = 16 / (int)sizeof(T);
@@ -660,8 +660,8 @@ __global__ void vc_prolong_kernel(int64_t ng, int64_t k, const int32_t* __restri
     const int64_t g = i / kv, c = (i - g * kv) * V;
     const T s = is1[g];
     alignas(16) T x[V], e[V];
-    ldv<T, V>(x2 + g * k + c, x);
-    ldv<T, V>(ec + (int64_t)agg[g] * k + c, e);
+    ldv_w<T, V>(x2 + g * k + c, x);
+    ldv_w<T, V>(ec + (int64_t)agg[g] * k + c, e);
 #pragma unroll
     for (int q = 0; q < V; ++q) x[q] = s_fma(s, e[q], x[q]);
     stv<T, V>(x2 + g * k + c, x);
