@@ -772,7 +772,8 @@ __global__ void vc_seg_factor_kernel(int64_t m, const OuterState* __restrict__ s
 }
 
 // r^ = T(S R64 scale) for active columns, 0 elsewhere; x = p = 0.  RT: the
-// residual's type (double for the right-hand side of a first sweep from 0);
+// residual's type (double for the right-hand side of a first sweep from 0,
+// the caller's array: read in 16-byte loads only where it lies on 16 bytes);
 // rinst / segf: the rows' instances and their factors, or NULL
 template <typename T64, typename RT, typename T>
 __global__ void __launch_bounds__(256)
@@ -782,6 +783,7 @@ vc_cast_kernel(int64_t n, int64_t k, const RT* __restrict__ R64, const T64* __re
   constexpr int V = 16 / (int)sizeof(T);
   __shared__ double fac[kMaxCols];
   if (!rinst) vc_factors<false>(k, os, fac);
+  const bool wide = (reinterpret_cast<uintptr_t>(R64) & 15) == 0;
   const int64_t kv = k / V;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n * kv; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t row = i / kv, c = (i - row * kv) * V;
@@ -789,7 +791,12 @@ vc_cast_kernel(int64_t n, int64_t k, const RT* __restrict__ R64, const T64* __re
     const T64 s = s64[row];
     alignas(16) RT v[V];
     alignas(16) T o[V], z[V];
-    ldv<RT, V>(R64 + row * k + c, v);
+    if (wide) {
+      ldv<RT, V>(R64 + row * k + c, v);
+    } else {
+#pragma unroll
+      for (int q = 0; q < V; ++q) v[q] = R64[row * k + c + q];
+    }
 #pragma unroll
     for (int q = 0; q < V; ++q) {
       const double fq = f[q];  // (a done column's residual may be non-finite: 0, not 0 x it)

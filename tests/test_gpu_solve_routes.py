@@ -1,0 +1,50 @@
+"""Which form of the block solve a call takes, and what each form accepts."""
+
+import numpy as np
+import pytest
+import torch
+
+import redbirdpy_b200 as rbb
+from redbirdpy_b200 import engine
+from redbirdpy_b200.meshgen import kuhn_box
+
+pytestmark = pytest.mark.gpu
+
+
+def _matrix(cells, omega=0.0, seed=0):
+    """The device matrix of a homogeneous box (1.5 mm, jittered properties)."""
+    rng = np.random.default_rng(seed)
+    size = np.array(cells) * 1.5
+    node, elem = kuhn_box(size, 1.5)
+    nn = node.shape[0]
+    prop = np.column_stack([rng.uniform(0.008, 0.012, nn), rng.uniform(0.9, 1.1, nn), np.zeros(nn),
+                            np.full(nn, 1.37)])
+    pos = size[None] * [[0.4, 0.4, 0.0]]
+    cfg = dict(node=node, elem=elem, prop=prop, srcpos=pos, srcdir=np.array([[0, 0, 1.0]]), detpos=pos,
+               detdir=np.array([[0, 0, 1.0]]), omega=omega)
+    cfg, _ = rbb.meshprep(cfg)
+    mesh = engine.mesh_of(cfg)
+    return engine.assemble(mesh, engine.Optics.from_cfg(mesh, cfg))
+
+
+def _rhs(n, k, seed=0):
+    g = torch.Generator("cuda").manual_seed(seed)
+    B = torch.randn((n, k), generator=g, device="cuda", dtype=torch.float64)
+    return B * (torch.rand((n, k), generator=g, device="cuda") < 0.01)
+
+
+@pytest.mark.parametrize("omega", [0.0, 2 * np.pi * 1e8])
+@pytest.mark.parametrize("k", [4, 68])
+def test_cycle_solve_of_a_right_hand_side_off_16_bytes(k, omega, monkeypatch):
+    """A contiguous view that starts 8 bytes into its storage is solved like
+    its copy, bit for bit."""
+    monkeypatch.setattr(engine, "VCYCLE_ENTRIES", 0)
+    mat = _matrix((28, 27, 25), omega)
+    B = _rhs(mat.n, k)
+    view = torch.empty(mat.n * k + 1, dtype=torch.float64, device="cuda")[1:].view(mat.n, k)
+    view.copy_(B)
+    assert view.is_contiguous() and view.data_ptr() % 16 == 8
+    X, info = engine.solve(mat, B)
+    Y, info2 = engine.solve(mat, view)
+    assert info["coarse_nc"] > 0 and info2["coarse_nc"] > 0 and info["flag"] == 0
+    assert torch.equal(X, Y)
