@@ -437,7 +437,8 @@ template <typename T64, typename T>
 static int coarse_setup(const rb_csr& A, CoarseBufs<T64, T>& c, cudaStream_t st) {
   const int64_t nc = c.op.nc;
   const size_t rowb = (size_t)nc * sizeof(T64);
-  RB_CUDA_TRY(cudaFuncSetAttribute(coarse_build_kernel<T64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rowb));
+  constexpr int kRowMax = kCoarseMax * (int)sizeof(T64);
+  RB_CUDA_TRY(cudaFuncSetAttribute(coarse_build_kernel<T64>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowMax));
   coarse_build_kernel<T64><<<(unsigned)nc, 32, rowb, st>>>(nc, A.indptr, A.indices, (const T64*)A.val64, c.op.agg,
                                                            c.op.agg_ptr, c.op.agg_rows, c.A64);
   RB_LAUNCH_CHECK();

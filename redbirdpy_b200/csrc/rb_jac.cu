@@ -608,6 +608,10 @@ int* jac_err_word() {
   return cudaGetSymbolAddress(reinterpret_cast<void**>(&p), g_jac_tc_err) == cudaSuccess ? p : nullptr;
 }
 
+// dynamic shared memory at most (the functions' bound: set to the same value
+// by every call, so that no thread lowers it under another's launch)
+constexpr size_t kJacSmemMax = 200 * 1024, kJtcSmemMax = 220 * 1024;
+
 // launches the tensor-core form when the pairs are the full grid with FP32
 // output and the sizes fit it; returns 1 when it did not apply
 template <typename C, typename In>
@@ -617,13 +621,13 @@ static int launch_jac_tc(const JacArgs& a, const void* phi, void* J, cudaStream_
   const int nsu = a.det0;
   if (a.rmax > 32 || nsu < 1 || nsu > 128 || a.ndet > (Scalar<C>::is_complex ? 64 : 128)) return RB_OK;
   const JtcLayout T = jtc_layout<C>(a.rmax, a.nc, a.ndet, a.emax, nsu);
-  if (T.total > 220 * 1024) return RB_OK;
+  if (T.total > kJtcSmemMax) return RB_OK;
   uint32_t cols = 32;
   while (cols < (uint32_t)(kJtcTN * T.N)) cols <<= 1;
   if (cols > 512) return RB_OK;
   int* err = nullptr;
   RB_CUDA_TRY(cudaGetSymbolAddress(reinterpret_cast<void**>(&err), g_jac_tc_err));
-  RB_CUDA_TRY(cudaFuncSetAttribute(jac_tc_kernel<C, In>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T.total));
+  RB_CUDA_TRY(cudaFuncSetAttribute(jac_tc_kernel<C, In>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kJtcSmemMax));
   const unsigned g = (unsigned)ceil_div(a.nn - a.node0, kJtcTN);
   jac_tc_kernel<C, In><<<g, kJacThreads, T.total, st>>>(a, (const In*)phi, (float*)J, cols, err);
   RB_LAUNCH_CHECK();
@@ -637,12 +641,12 @@ static int launch_jac_t(const JacArgs& a, const void* phi, void* J, cudaStream_t
   const size_t budget = 110 * 1024;
   while (TN > 1 && jac_smem<C>(TN, a.rmax, a.nc, a.ndet, a.emax) > budget) TN >>= 1;
   const size_t sm = jac_smem<C>(TN, a.rmax, a.nc, a.ndet, a.emax);
-  if (sm > 200 * 1024) return fail(RB_ESIZE, "rb_jac: staging needs %zu bytes of shared memory", sm);
+  if (sm > kJacSmemMax) return fail(RB_ESIZE, "rb_jac: staging needs %zu bytes of shared memory", sm);
   const unsigned g = (unsigned)ceil_div(a.nn - a.node0, TN);
 #define RB_JL(TN_)                                                                                     \
   do {                                                                                                 \
     RB_CUDA_TRY(cudaFuncSetAttribute(jac_kernel<C, In, TN_, SPLIT, GRID, BF, NARROW>,                  \
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));           \
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kJacSmemMax));  \
     jac_kernel<C, In, TN_, SPLIT, GRID, BF, NARROW><<<g, kJacThreads, sm, st>>>(a, (const In*)phi, J);   \
   } while (0)
   switch (TN) {

@@ -451,7 +451,7 @@ static int jg_run(JgArgs a, int64_t node1, const C* phi, float* J, double* work,
     if (L.total > kJgSmem) return RB_OK;
   }
   auto kern = nbuf == 2 ? jac_grid_kernel<C, SPLIT, RM, TN, 2> : jac_grid_kernel<C, SPLIT, RM, TN, 1>;
-  RB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.total));
+  RB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kJgSmem));
   const int ntile = L.nst * L.ndt;
   const int64_t chunk = jg_chunk(a.rmax, RM);
   // node blocks start where the J column is a multiple of the block: the row's

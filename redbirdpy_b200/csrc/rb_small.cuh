@@ -678,7 +678,9 @@ static SmallPlan small_plan(int64_t n, int64_t nnz, int64_t k) {
 template <typename T64, typename T, int V, int RPT>
 static int small_launch_t(const SmallArgs<T64, T>& a, const SmallPlan& p, cudaStream_t st) {
   auto kern = small_solve_kernel<T64, T, V, RPT>;
-  RB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem));
+  // the bound is the same for every plan: it belongs to the function, not to
+  // the launch, and another thread's smaller plan must not lower it in between
+  RB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmBytes));
   RB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(ceil_div(a.k, V) * p.cl));

@@ -48,3 +48,34 @@ def test_cycle_solve_of_a_right_hand_side_off_16_bytes(k, omega, monkeypatch):
     Y, info2 = engine.solve(mat, view)
     assert info["coarse_nc"] > 0 and info2["coarse_nc"] > 0 and info["flag"] == 0
     assert torch.equal(X, Y)
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+def test_small_solves_of_different_sizes_from_several_threads(cplx):
+    """Solves whose plans need different amounts of shared memory, through
+    the same kernel, from threads of one process: each its own solution."""
+    import threading
+
+    omega = 2 * np.pi * 1e8 if cplx else 0.0
+    mats = [_matrix(c, omega) for c in ((4, 4, 3), (9, 8, 7), (12, 11, 10), (15, 14, 13))]
+    rhs = [_rhs(m.n, 2, seed=i) for i, m in enumerate(mats)]
+    want = [engine.solve(m, b)[0] for m, b in zip(mats, rhs)]
+    torch.cuda.synchronize()
+    bad = []
+
+    def work(i):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for _ in range(40):
+                    X, info = engine.solve(mats[i], rhs[i])
+                    if info["flag"] or info["launches"] != 2 or not torch.equal(X, want[i]):
+                        bad.append((i, info))
+        except Exception as e:  # a refused launch
+            bad.append((i, repr(e)))
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(mats))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad, bad[:3]
