@@ -381,6 +381,9 @@ size_t rb_femsolve_work_bytes(int64_t n, int64_t nnz, int64_t nrhs, int32_t is_c
 int rb_femsolve(const rb_csr* A, const double* B, void* X, int64_t nrhs,
                 const rb_solve_opts* opts, rb_solve_info* info /* host */, void* work,
                 size_t work_bytes, void* stream);
+/* 1 where rb_femsolve (mixed precision, no coarse space, groups, instances,
+ * profile, fixed budget or lane layout) solves nrhs columns in one launch. */
+int rb_femsolve_one_launch(int64_t n, int64_t nnz, int64_t nrhs, int32_t is_complex);
 /* rb_femsolve (mixed precision) with the three-level V-cycle preconditioner:
  * opts->coarse and groups must be NULL, check_every >= 1, and n x (nrhs
  * rounded up to 4) < 2^31.  work: rb_femsolve_mid_work_bytes, with instances

@@ -121,6 +121,7 @@ _SIGS = {
     "rb_midlevel_count": (ctypes.c_int, [ctypes.POINTER(RbRowGroups), _i64, _vp, _vp, ctypes.POINTER(_i64), _vp, _sz,
                                          _vp]),
     "rb_midlevel_fill": (ctypes.c_int, [ctypes.POINTER(RbRowGroups), _vp, _vp, _vp, _vp]),
+    "rb_femsolve_one_launch": (ctypes.c_int, [_i64, _i64, _i64, _i32]),
     "rb_femsolve_mid_work_bytes": (_sz, [ctypes.POINTER(RbCsr), ctypes.POINTER(RbMidlevel), _i64]),
     "rb_femsolve_mid": (ctypes.c_int, [ctypes.POINTER(RbCsr), ctypes.POINTER(RbMidlevel), _vp, _vp, _i64,
                                        ctypes.POINTER(RbSolveOpts), ctypes.POINTER(RbSolveInfo), _vp, _sz, _vp]),

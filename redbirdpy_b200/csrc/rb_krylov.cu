@@ -2279,14 +2279,14 @@ static int femsolve_t(const rb_csr& A, const double* B, T64* X, int64_t nrhs, co
   carve(cv, b, n, A.nnz, kb);
   if (!b.scan_work) return fail(RB_EARG, "rb_femsolve: workspace too small");
   // A small system without coarse space or instances: the whole solve in one
-  // launch (rb_small.cuh) where its clusters hold the matrix.  Options that
-  // ask for the separate kernels (their timing, a fixed budget, a lane
-  // layout) keep them.
+  // launch (rb_small.cuh) where its clusters hold the matrix and its columns
+  // do not take too many waves.  Options that ask for the separate kernels
+  // (their timing, a fixed budget, a lane layout, row groups) keep them.
   if constexpr (sizeof(T) != sizeof(T64)) {
-    if (!mid && !o.coarse && !o.instances && !o.profile && o.check_every > 0 && o.spmm_lanes == 0) {
+    if (!mid && !o.coarse && !o.groups && !o.instances && !o.profile && o.check_every > 0 && o.spmm_lanes == 0) {
       const SmallPlan sp = small_plan<T64, T>(n, A.nnz, nrhs);
       static_assert(sizeof(SmallOut) <= sizeof(ColState), "the outcome words share the column states' space");
-      if (sp.ok)
+      if (small_wins<T>(sp, n, A.nnz, nrhs))
         return solve_small<T64, T>(A, B, X, nrhs, o, info, reinterpret_cast<SmallOut*>(b.cs), val, dinv, sp, cv, st);
     }
   }
@@ -2467,6 +2467,12 @@ int rb_femsolve(const rb_csr* A, const double* B, void* X, int64_t nrhs, const r
                                       (const double*)A->val64, (const double*)A->dinv64, st);
   return femsolve_t<double, float>(*A, B, (double*)X, nrhs, o, *info, work, work_bytes,
                                    (const float*)A->val32, (const float*)A->dinv32, st);
+}
+
+int rb_femsolve_one_launch(int64_t n, int64_t nnz, int64_t nrhs, int32_t is_complex) {
+  if (n < 1 || nrhs < 1 || nrhs > kMaxCols) return 0;
+  return is_complex ? small_wins<cfloat>(small_plan<cdouble, cfloat>(n, nnz, nrhs), n, nnz, nrhs)
+                    : small_wins<float>(small_plan<double, float>(n, nnz, nrhs), n, nnz, nrhs);
 }
 
 size_t rb_femsolve_mid_work_bytes(const rb_csr* A, const rb_midlevel* mid, int64_t nrhs) {

@@ -562,7 +562,7 @@ __global__ void __launch_bounds__(kSmThreads, 1) small_solve_kernel(SmallArgs<T6
 // barriers, reductions and scalars, then a thread's entries, each a gather
 // and V products.
 template <typename T>
-static double small_time(int64_t nnz, int cl, int V, double waves, int64_t cap) {
+static double small_time(int64_t nnz, int cl, int V, double waves) {
   const double e = (double)nnz / cl / kSmThreads;
   return waves * (3.0 + 0.3 * V + e * (0.03 + (Scalar<T>::is_complex ? 0.08 : 0.055) * V));
 }
@@ -580,6 +580,7 @@ struct SmallPlan {
   bool ok = false;
   int cl = 0, V = 0, rpt = 0, nr = 0, cap = 0, slots = 0;
   size_t smem = 0;
+  double us = 0.0;  // model time of an iteration (small_time)
 };
 constexpr size_t kSmBytes = 227 * 1024 - 12 * 1024;  // dynamic shared memory beside the static arrays
 
@@ -658,10 +659,11 @@ static SmallPlan small_plan(int64_t n, int64_t nnz, int64_t k) {
       const int fit = small_fit<T64, T>(V, rpt, cl);
       if (fit < 1) continue;
       const double waves = (double)ceil_div(ceil_div(k, V), fit);
-      const double t = small_time<T>(nnz, cl, V, waves, cap);
+      const double t = small_time<T>(nnz, cl, V, waves);
       if (!p.ok || t < best) {
         best = t;
         p.ok = true;
+        p.us = t;
         p.cl = cl;
         p.V = V;
         p.rpt = rpt;
@@ -673,6 +675,26 @@ static SmallPlan small_plan(int64_t n, int64_t nnz, int64_t k) {
     }
   }
   return p;
+}
+
+// Whether a solve goes faster in one launch than by the separate kernels.
+// Their iteration takes about 28 us of launches and read-backs and, streaming
+// all columns in one wave, a time per row and column (half of it the product's:
+// per entry); the one launch's waves grow with the columns.  Fit on boxes of
+// 1,210 to 32,736 nodes x 1 to 128 columns; the separate kernels stop at their
+// next host check (15% more iterations) and the model above is a third low for
+// complex columns, four rows a thread.  Separate kernels / one launch, ms: real 9,261
+// x 128 7.5 / 5.3, 16,900 x 64 7.4 / 6.0, x 96 8.0 / 8.4, x 128 8.4 / 11.8, 24,273 x
+// 64 8.1 / 6.8, x 96 9.4 / 9.6, 32,736 x 48 8.8 / 7.5, x 64 9.3 / 9.1, x 128 11.8 /
+// 18.3; complex 9,261 x 96 8.1 / 7.2, x 128 8.9 / 8.8, 16,900 x 48 8.5 / 8.4, x 64
+// 9.3 / 10.4, x 128 12.0 / 20.5, 24,273 x 32 8.8 / 7.4, x 48 9.6 / 10.0, 32,736 x 32
+// 9.5 / 9.2, x 48 11.6 / 12.4, x 128 20.5 / 30.5.
+template <typename T>
+static bool small_wins(const SmallPlan& p, int64_t n, int64_t nnz, int64_t k) {
+  constexpr bool CX = Scalar<T>::is_complex;
+  const double work = 0.5 * (double)(n + nnz / 14.4) * (double)k;  // (14.4 entries per row of those boxes)
+  const double sep = CX ? 29.8 + 0.03 * k + 16.7e-6 * work : 28.4 + 0.05 * k + 6.3e-6 * work;
+  return p.ok && (CX ? 1.3 : 1.0) * p.us < 1.15 * sep;
 }
 
 template <typename T64, typename T, int V, int RPT>

@@ -957,13 +957,18 @@ def solve(mat, B, precision="mixed", tol=DEFAULT_TOL, inner_tol=None, maxiter=20
         inner_tol = 1e-5 if cs is not None or mid is not None else 1e-4
     if prec == _lib.RB_FP64 and inner_tol > 1e-6:
         inner_tol = max(tol, 1e-15)
-    rg = _resolve_groups(mat, groups) if prec == _lib.RB_MIXED and mid is None else None
+    def takes_one_launch(kb):
+        """Whether the library solves kb columns in one launch, which reads no row groups."""
+        return bool(prec == _lib.RB_MIXED and mid is None and cs is None and instances is None and budget is None
+                    and not profile and not spmm_lanes and groups in ("auto", None, False)
+                    and _lib.lib().rb_femsolve_one_launch(n, mat.struct.nnz, kb, int(mat.is_complex)))
+
+    rg = None
     if instances is not None and instances.n != n:
         raise ValueError("instances do not cover the matrix's rows")
     opts = _lib.RbSolveOpts(prec, int(max_outer), int(maxiter), int(check_every), float(tol), float(inner_tol),
                             int(bool(profile)), int(x0 is not None),
-                            ctypes.pointer(cs.struct) if cs is not None else None,
-                            ctypes.pointer(rg.struct) if rg is not None else None, None, int(spmm_lanes))
+                            ctypes.pointer(cs.struct) if cs is not None else None, None, None, int(spmm_lanes))
     inst_status, inst_relres = [], []
     for c0 in range(0, k, 128):
         kb = min(128, k - c0)
@@ -992,9 +997,8 @@ def solve(mat, B, precision="mixed", tol=DEFAULT_TOL, inner_tol=None, maxiter=20
                 # the cycle assumes a definite operator (positive diagonal,
                 # real part); what it does not solve gets the two-level form
                 work = None
-                cs, rg = _resolve_coarse(mat, coarse), _resolve_groups(mat, groups)
+                cs = _resolve_coarse(mat, coarse)
                 opts.coarse = ctypes.pointer(cs.struct) if cs is not None else None
-                opts.groups = ctypes.pointer(rg.struct) if rg is not None else None
                 mid = None
                 if x0 is not None:
                     Xb.copy_(x0[:, c0:c0 + kb])
@@ -1006,6 +1010,10 @@ def solve(mat, B, precision="mixed", tol=DEFAULT_TOL, inner_tol=None, maxiter=20
                 inst_status.append(instances.status.cpu().numpy())
                 inst_relres.append(rel)
             continue
+        if prec == _lib.RB_MIXED:
+            one = takes_one_launch(kb)
+            rg = rg if one or rg is not None else _resolve_groups(mat, groups)
+            opts.groups = ctypes.pointer(rg.struct) if rg is not None and not one else None
         wb = _lib.lib().rb_femsolve_work_bytes(n, mat.struct.nnz, kb, int(mat.is_complex), prec)
         if cs is not None:
             wb += _lib.lib().rb_coarse_work_bytes(cs.nc, kb, int(mat.is_complex), prec)

@@ -5,7 +5,7 @@ import pytest
 import torch
 
 import redbirdpy_b200 as rbb
-from redbirdpy_b200 import engine
+from redbirdpy_b200 import _lib, engine
 from redbirdpy_b200.meshgen import kuhn_box
 
 pytestmark = pytest.mark.gpu
@@ -79,3 +79,25 @@ def test_small_solves_of_different_sizes_from_several_threads(cplx):
     for t in threads:
         t.join()
     assert not bad, bad[:3]
+
+
+@pytest.mark.parametrize("cells,k,cplx,one", [((9, 9, 8), 128, False, True), ((20, 20, 20), 128, False, True),
+                                              ((25, 25, 24), 128, False, False), ((25, 25, 24), 128, True, False),
+                                              ((25, 25, 24), 8, True, True), ((32, 31, 30), 128, False, False),
+                                              ((32, 31, 30), 130, False, False), ((32, 31, 30), 16, False, True)])
+def test_wide_solves_leave_the_one_launch_form(cells, k, cplx, one):
+    """Jacobi solves whose columns would take many waves of the one launch run
+    the separate kernels; row groups asked for are used; every form refines to
+    a relative residual of 1e-15 (condition below 1e4: 1e-10 with a margin of 10)."""
+    mat = _matrix(cells, 2 * np.pi * 1e8 if cplx else 0.0)
+    B = _rhs(mat.n, k)
+    assert bool(_lib.lib().rb_femsolve_one_launch(mat.n, mat.struct.nnz, min(k, 128), int(cplx))) == one
+    X, info = engine.solve(mat, B, coarse=False, groups=None)
+    assert info["flag"] == 0 and (info["launches"] == 2) == one
+    Y, info2 = engine.solve(mat, B, coarse=False)
+    assert info2["flag"] == 0 and (info2["launches"] == 2) == one
+    assert float((X - Y).abs().max()) <= 1e-10 * float(X.abs().max())
+    if not cplx:
+        Z, info3 = engine.solve(mat, B, coarse=False, groups=mat.mesh.row_groups())
+        assert info3["flag"] == 0 and info3["launches"] > 2
+        assert float((X - Z).abs().max()) <= 1e-10 * float(X.abs().max())
