@@ -1189,25 +1189,39 @@ def _jac_what(name, mode):
 JAC_GRID_NODES = 8192
 
 
-def _jac_params(mesh, whats, phi, phi_kind, colsd, nc, det0, ndet, ps, pd, gnsd, J, ldj, out_kind, stride, node0, count):
-    """The rows of every parameter (rb_jac_multi), parameter p's columns from
-    p * stride."""
-    npar = len(whats)
+def _jac_grid_bytes(mesh, phi, det0, ndet, psrc, pdet, acc64, count):
+    """Workspace of the pipelined kernel (rb_jac_multi) for rows over ``count``
+    nodes, 0 where the general kernel forms them."""
+    if not acc64 or count < JAC_GRID_NODES or phi.dtype not in (torch.float64, torch.complex128):
+        return 0
     wb = _lib.lib().rb_jac_multi_work_bytes(mesh.rmax, det0, ndet, int(phi.is_complex()))
-    if gnsd >= 0 or count < JAC_GRID_NODES or out_kind not in (_lib.RB_JAC_SPLIT_F32_ACC64, _lib.RB_JAC_F32_ACC64):
-        wb = 0  # not the pipelined kernel's: no workspace
-    work = torch.empty(wb, dtype=torch.uint8, device=phi.device) if wb else None
-    need_ddd = _lib.RB_JAC_D in whats
-    call("rb_jac_multi", ctypes.byref(mesh.struct), npar, (ctypes.c_int32 * npar)(*whats),
-         (ctypes.c_int64 * npar)(*(p * stride for p in range(npar))), ptr(phi), phi_kind, phi.shape[1], ptr(colsd), nc,
-         det0, ndet, ptr(ps), ptr(pd), gnsd, ptr(J), ldj, out_kind, mesh.rmax, mesh.emax, ptr(mesh.evol),
-         ptr(mesh.ddd if need_ddd else None), node0, count, ptr(work), wb, stream())
+    return wb if wb and _grid_nsd(psrc, pdet, det0, ndet, 1) < 0 else 0
+
+
+def _jac_params(mesh, whats, phi, phi_kind, colsd, nc, det0, ndet, ps, pd, gnsd, wb, J, ldj, out_kind, stride, node0,
+                count):
+    """The rows of every parameter, parameter p's columns from p * stride, by
+    the pipelined kernel with wb bytes of workspace (the full grid) or, wb = 0,
+    by the general one."""
+    if wb and whats:
+        npar = len(whats)
+        work = torch.empty(wb, dtype=torch.uint8, device=phi.device)
+        need_ddd = _lib.RB_JAC_D in whats
+        call("rb_jac_multi", ctypes.byref(mesh.struct), npar, (ctypes.c_int32 * npar)(*whats),
+             (ctypes.c_int64 * npar)(*(p * stride for p in range(npar))), ptr(phi), phi_kind, phi.shape[1], ptr(colsd),
+             nc, det0, ndet, ptr(ps), ptr(pd), -abs(gnsd), ptr(J), ldj, out_kind, mesh.rmax, mesh.emax, ptr(mesh.evol),
+             ptr(mesh.ddd if need_ddd else None), node0, count, ptr(work), wb, stream())
+        return
+    m, f, c, s, d, v, st = (ctypes.byref(mesh.struct), ptr(phi), ptr(colsd), ptr(ps), ptr(pd), ptr(mesh.evol), stream())
+    for p, w in enumerate(whats):
+        call("rb_jac_range", m, w, f, phi_kind, phi.shape[1], c, nc, det0, ndet, s, d, gnsd, ptr(J[:, p * stride:]), ldj,
+             out_kind, mesh.rmax, mesh.emax, v, ptr(mesh.ddd if w == _lib.RB_JAC_D else None), node0, count, st)
 
 
 def jacobian_matrix(mesh, phi, sd, params=("mua",), mode="reference", dtype=torch.float32, acc64=False):
     """The real Jacobian of the GN step (FP32, or BF16 with ``dtype``), rows x
     columns = (nsd or 2 nsd) x (len(params) * nn), stored with a row stride
-    padded to 16 bytes.
+    padded to 16 bytes (32, a whole sector, where the pipelined kernel writes them).
     Complex fields give matreform 'real' stacking [Re; Im] (recon.py:532-546).
     mode 'reference' = redbirdpy's jac for mua (forward.py:509-569);
     'exact' = derivatives of the node-based assembly ('mua' at fixed D, 'D').
@@ -1219,7 +1233,8 @@ def jacobian_matrix(mesh, phi, sd, params=("mua",), mode="reference", dtype=torc
     rows = 2 * nsd if cplx else nsd
     nn = mesh.nn
     bf = dtype == torch.bfloat16
-    ldj = _pad8(len(params) * nn)  # (FP32: whole 32-byte sectors per row)
+    wb = _jac_grid_bytes(mesh, phi, det0, ndet, psrc, pdet, acc64 and not bf, nn)
+    ldj = _pad8(len(params) * nn) if bf or wb else _pad4(len(params) * nn)
     # every column below len(params) * nn is written by rb_jac; only the
     # row padding (read by the gram's aligned tiles) is cleared here
     J = torch.empty((rows, ldj), dtype=dtype, device=phi.device)
@@ -1233,9 +1248,9 @@ def jacobian_matrix(mesh, phi, sd, params=("mua",), mode="reference", dtype=torc
         out_kind = _lib.RB_JAC_SPLIT_F32 if cplx else _lib.RB_F32
     phi_kind = {torch.float64: _lib.RB_F64, torch.complex128: _lib.RB_C128, torch.float32: _lib.RB_F32,
                 torch.complex64: _lib.RB_C64}[phi.dtype]
-    colsd, ps, pd = _i32(cols, phi.device), _i32(psrc, phi.device), _i32(pdet, phi.device)
+    colsd, ps, pd = _i32(np.concatenate([cols, psrc, pdet]), phi.device).split([len(cols), nsd, nsd])  # one upload
     _jac_params(mesh, [_jac_what(name, mode) for name in params], phi, phi_kind, colsd, len(cols), det0, ndet, ps, pd,
-                _grid_nsd(psrc, pdet, det0, ndet, 1), J, ldj, out_kind, nn, 0, nn)
+                nsd if wb else _grid_nsd(psrc, pdet, det0, ndet), wb, J, ldj, out_kind, nn, 0, nn)
     _jac_checked()
     return J, len(params) * nn
 
@@ -1380,8 +1395,7 @@ class SlabJacobian:
     def __init__(self, mesh, phi, sd, params=("mua",), mode="reference", width=4096, dtype=torch.float32,
                  acc64=False):
         self.mesh, self.phi, self.params, self.dtype = mesh, phi, tuple(params), dtype
-        self.cols, self.det0, self.ndet, psrc, pdet, self.colsd, self.ps, self.pd, _ = _pair_dev(sd, phi.device)
-        self.gnsd = _grid_nsd(psrc, pdet, self.det0, self.ndet, 1)
+        self.cols, self.det0, self.ndet, psrc, pdet, self.colsd, self.ps, self.pd, self.gnsd = _pair_dev(sd, phi.device)
         if len(self.cols) > 128 or self.ndet > 64:
             raise ValueError("rb_jac stages at most 128 phi columns and 64 detectors per call")
         nsd = len(psrc)
@@ -1391,7 +1405,8 @@ class SlabJacobian:
         self.K = len(self.params) * self.nn
         self.width = int(max(1, min(width, self.nn)))
         self.bf = dtype == torch.bfloat16
-        pad = self._pad = _pad8
+        self.wb = _jac_grid_bytes(mesh, phi, self.det0, self.ndet, psrc, pdet, acc64 and not self.bf, self.width)
+        pad = self._pad = _pad8 if self.bf or self.wb else _pad4
         self.buf = torch.empty(self.rows * pad(len(self.params) * self.width), dtype=dtype, device=phi.device)
         if self.bf:
             self.out_kind = _lib.RB_JAC_SPLIT_BF16 if self.cplx else _lib.RB_JAC_BF16
@@ -1418,7 +1433,7 @@ class SlabJacobian:
         if ld > ks:
             Js[:, ks:].zero_()
         _jac_params(self.mesh, self.whats, self.phi, self.phi_kind, self.colsd, len(self.cols), self.det0, self.ndet,
-                    self.ps, self.pd, self.gnsd, Js, ld, self.out_kind, c, a, c)
+                    self.ps, self.pd, self.gnsd, self.wb if c >= JAC_GRID_NODES else 0, Js, ld, self.out_kind, c, a, c)
         _jac_checked()
         return Js, ks
 

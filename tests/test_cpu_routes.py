@@ -1,0 +1,53 @@
+"""Host-side choice of routes, with the library's calls recorded."""
+
+import types
+
+import numpy as np
+import pytest
+import torch
+
+from redbirdpy_b200 import engine
+
+
+def _jac_calls(monkeypatch, nn, ns, nd, cplx, params, acc64=True, grid=True):
+    """(names of the library calls, their pair counts, J) of one jacobian_matrix call."""
+    log = []
+    monkeypatch.setattr(engine, "call", lambda name, *a: log.append((name, a)))
+    monkeypatch.setattr(engine, "stream", lambda: None)
+    monkeypatch.setattr(engine, "_jac_checked", lambda: None)
+    mesh = types.SimpleNamespace(nn=nn, struct=engine._lib.RbMesh(), rmax=15, emax=24, evol=None, ddd=None)
+    s, d = np.meshgrid(np.arange(ns), ns + np.arange(nd))
+    sd = np.column_stack([s.ravel(), d.ravel(), np.ones(ns * nd)])
+    if not grid:
+        sd = sd[:-1]
+    phi = torch.zeros((nn, ns + nd), dtype=torch.complex128 if cplx else torch.float64)
+    J, K = engine.jacobian_matrix(mesh, phi, sd, params, "exact", acc64=acc64)
+    assert K == len(params) * nn
+    counts = [a[11] if name == "rb_jac_range" else a[13] for name, a in log]
+    return [name for name, _ in log], counts, J
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+def test_jacobian_rows_below_the_line_take_the_general_kernel_alone(cplx, monkeypatch):
+    """Small meshes, other pair tables and other row types: rb_jac's own
+    preparation and row stride, nothing of the pipelined kernel's."""
+    asked = []
+    real = engine._grid_nsd
+    monkeypatch.setattr(engine, "_grid_nsd", lambda *a: asked.append(a[4:]) or real(*a))
+    w = 2 if cplx else 1
+    names, counts, J = _jac_calls(monkeypatch, 2002, 5, 7, cplx, ("mua", "D"))
+    assert names == ["rb_jac_range"] * 2 and counts == [35, 35] and asked == [()]
+    assert J.stride(0) == 4004 and J.shape[0] == 35 * w
+    names, counts, J = _jac_calls(monkeypatch, 2002, 4, 8, cplx, ("mua",))
+    assert names == ["rb_jac_range"] and counts == [-32] and J.stride(0) == 2004
+    names, counts, J = _jac_calls(monkeypatch, 9001, 16, 16, cplx, ("mua",), acc64=False)
+    assert names == ["rb_jac_range"] and counts == [-256] and J.stride(0) == 9004
+    names, counts, J = _jac_calls(monkeypatch, 9001, 16, 16, cplx, ("mua",), grid=False)
+    assert names == ["rb_jac_range"] and counts == [255] and J.stride(0) == 9004
+    assert _jac_calls(monkeypatch, 9001, 16, 16, cplx, ())[0] == []
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+def test_jacobian_rows_of_the_full_grid_take_the_pipelined_kernel(cplx, monkeypatch):
+    names, counts, J = _jac_calls(monkeypatch, 9001, 15, 16, cplx, ("mua", "D"))
+    assert names == ["rb_jac_multi"] and counts == [-240] and J.stride(0) == 18008
