@@ -47,9 +47,14 @@ __device__ __forceinline__ void chain_wait() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
-// the live-column count of an iteration's kernels (written by an earlier one)
+// the live-column count of an iteration's kernels (written by an earlier one):
+// an ordinary load, kept behind the wait.  (As a C++ volatile it went past L1
+// for every warp: Jacobi solves of 16,900 nodes x 96 columns 7.96 -> 8.35 ms.)
 __device__ __forceinline__ bool chain_dead(const int32_t* live) {
-  return live && *reinterpret_cast<const volatile int32_t*>(live) == 0;
+  if (!live) return false;
+  int32_t v;
+  asm volatile("ld.global.b32 %0, [%1];" : "=r"(v) : "l"(live));
+  return v == 0;
 }
 template <typename... P, typename... A>
 inline cudaError_t launch_early(bool early, void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t st, A... a) {

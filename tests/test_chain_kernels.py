@@ -47,3 +47,10 @@ def test_chain_waits_come_first():
     for name, _, body in _kernels():
         before = re.sub(r"constexpr [^;]*;", "", body.split("chain_wait()")[0])
         assert not re.search(r"\[|\*\w|->", re.sub(r"__shared__[^;]*;", "", before)), (name, before)
+
+
+def test_live_counts_are_read_through_l1():
+    """Every warp of every iteration kernel reads the live count: a C++
+    volatile read passes L1 by; an ordinary load in ordered assembly does not."""
+    body = (CSRC / "rb_common.cuh").read_text().split("bool chain_dead(")[1].split("\n}")[0]
+    assert "volatile int32_t" not in body and "asm volatile(\"ld.global.b32" in body
