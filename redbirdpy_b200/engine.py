@@ -948,15 +948,21 @@ def solve(mat, B, precision="mixed", tol=DEFAULT_TOL, inner_tol=None, maxiter=20
         coarse = False
         if instances is None:
             instances = Instances([0, n], B.device)
+    redo = False
     if (coarse == "auto" and groups == "auto" and prec == _lib.RB_MIXED and instances is None and not profile
             and not spmm_lanes and _one_launch(n, k, mat.is_complex)):
-        coarse = None  # (no coarse space: the library then solves it in one launch)
+        # no coarse space: the library then solves it in one launch; what that
+        # does not bring to convergence is redone with the two-level form
+        # where the mesh is large enough for one
+        redo, coarse = n >= COARSE_MIN_NODES, None
     mid = _resolve_mid(mat, n, k, prec, coarse, groups, instances, budget) if k else None
     cs = _resolve_coarse(mat, coarse) if mid is None else None
-    if inner_tol is None:
-        inner_tol = 1e-5 if cs is not None or mid is not None else 1e-4
-    if prec == _lib.RB_FP64 and inner_tol > 1e-6:
-        inner_tol = max(tol, 1e-15)
+
+    def inner_of(space):
+        """The inner tolerance with a coarse space or level (None: without)."""
+        t = inner_tol if inner_tol is not None else 1e-5 if space is not None else 1e-4
+        return max(tol, 1e-15) if prec == _lib.RB_FP64 and t > 1e-6 else t
+
     def takes_one_launch(kb):
         """Whether the library solves kb columns in one launch, which reads no row groups."""
         return bool(prec == _lib.RB_MIXED and mid is None and cs is None and instances is None and budget is None
@@ -966,8 +972,8 @@ def solve(mat, B, precision="mixed", tol=DEFAULT_TOL, inner_tol=None, maxiter=20
     rg = None
     if instances is not None and instances.n != n:
         raise ValueError("instances do not cover the matrix's rows")
-    opts = _lib.RbSolveOpts(prec, int(max_outer), int(maxiter), int(check_every), float(tol), float(inner_tol),
-                            int(bool(profile)), int(x0 is not None),
+    opts = _lib.RbSolveOpts(prec, int(max_outer), int(maxiter), int(check_every), float(tol),
+                            float(inner_of(mid if mid is not None else cs)), int(bool(profile)), int(x0 is not None),
                             ctypes.pointer(cs.struct) if cs is not None else None, None, None, int(spmm_lanes))
     inst_status, inst_relres = [], []
     for c0 in range(0, k, 128):
@@ -999,6 +1005,7 @@ def solve(mat, B, precision="mixed", tol=DEFAULT_TOL, inner_tol=None, maxiter=20
                 work = None
                 cs = _resolve_coarse(mat, coarse)
                 opts.coarse = ctypes.pointer(cs.struct) if cs is not None else None
+                opts.inner_tol = float(inner_of(cs))
                 mid = None
                 if x0 is not None:
                     Xb.copy_(x0[:, c0:c0 + kb])
@@ -1010,18 +1017,28 @@ def solve(mat, B, precision="mixed", tol=DEFAULT_TOL, inner_tol=None, maxiter=20
                 inst_status.append(instances.status.cpu().numpy())
                 inst_relres.append(rel)
             continue
-        if prec == _lib.RB_MIXED:
-            one = takes_one_launch(kb)
-            rg = rg if one or rg is not None else _resolve_groups(mat, groups)
-            opts.groups = ctypes.pointer(rg.struct) if rg is not None and not one else None
-        wb = _lib.lib().rb_femsolve_work_bytes(n, mat.struct.nnz, kb, int(mat.is_complex), prec)
-        if cs is not None:
-            wb += _lib.lib().rb_coarse_work_bytes(cs.nc, kb, int(mat.is_complex), prec)
-        if instances is not None:
-            wb += _lib.lib().rb_instances_work_bytes(instances.ninst, kb)
-        work = torch.empty(wb, dtype=torch.uint8, device=B.device)
-        call("rb_femsolve", ctypes.byref(mat.struct), ptr(Bb), ptr(Xb), kb, ctypes.byref(opts), ctypes.byref(inf),
-             ptr(work), wb, stream())
+        while True:
+            if prec == _lib.RB_MIXED:
+                one = takes_one_launch(kb)
+                rg = rg if one or rg is not None else _resolve_groups(mat, groups)
+                opts.groups = ctypes.pointer(rg.struct) if rg is not None and not one else None
+            wb = _lib.lib().rb_femsolve_work_bytes(n, mat.struct.nnz, kb, int(mat.is_complex), prec)
+            if cs is not None:
+                wb += _lib.lib().rb_coarse_work_bytes(cs.nc, kb, int(mat.is_complex), prec)
+            if instances is not None:
+                wb += _lib.lib().rb_instances_work_bytes(instances.ninst, kb)
+            work = torch.empty(wb, dtype=torch.uint8, device=B.device)
+            call("rb_femsolve", ctypes.byref(mat.struct), ptr(Bb), ptr(Xb), kb, ctypes.byref(opts), ctypes.byref(inf),
+                 ptr(work), wb, stream())
+            if inf.flag == 0 or not redo:
+                break
+            redo, cs = False, _resolve_coarse(mat, "auto")
+            if cs is None:
+                break
+            opts.coarse = ctypes.pointer(cs.struct)
+            opts.inner_tol = float(inner_of(cs))
+            if x0 is not None:
+                Xb.copy_(x0[:, c0:c0 + kb])
         if Xb is not X:
             X[:, c0:c0 + kb] = Xb
         _add_info(info, inf)

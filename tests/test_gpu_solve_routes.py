@@ -101,3 +101,19 @@ def test_wide_solves_leave_the_one_launch_form(cells, k, cplx, one):
         Z, info3 = engine.solve(mat, B, coarse=False, groups=mat.mesh.row_groups())
         assert info3["flag"] == 0 and info3["launches"] > 2
         assert float((X - Z).abs().max()) <= 1e-10 * float(X.abs().max())
+
+
+@pytest.mark.parametrize("omega", [0.0, 2 * np.pi * 1e8])
+@pytest.mark.parametrize("start", [False, True])
+def test_what_one_launch_does_not_solve_gets_the_coarse_space(omega, start):
+    """21,112 nodes, 3 columns: one launch by default; capped at 10 iterations
+    a sweep it stagnates, and the two-level form, which takes 80, answers."""
+    mat = _matrix((28, 27, 25), omega)
+    B = _rhs(mat.n, 3)
+    want, info = engine.solve(mat, B)
+    assert info["flag"] == 0 and info["launches"] == 2 and info["coarse_nc"] == 0
+    x0 = 0.5 * want if start else None
+    X, info = engine.solve(mat, B, maxiter=10, x0=x0)
+    assert info["flag"] == 0 and info["coarse_nc"] > 0 and info["relres"] <= 1e-14
+    assert float((X - want).abs().max()) <= 1e-10 * float(want.abs().max())
+    assert engine.solve(mat, B, maxiter=10, coarse=False)[1]["flag"] == 1
