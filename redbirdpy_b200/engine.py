@@ -997,8 +997,13 @@ def solve(mat, B, precision="mixed", tol=DEFAULT_TOL, inner_tol=None, maxiter=20
             except torch.cuda.OutOfMemoryError:
                 work = None  # the two-level form needs a fifth less
             if work is not None:
-                call("rb_femsolve_mid", ctypes.byref(mat.struct), ctypes.byref(mid.struct), ptr(Bb), ptr(Xb), kb,
-                     ctypes.byref(opts), ctypes.byref(inf), ptr(work), wb, stream())
+                try:
+                    call("rb_femsolve_mid", ctypes.byref(mat.struct), ctypes.byref(mid.struct), ptr(Bb), ptr(Xb), kb,
+                         ctypes.byref(opts), ctypes.byref(inf), ptr(work), wb, stream())
+                except _lib.RedbirdError as e:
+                    if e.code != _lib.RB_EBREAKDOWN:  # (a zero or non-finite pivot of the dense level)
+                        raise
+                    work = None
             if work is None or inf.flag != 0:
                 # the cycle assumes a definite operator (positive diagonal,
                 # real part); what it does not solve gets the two-level form

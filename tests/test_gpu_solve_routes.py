@@ -117,3 +117,18 @@ def test_what_one_launch_does_not_solve_gets_the_coarse_space(omega, start):
     assert info["flag"] == 0 and info["coarse_nc"] > 0 and info["relres"] <= 1e-14
     assert float((X - want).abs().max()) <= 1e-10 * float(want.abs().max())
     assert engine.solve(mat, B, maxiter=10, coarse=False)[1]["flag"] == 1
+
+
+def test_a_broken_dense_level_leaves_the_answer_to_jacobi():
+    """A non-finite entry on a mesh below the coarse space's size: the cycle
+    cannot set up its dense level, and the Jacobi solve reports the breakdown
+    (flag 2) instead of an exception."""
+    mat = _matrix((25, 25, 24))
+    assert mat.n < engine.COARSE_MIN_NODES
+    B = _rhs(mat.n, 64)
+    assert engine.solve(mat, B)[1]["coarse_nc"] > 0  # the cycle's size
+    at = int(mat.mesh.indptr[1000])
+    mat.val64[at] = float("nan")
+    mat.val32[at] = float("nan")
+    _, info = engine.solve(mat, B)
+    assert info["flag"] == 2 and info["coarse_nc"] == 0
