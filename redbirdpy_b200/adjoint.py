@@ -222,8 +222,8 @@ class BatchModel(DeviceModel):
         self.status = None
 
     def _layout(self, cfgs):
-        """(positions, bbox, edge) with the instances side by side along x,
-        each scaled by its typical edge length (so that a group is 2 x 2 x 2
+        """(positions, bbox, edge, gap) with the instances side by side along
+        x, each scaled by its typical edge length (so that a group is 2 x 2 x 2
         nodes in every one), a gap of the largest extent between them."""
         edges = []
         for c in cfgs:
@@ -250,7 +250,7 @@ class BatchModel(DeviceModel):
         inst = self.instances.row_inst.long()
         pos = self.mesh.node * scale[inst, None] + torch.as_tensor(shift, device=self.mesh.device)[inst]
         hi = np.array([x0[-2] + ext[-1, 0], ext[:, 1].max(), ext[:, 2].max()])
-        return pos.contiguous(), (np.zeros(3), hi), 1.0
+        return pos.contiguous(), (np.zeros(3), hi), 1.0, gap
 
     def tune(self, mua, dcoef):
         """Pick the solve's launch shapes for this batch with the autotuner

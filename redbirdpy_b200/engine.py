@@ -51,7 +51,7 @@ class DeviceMesh:
         self._coarse = {}
         self._groups = None
         self._mid = False  # not built yet
-        self.layout = None  # (positions, bbox, edge) for the groups, where not the nodes' own
+        self.layout = None  # (positions, bbox, edge, gap) for the groups, where not the nodes' own
         self._edge = None
         if self.ne:
             sel = np.arange(0, self.ne, max(1, self.ne // 65536))
@@ -166,7 +166,8 @@ class DeviceMesh:
 
     def mid_level(self):
         """The MidLevel of the V-cycle preconditioner (built once), or None
-        when the mesh has no row groups or a group has too many neighbours."""
+        when the mesh has no row groups, a group has too many neighbours or
+        the dense level cannot keep a batch's instances apart."""
         if self._mid is False:
             rg = self.row_groups()
             try:
@@ -727,9 +728,17 @@ class MidLevel:
         self.nnz1 = int(nnz1.value)
         self.mcol = torch.empty(max(self.nnz1, 1), dtype=torch.int32, device=dev)
         call("rb_midlevel_fill", ctypes.byref(rg.struct), ptr(self.grp), ptr(self.mptr), ptr(self.mcol), stream())
-        # (a layout of instances side by side leaves about half the cells empty)
-        target = mid_coarse_target(rg.ng) * (1 if mesh.layout is None else 2)
+        target = mid_coarse_target(rg.ng)
+        if mesh.layout is not None:
+            # instances side by side leave about half the cells empty; a cell
+            # must not reach from one to the next (gap), which takes more of
+            # them in a long row of instances
+            (lo, hi), gap = mesh.layout[1], mesh.layout[3]
+            ext = np.maximum(hi - lo, 1e-6 * float(np.max(hi - lo)))
+            target = max(2 * target, int(np.ceil(np.prod(ext) / gap ** 3)))
         self.coarse = CoarseSpace(_GroupNodes(mesh, rg), target)
+        if mesh.layout is not None and self.coarse.h > gap:
+            raise _lib.RedbirdError("MidLevel", _lib.RB_ESIZE, "cells of the dense level wider than the instances' gap")
         self.struct = _lib.RbMidlevel(ctypes.pointer(rg.struct), self.grp.data_ptr(), self.mptr.data_ptr(),
                                       self.mcol.data_ptr(), self.nnz1, ctypes.pointer(self.coarse.struct))
 

@@ -132,3 +132,38 @@ def test_a_broken_dense_level_leaves_the_answer_to_jacobi():
     mat.val32[at] = float("nan")
     _, info = engine.solve(mat, B)
     assert info["flag"] == 2 and info["coarse_nc"] == 0
+
+
+@pytest.mark.parametrize("cells_max", [4096, 3])
+def test_dense_level_of_a_batch_keeps_instances_apart(cells_max, monkeypatch):
+    """However few aggregates are asked for, none holds rows of two instances;
+    where the dense level cannot have that many, the batch solves by Jacobi."""
+    from redbirdpy_b200.adjoint import BatchModel
+
+    monkeypatch.setattr(engine, "mid_coarse_target", lambda ng: 1)
+    cfgs = []
+    for i in range(20):
+        size = np.array([20, 18, 15]) * (1.0 + 0.1 * i)
+        node, elem = kuhn_box(size, 1.0 + 0.1 * i)
+        prop = np.tile([0.01, 1.0, 0.0, 1.37], (node.shape[0], 1))
+        cfgs.append(rbb.meshprep(dict(node=node, elem=elem, prop=prop, srcpos=size[None] * [[0.4, 0.4, 0.0]],
+                                      srcdir=np.array([[0, 0, 1.0]]), detpos=size[None] * [[0.6, 0.4, 0.0]],
+                                      detdir=np.array([[0, 0, 1.0]]), omega=0.0))[0])
+    bm = BatchModel(cfgs)
+    monkeypatch.setattr(engine, "COARSE_MAX", cells_max)
+    p = np.vstack([c["prop"] for c in cfgs])
+    mua = torch.as_tensor(p[:, 0].copy(), device="cuda")
+    mat = engine.assemble(bm.mesh, bm.optics(mua, 1.0 / (3.0 * (mua + 1.0))))
+    mid = bm.mesh.mid_level()
+    assert (mid is not None) == (cells_max > 3)
+    if mid is not None:
+        rows = mid.groups.rows[: 8 * mid.groups.ng].view(-1, 8).long()
+        inst = bm.instances.row_inst.long()
+        of_group = inst[rows[:, 0]]
+        assert bool(((rows < 0) | (inst[rows.clamp_min(0)] == of_group[:, None])).all())
+        agg = mid.coarse.agg[: mid.groups.ng].long()
+        lo = torch.full((mid.coarse.nc,), 99, device="cuda").scatter_reduce(0, agg, of_group, "amin")
+        hi = torch.full((mid.coarse.nc,), -1, device="cuda").scatter_reduce(0, agg, of_group, "amax")
+        assert torch.equal(lo, hi)
+    X, info = engine.solve(mat, bm.B, **bm.solve_kw)
+    assert info["flag"] == 0 and not info["inst_status"].any() and (info["coarse_nc"] > 0) == (mid is not None)
