@@ -575,6 +575,9 @@ int rb_cholesky(double* H, int64_t M, int64_t ldh, void* work, size_t work_bytes
  * of M doubles is taken too; the segments are then allocated on the stream) */
 size_t rb_chol_solve_work_bytes(int64_t M);
 int rb_chol_solve(const double* L, int64_t M, int64_t ldh, double* x, void* work, size_t work_bytes, void* stream);
+/* RB_ECUDA when a rb_chol_solve so far gave up a (bounded) wait between its
+ * blocks, whose solution then holds NaN; synchronizes `stream` and clears it */
+int rb_chol_solve_status(void* stream);
 size_t rb_gemv_t_work_bytes(int64_t K);
 int rb_gemv_t(const float* J, int64_t M, int64_t K, int64_t ldj, const double* y, double alpha,
               double beta, double* out, void* work, size_t work_bytes, void* stream);

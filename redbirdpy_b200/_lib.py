@@ -153,6 +153,7 @@ _SIGS = {
     "rb_cholesky_work_bytes": (_sz, []),
     "rb_cholesky": (ctypes.c_int, [_vp, _i64, _i64, _vp, _sz, _vp]),
     "rb_chol_solve_work_bytes": (_sz, [_i64]),
+    "rb_chol_solve_status": (ctypes.c_int, [_vp]),
     "rb_chol_solve": (ctypes.c_int, [_vp, _i64, _i64, _vp, _vp, _sz, _vp]),
     "rb_gemv_t_work_bytes": (_sz, [_i64]),
     "rb_gemv_t": (ctypes.c_int, [_vp, _i64, _i64, _i64, _vp, _dbl, _dbl, _vp, _vp, _sz, _vp]),

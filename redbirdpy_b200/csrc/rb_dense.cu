@@ -398,9 +398,11 @@ __global__ void __launch_bounds__(kSyrkThreads) syrk_update_kernel(double* __res
 // reduction and the product with the block's inverse.  One launch per block
 // row and direction before: 1024 launches of 8-11 us for the four solves of a
 // refined M = 8192 step, 2.36 ms per solve, now 0.43 ms (M = 8192).  Waits are bounded;
-// one that gives up ends its block with NaN in its segment.
+// one that gives up ends its block with NaN in its segment and sets the word
+// that rb_chol_solve_status reads.
 constexpr unsigned long long kEmpty = ~0ull;
 constexpr int kTrsvSpins = 1 << 20;  // about a second
+__device__ int g_trsv_err;
 
 __device__ __forceinline__ double2 ld_seg(const double* p) {
   double2 v;
@@ -563,6 +565,7 @@ __global__ void __launch_bounds__(256, 1) chol_solve_kernel(const double* __rest
       __syncthreads();
     }
   }
+  if (tid == 0 && bad) atomicExch(&g_trsv_err, 1);
 }
 
 constexpr int kGemvSlabs = 16;
@@ -1035,6 +1038,18 @@ int rb_chol_solve(const double* L, int64_t M, int64_t ldh, double* x, void* work
     if (e == cudaSuccess) e = f;
   }
   RB_CUDA_TRY(e);
+  return RB_OK;
+}
+
+int rb_chol_solve_status(void* stream) {
+  RB_CUDA_TRY(cudaStreamSynchronize(as_stream(stream)));
+  int h = 0;
+  RB_CUDA_TRY(cudaMemcpyFromSymbol(&h, g_trsv_err, sizeof(int)));
+  if (h) {
+    const int zero = 0;
+    RB_CUDA_TRY(cudaMemcpyToSymbol(g_trsv_err, &zero, sizeof(int)));
+    return fail(RB_ECUDA, "rb_chol_solve: a wait for another block row gave up; the solution is not valid");
+  }
   return RB_OK;
 }
 

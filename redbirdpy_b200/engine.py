@@ -1573,6 +1573,7 @@ def normal_solve(J, K, H, di, r, lam, alpha=1.0, lo=None, refine=3, refine_tol=1
         return out
 
     y = precond(rr)
+    unchecked = True  # a solve whose result no finite residual norm vouches for
     sweeps, rel = 0, None
     u_now = None  # J^T y for the current y, when a residual pass left it
     if refine:
@@ -1584,11 +1585,15 @@ def normal_solve(J, K, H, di, r, lam, alpha=1.0, lo=None, refine=3, refine_tol=1
             call("rb_axpby", M, -float(alpha), ptr(Ju), 1.0, ptr(res), stream())  # res = r - alpha J J^T y
             call("rb_axpby", M, -float(lam), ptr(y), 1.0, ptr(res), stream())  # res -= lam y
             rel = norm2(res) / rnorm
+            unchecked = not np.isfinite(rel)
             if rel <= refine_tol:
                 u_now = u
                 break
             call("rb_axpby", M, 1.0, ptr(precond(res)), 1.0, ptr(y), stream())
+            unchecked = True
             sweeps = it + 1
+    if unchecked and not torch.cuda.is_current_stream_capturing():
+        call("rb_chol_solve_status", stream())
     if info is not None:
         info.update(refine_sweeps=sweeps, refine_relres=rel, lam=float(lam))
     if return_y:

@@ -51,3 +51,43 @@ def test_jacobian_rows_below_the_line_take_the_general_kernel_alone(cplx, monkey
 def test_jacobian_rows_of_the_full_grid_take_the_pipelined_kernel(cplx, monkeypatch):
     names, counts, J = _jac_calls(monkeypatch, 9001, 15, 16, cplx, ("mua", "D"))
     assert names == ["rb_jac_multi"] and counts == [-240] and J.stride(0) == 18008
+
+
+@pytest.mark.parametrize("refine,norms,checked", [(0, [], True), (3, [1.0, 1e-3, 1e-15], False),
+                                                  (3, [1.0, 1e-3, 1e-6, 1e-9], True), (2, [1.0, float("nan"), 1.0], True)])
+def test_normal_solve_asks_after_waits_that_gave_up(refine, norms, checked, monkeypatch):
+    """A triangular solve whose result no finite residual vouches for is asked
+    whether a wait gave up; its error reaches the caller."""
+    log, fail = [], []
+
+    def call(name, *a):
+        log.append(name)
+        if name == "rb_chol_solve_status" and fail:
+            raise engine._lib.RedbirdError(name, engine._lib.RB_ECUDA, "a wait gave up")
+
+    class Op(engine.StoredJacobian):
+        def __init__(self, J, K, lo):
+            self.rows = J.shape[0]
+
+        def jt_then_j(self, y):
+            return torch.zeros(9), torch.zeros(self.rows)
+
+        def jt(self, y, alpha):
+            return torch.zeros(9)
+
+    monkeypatch.setattr(engine, "call", call)
+    monkeypatch.setattr(engine, "stream", lambda: None)
+    monkeypatch.setattr(engine, "StoredJacobian", Op)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    H, di, r = torch.zeros((4, 4), dtype=torch.float64), torch.ones(4, dtype=torch.float64), np.ones(4)
+    for broken in (False, True):
+        log.clear()
+        fail[:] = [1] * broken
+        left = list(norms)
+        monkeypatch.setattr(engine, "norm2", lambda t: left.pop(0))
+        if broken and checked:
+            with pytest.raises(engine._lib.RedbirdError):
+                engine.normal_solve(torch.zeros((4, 9)), 9, H, di, r, 0.1, refine=refine)
+        else:
+            engine.normal_solve(torch.zeros((4, 9)), 9, H, di, r, 0.1, refine=refine)
+        assert log.count("rb_chol_solve_status") == checked

@@ -167,3 +167,14 @@ def test_dense_level_of_a_batch_keeps_instances_apart(cells_max, monkeypatch):
         assert torch.equal(lo, hi)
     X, info = engine.solve(mat, bm.B, **bm.solve_kw)
     assert info["flag"] == 0 and not info["inst_status"].any() and (info["coarse_nc"] > 0) == (mid is not None)
+
+
+def test_triangular_solves_that_finish_report_nothing():
+    M = 700
+    L = torch.eye(M, device="cuda", dtype=torch.float64)
+    x = torch.ones(M, device="cuda", dtype=torch.float64)
+    wb = _lib.lib().rb_chol_solve_work_bytes(M)
+    work = torch.empty(wb, dtype=torch.uint8, device="cuda")
+    engine.call("rb_chol_solve", engine.ptr(L), M, M, engine.ptr(x), engine.ptr(work), wb, engine.stream())
+    engine.call("rb_chol_solve_status", engine.stream())
+    assert bool((x == 1).all())
