@@ -477,6 +477,9 @@ int rb_jac_remap(const void* J, int32_t kind, int64_t rows, int64_t ldj, const i
  * bytes, 16-byte aligned, or NULL (the bytes are 0 when the kernel does not
  * apply or its tiles would be mostly empty). */
 size_t rb_jac_multi_work_bytes(int32_t rmax, int32_t nsu, int32_t ndet, int32_t is_complex);
+/* 1 where the pipelined kernel was measured to be the faster one (from about
+ * 8000 nodes); elsewhere rb_jac_multi goes faster without a workspace */
+int rb_jac_multi_wins(int32_t rmax, int32_t emax, int32_t nsu, int32_t ndet, int32_t is_complex);
 int rb_jac_multi(const rb_mesh* mesh, int32_t nparam, const int32_t* what, const int64_t* col0, const void* phi,
                  int32_t phi_kind, int64_t ld, const int32_t* cols, int32_t nc, int32_t det0, int32_t ndet,
                  const int32_t* pair_src, const int32_t* pair_det, int64_t nsd, void* J, int64_t ldj,

@@ -136,6 +136,7 @@ _SIGS = {
     "rb_jac_range": (ctypes.c_int, [ctypes.POINTER(RbMesh), _i32, _vp, _i32, _i64, _vp, _i32, _i32, _i32, _vp,
                                     _vp, _i64, _vp, _i64, _i32, _i32, _i32, _vp, _vp, _i64, _i64, _vp]),
     "rb_jac_multi_work_bytes": (_sz, [_i32, _i32, _i32, _i32]),
+    "rb_jac_multi_wins": (ctypes.c_int, [_i32, _i32, _i32, _i32, _i32]),
     "rb_jac_multi": (ctypes.c_int, [ctypes.POINTER(RbMesh), _i32, ctypes.POINTER(_i32), ctypes.POINTER(_i64), _vp, _i32,
                                     _i64, _vp, _i32, _i32, _i32, _vp, _vp, _i64, _vp, _i64, _i32, _i32, _i32, _vp, _vp,
                                     _i64, _i64, _vp, _sz, _vp]),

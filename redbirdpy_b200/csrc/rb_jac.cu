@@ -635,11 +635,25 @@ static int launch_jac_tc(const JacArgs& a, const void* phi, void* J, cudaStream_
   return RB_OK;
 }
 
-template <typename C, typename In, bool SPLIT, bool GRID, bool BF, bool NARROW = false>
-static int launch_jac_t(const JacArgs& a, const void* phi, void* J, cudaStream_t st) {
+// nodes of a block: as many as leave two blocks to an SM
+template <typename C>
+static int jac_tn(int rmax, int nc, int ndet, int emax) {
   int TN = 8;
   const size_t budget = 110 * 1024;
-  while (TN > 1 && jac_smem<C>(TN, a.rmax, a.nc, a.ndet, a.emax) > budget) TN >>= 1;
+  while (TN > 1 && jac_smem<C>(TN, rmax, nc, ndet, emax) > budget) TN >>= 1;
+  return TN;
+}
+// nodes of jac_kernel's FP64 products at work on an SM: its blocks share 228 KB,
+// and the full grid's (74 registers, complex 114) are 3 or 2 at most
+int jac_resident(bool cx, bool grid, int rmax, int nc, int ndet, int emax) {
+  const int TN = cx ? jac_tn<cdouble>(rmax, nc, ndet, emax) : jac_tn<double>(rmax, nc, ndet, emax);
+  const size_t sm = cx ? jac_smem<cdouble>(TN, rmax, nc, ndet, emax) : jac_smem<double>(TN, rmax, nc, ndet, emax);
+  return TN * (int)std::min<size_t>(228 * 1024 / (sm + 1024), grid ? (cx ? 2 : 3) : 8);
+}
+
+template <typename C, typename In, bool SPLIT, bool GRID, bool BF, bool NARROW = false>
+static int launch_jac_t(const JacArgs& a, const void* phi, void* J, cudaStream_t st) {
+  const int TN = jac_tn<C>(a.rmax, a.nc, a.ndet, a.emax);
   const size_t sm = jac_smem<C>(TN, a.rmax, a.nc, a.ndet, a.emax);
   if (sm > kJacSmemMax) return fail(RB_ESIZE, "rb_jac: staging needs %zu bytes of shared memory", sm);
   const unsigned g = (unsigned)ceil_div(a.nn - a.node0, TN);

@@ -44,6 +44,7 @@
 namespace rb {
 
 int* jac_err_word();  // rb_jac.cu: what rb_jac_status reads
+int jac_resident(bool cx, bool grid, int rmax, int nc, int ndet, int emax);  // rb_jac.cu
 
 enum { JG_MUA_REF = 0, JG_MUA_NODAL = 1, JG_D = 2 };
 constexpr int kJgThreads = 256;    // threads that compute
@@ -496,6 +497,33 @@ size_t rb_jac_multi_work_bytes(int32_t rmax, int32_t nsu, int32_t ndet, int32_t 
   if (fill < (is_complex ? 0.4 : 0.7)) return 0;
   const int RM = jg_rm(rmax);
   return (size_t)jg_chunk(rmax, RM) * rmax * RM * sizeof(double) + 256;
+}
+
+// Where the pipelined kernel is the faster one.  Rows of at most 16 neighbours:
+// wherever its tiles are filled, but real 3 x 4 pairs (8,400 nodes x 2 quantities,
+// jac_kernel / this, ms: 0.25 / 0.29; 4 x 4 0.30 / 0.27).
+// Longer rows: an item has four nodes and half of the threads' columns, a
+// store half a sector, so it depends on the other side, which is as fast as it
+// has nodes at work on an SM (R).  Meshes of Delaunay tets, rmax 24 to 32, ms:
+// R >= 12 (small rows and few columns) goes to jac_kernel: 12,000 nodes real 8 x 8
+// 0.51 / 0.50, 60,480 nodes 4 x 4 1.92 / 2.11, 12 x 12 2.00 / 2.11, complex 5 x 7 at
+// 9,196 0.44 / 0.49.  Complex below that comes here: 60,480 nodes 16 x 16 4.43 /
+// 2.45, 64 x 64 17.4 / 11.0, 61 x 64 19.3 / 11.0, rmax 32 18.3 / 13.8; real counts off
+// 4 as well: 61 x 64 11.5 / 8.3.  Real blocked pairs: a fit to 30 counts, us per
+// node; 60,480 nodes 16 x 16 2.74 / 2.09, 32 x 64 5.83 / 4.49, 64 x 48 6.84 / 6.03 here,
+// 40 x 40 4.27 / 6.12, 56 x 56 6.99 / 7.71, 64 x 64 6.91 / 7.66 there (at rmax 29 R falls
+// to 3: 20,160 nodes 3.20 / 2.85).
+int rb_jac_multi_wins(int32_t rmax, int32_t emax, int32_t nsu, int32_t ndet, int32_t is_complex) {
+  if (emax < 1 || emax > kJgMaxE || !rb_jac_multi_work_bytes(rmax, nsu, ndet, is_complex)) return 0;
+  const double pairs = (double)nsu * ndet;
+  if (rmax <= 16) return is_complex || pairs >= 16.0;
+  const bool blocked = nsu % 4 == 0 && ndet % 4 == 0;
+  const int R = jac_resident(is_complex != 0, blocked, rmax, nsu + ndet, ndet, emax);
+  if (R >= 12) return 0;
+  if (is_complex || !blocked || R < 4 || R >= 8) return 1;
+  const JgLayout L = jg_layout<double, 4, 32>(rmax, nsu, ndet, 2);
+  const double general = R >= 6 ? 0.053 + 1.2e-5 * pairs : 0.075 + 1.35e-5 * pairs;
+  return 0.025 + 0.0137 * L.nst * L.ndt < general;
 }
 
 int rb_jac_multi(const rb_mesh* mesh, int32_t nparam, const int32_t* what, const int64_t* col0, const void* phi,

@@ -1225,8 +1225,12 @@ def _jac_grid_bytes(mesh, phi, det0, ndet, psrc, pdet, acc64, count):
     nodes, 0 where the general kernel forms them."""
     if not acc64 or count < JAC_GRID_NODES or phi.dtype not in (torch.float64, torch.complex128):
         return 0
-    wb = _lib.lib().rb_jac_multi_work_bytes(mesh.rmax, det0, ndet, int(phi.is_complex()))
-    return wb if wb and _grid_nsd(psrc, pdet, det0, ndet, 1) < 0 else 0
+    cplx = int(phi.is_complex())
+    if not _lib.lib().rb_jac_multi_wins(mesh.rmax, mesh.emax, det0, ndet, cplx):
+        return 0
+    if _grid_nsd(psrc, pdet, det0, ndet, 1) >= 0:
+        return 0
+    return _lib.lib().rb_jac_multi_work_bytes(mesh.rmax, det0, ndet, cplx)
 
 
 def _jac_params(mesh, whats, phi, phi_kind, colsd, nc, det0, ndet, ps, pd, gnsd, wb, J, ldj, out_kind, stride, node0,

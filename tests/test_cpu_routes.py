@@ -91,3 +91,15 @@ def test_normal_solve_asks_after_waits_that_gave_up(refine, norms, checked, monk
         else:
             engine.normal_solve(torch.zeros((4, 9)), 9, H, di, r, 0.1, refine=refine)
         assert log.count("rb_chol_solve_status") == checked
+
+
+@pytest.mark.parametrize("rmax,emax,ns,nd,cplx,wins", [
+    (15, 24, 3, 4, False, 0), (15, 24, 4, 4, False, 1), (15, 24, 3, 4, True, 1), (15, 24, 64, 64, True, 1),
+    (25, 44, 4, 4, False, 0), (25, 44, 12, 12, False, 0), (25, 44, 12, 16, False, 1), (24, 42, 5, 7, True, 0),
+    (25, 44, 16, 16, True, 1), (25, 44, 64, 64, True, 1), (25, 44, 61, 64, False, 1), (25, 44, 40, 40, False, 0),
+    (25, 44, 64, 48, False, 1), (25, 44, 64, 64, False, 0), (29, 44, 64, 64, False, 1), (40, 44, 64, 64, True, 0),
+    (25, 70, 64, 64, True, 0)])
+def test_rows_of_long_neighbour_lists_take_the_faster_kernel(rmax, emax, ns, nd, cplx, wins):
+    """The line between the general and the pipelined Jacobian kernel on
+    meshes off the box (17 to 32 neighbours), on both sides of each of its terms."""
+    assert engine._lib.lib().rb_jac_multi_wins(rmax, emax, ns, nd, int(cplx)) == wins
