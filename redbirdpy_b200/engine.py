@@ -897,6 +897,27 @@ class SolveTuner:
 solve_tuner = SolveTuner()
 
 
+def _product_kernel(n, k, cplx, prec, form):
+    """The kernel of the Krylov product of k columns (the library's dispatch):
+    ``form`` 'cycle' (V-cycle), 'one' (one launch), 'groups' (row groups
+    given) or 'rows'."""
+    if form == "one":
+        return "small_solve_kernel"
+    pad = (k + 3) // 4 * 4
+    if form != "cycle" and (k <= 32 or (k % 2 == 0 and k <= 64)):
+        pad = k
+    wide, o32 = 64 < pad <= 128, n * pad < 2 ** 31
+    if prec == _lib.RB_FP64:
+        return "spmm_grp_kernel" if pad in (32, 64, 128) else "spmm_kernel"
+    if cplx:
+        return "spmm_pair_kernel" if pad == 128 and o32 else "spmm_kernel"
+    if wide and form == "cycle":
+        return "vc_spmm_kernel"
+    if wide and o32:
+        return "spmm_blk_kernel" if form == "groups" else "spmm_pair_kernel"
+    return "spmm_kernel"
+
+
 def _add_info(info, inf):
     """One library call's RbSolveInfo into solve's info dict."""
     info["iters"] += inf.iters
@@ -939,7 +960,9 @@ def solve(mat, B, precision="mixed", tol=DEFAULT_TOL, inner_tol=None, maxiter=20
     needs ``instances`` (one covering all rows is made when None) and no
     coarse space; ``inst_status`` / ``inst_relres`` are then device tensors
     and ``flag`` is None until read.  ``spmm_lanes``: lanes per row of the
-    per-row SpMM (0: chosen from the column count; see SolveTuner)."""
+    per-row SpMM (0: chosen from the column count; see SolveTuner).  info's
+    ``product`` names the kernel of the inner products (last column block),
+    ``spmm_kernel`` the same but 'vc_spmm_kernel' for every cycle solve."""
     prec = _lib.RB_FP64 if precision == "fp64" else _lib.RB_MIXED
     n, k = B.shape
     xdt = torch.complex128 if mat.is_complex else torch.float64
@@ -1068,12 +1091,12 @@ def solve(mat, B, precision="mixed", tol=DEFAULT_TOL, inner_tol=None, maxiter=20
         info["inst_status"] = np.max(np.stack(inst_status), axis=0)
         info["inst_relres"] = torch.cat(inst_relres, dim=1).cpu().numpy()
     info["coarse_nc"] = mid.coarse.nc if mid is not None else cs.nc if cs is not None else 0
-    # the FP32 product of the last column block: the row-group kernel when
-    # groups were given and the block width suits its lane layout
+    # the inner product of the last column block
     kb = k - 128 * ((k - 1) // 128) if k else 0
-    info["spmm_kernel"] = ("vc_spmm_kernel" if mid is not None and not (mat.is_complex and kb > 124)
-                           else "spmm_blk_kernel" if rg is not None and 65 <= kb <= 128 and kb % 4 == 0
-                           else "spmm_pair_kernel")
+    form = "cycle" if mid is not None else "one" if k and prec == _lib.RB_MIXED and one else "groups" if rg else "rows"
+    info["product"] = _product_kernel(n, kb, mat.is_complex, prec, form)
+    # (a cycle solve's products go by one name here, whichever kernel fits the width)
+    info["spmm_kernel"] = "vc_spmm_kernel" if mid is not None else info["product"]
     return X, info
 
 

@@ -103,3 +103,18 @@ def test_rows_of_long_neighbour_lists_take_the_faster_kernel(rmax, emax, ns, nd,
     """The line between the general and the pipelined Jacobian kernel on
     meshes off the box (17 to 32 neighbours), on both sides of each of its terms."""
     assert engine._lib.lib().rb_jac_multi_wins(rmax, emax, ns, nd, int(cplx)) == wins
+
+
+@pytest.mark.parametrize("k,cplx,form,name", [
+    (7, False, "cycle", "spmm_kernel"), (65, False, "cycle", "vc_spmm_kernel"), (125, True, "cycle", "spmm_pair_kernel"),
+    (64, True, "cycle", "spmm_kernel"), (3, True, "one", "small_solve_kernel"), (67, False, "groups", "spmm_blk_kernel"),
+    (64, False, "groups", "spmm_kernel"), (66, False, "rows", "spmm_pair_kernel"), (128, True, "rows", "spmm_pair_kernel"),
+    (100, True, "rows", "spmm_kernel")])
+def test_product_names_follow_the_dispatch(k, cplx, form, name):
+    assert engine._product_kernel(40000, k, cplx, engine._lib.RB_MIXED, form) == name
+
+
+def test_fp64_product_names():
+    assert engine._product_kernel(9, 64, False, engine._lib.RB_FP64, "rows") == "spmm_grp_kernel"
+    assert engine._product_kernel(9, 63, False, engine._lib.RB_FP64, "rows") == "spmm_grp_kernel"
+    assert engine._product_kernel(9, 48, False, engine._lib.RB_FP64, "rows") == "spmm_kernel"

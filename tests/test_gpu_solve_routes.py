@@ -178,3 +178,17 @@ def test_triangular_solves_that_finish_report_nothing():
     engine.call("rb_chol_solve", engine.ptr(L), M, M, engine.ptr(x), engine.ptr(work), wb, engine.stream())
     engine.call("rb_chol_solve_status", engine.stream())
     assert bool((x == 1).all())
+
+
+def test_one_launch_solves_build_no_row_groups(monkeypatch):
+    """A default solve in one launch names its kernel and leaves the mesh's
+    row groups unbuilt; a wide one builds and names them."""
+    mat = _matrix((24, 22, 20))
+    monkeypatch.setattr(engine.DeviceMesh, "mid_level", lambda self: None)
+    _, info = engine.solve(mat, _rhs(mat.n, 4))
+    assert info["product"] == info["spmm_kernel"] == "small_solve_kernel" and mat.mesh._groups is None
+    _, info = engine.solve(mat, _rhs(mat.n, 128), coarse=False)
+    assert info["product"] in ("spmm_blk_kernel", "small_solve_kernel")
+    big = _matrix((32, 31, 30))
+    _, info = engine.solve(big, _rhs(big.n, 128), coarse=False)
+    assert info["product"] == "spmm_blk_kernel" and big.mesh._groups is not None
