@@ -599,6 +599,12 @@ def coarse_target(nn, is_complex=False):
     return int(max(1, min(max(lo, min(hi, nn // per)), nn // 16)))
 
 
+def _finished(dev):
+    """Waits for what the current stream has under way: a plan kept on a mesh
+    may next be used by another thread on another stream."""
+    torch.cuda.current_stream(dev).synchronize()
+
+
 class CoarseSpace:
     """Aggregates of the two-level preconditioner (``rb_coarse``): the mesh
     nodes binned into cubes of edge h chosen for about ``target`` cubes over
@@ -640,6 +646,7 @@ class CoarseSpace:
         self.h = h
         self.nb = tuple(int(v) for v in nb)
         self.struct = _lib.RbCoarse(self.nc, self.agg.data_ptr(), self.agg_ptr.data_ptr(), self.agg_rows.data_ptr())
+        _finished(dev)
 
 
 class RowGroups:
@@ -688,6 +695,7 @@ class RowGroups:
         self.h = h
         self.struct = _lib.RbRowGroups(self.ng, self.rows.data_ptr(), self.uptr.data_ptr(), self.ucol.data_ptr(),
                                        self.umask.data_ptr(), self.nu, self.coef.data_ptr())
+        _finished(dev)
 
 
 def mid_coarse_target(ng):

@@ -192,3 +192,13 @@ def test_one_launch_solves_build_no_row_groups(monkeypatch):
     big = _matrix((32, 31, 30))
     _, info = engine.solve(big, _rhs(big.n, 128), coarse=False)
     assert info["product"] == "spmm_blk_kernel" and big.mesh._groups is not None
+
+
+def test_plans_kept_on_a_mesh_are_finished_when_handed_out():
+    """Another thread may use a kept plan on another stream at once: nothing
+    of its making is under way on the stream that made it."""
+    for build in ("row_groups", "mid_level", "coarse"):
+        mesh = _matrix((60, 50, 40)).mesh
+        torch.cuda.synchronize()
+        plan = mesh.coarse_space(512) if build == "coarse" else getattr(mesh, build)()
+        assert torch.cuda.current_stream().query() and plan is not None, build
