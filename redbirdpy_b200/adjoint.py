@@ -254,7 +254,9 @@ class BatchModel(DeviceModel):
 
     def tune(self, mua, dcoef):
         """Pick the solve's launch shapes for this batch with the autotuner
-        (engine.SolveTuner; cached per size bucket) and keep them."""
+        (engine.SolveTuner; cached per size bucket) and keep them.  They are
+        the separate Jacobi kernels': batches that take the V-cycle
+        (solve_kw['coarse'] 'blocks') use them in captured steps alone."""
         mat = engine.assemble(self.mesh, self.optics(mua.detach(), dcoef.detach()))
         self.solve_kw.update(engine.solve_tuner.options(mat, self.B, **self.solve_kw))
         return self.solve_kw

@@ -1214,7 +1214,7 @@ def jacobian_grad(mesh, phi, lam, ns, mua=True, dcoef=True):
     the exact node-based rows 'mua_nodal' and 'D' (real parts), one pass over
     the tets without forming a row (rb_jac_grad); None for one not asked."""
     if ns > 64:
-        raise ValueError("rb_jac stages at most 128 phi columns and 64 detectors per call")
+        raise ValueError("jacobian_grad: at most 64 column pairs per call")
     phi, lam = phi.contiguous(), lam.contiguous()
     kind = _lib.RB_C128 if phi.is_complex() else _lib.RB_F64
     gm = torch.empty(mesh.nn, dtype=torch.float64, device=phi.device) if mua else None
