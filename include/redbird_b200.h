@@ -355,6 +355,10 @@ typedef struct rb_solve_opts {
                           takes ceil(nrhs / lanes) columns, 1, 2 or 4 of them);
                           0: chosen from nrhs.  Row-pair and row-group
                           products ignore it. */
+  int32_t one_launch_only; /* nonzero: a solve in one launch (rb_femsolve_one_launch)
+                          is returned as it ends; zero: a complex solve that
+                          does not converge there within 600 iterations starts
+                          over in the separate kernels */
 } rb_solve_opts;
 
 typedef struct rb_solve_info {

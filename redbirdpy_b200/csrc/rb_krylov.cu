@@ -12,6 +12,7 @@
 // iterations.  Columns are frozen individually when they converge.
 #include <algorithm>
 #include <cmath>
+#include <limits>
 #include <type_traits>
 #include <vector>
 
@@ -2232,24 +2233,36 @@ static int solve_block(const rb_csr& A, const double* B, T64* X, int64_t ldx, in
   return RB_OK;
 }
 
-// The small-system form of femsolve_t's solve: one launch, then the outcome
+// The small-system form of femsolve_t's solve: one launch, then the outcome.
+// again: complex columns did not converge though their data are finite.  The
+// separate kernels then start over (from an initial guess: go on from X, made 0
+// in the columns where it is not finite or worse than nothing; from where these
+// FP32 iterations stalled a second solve stalled as well, from 0 it did not).
 template <typename T64, typename T>
 static int solve_small(const rb_csr& A, const double* B, T64* X, int64_t k, const rb_solve_opts& o,
                        rb_solve_info& info, SmallOut* out, const T* val, const T* dinv, const SmallPlan& p,
-                       Carver& cv, cudaStream_t st) {
+                       Carver& cv, bool* again, cudaStream_t st) {
   const T* sval = cv.take<T>((size_t)p.slots * p.cl);
   const uint16_t* scol = cv.take<uint16_t>((size_t)p.slots * p.cl);
   const int32_t* soff = cv.take<int32_t>(small_soff(p.cl, p.rpt));
   if (!sval || !scol || !soff) return fail(RB_EARG, "rb_femsolve: workspace too small");
   SmallArgs<T64, T> a{(int32_t)A.n, (int32_t)k, p.nr, p.cap, A.indptr, A.indices, (const T64*)A.val64, val, dinv,
-                      soff, sval, scol, p.slots, B, X, o.tol, o.inner_tol, std::min(o.inner_tol, 1e-6), 0.25, o.maxiter, o.max_outer, o.use_x0, out};
+                      soff, sval, scol, p.slots, B, X, o.tol, o.inner_tol, std::min(o.inner_tol, 1e-6), 0.25, o.maxiter, o.max_outer, o.use_x0,
+                      Scalar<T>::is_complex ? kSmComplexCap : std::numeric_limits<int32_t>::max() / 2, out};
   RB_TRY((small_launch<T64, T>(a, p, st)));
   std::vector<SmallOut> h(k);
   RB_CUDA_TRY(cudaMemcpyAsync(h.data(), out, sizeof(SmallOut) * k, cudaMemcpyDeviceToHost, st));
   RB_CUDA_TRY(cudaStreamSynchronize(st));
   double worst = 0.0;
   int flag = 0, iters = 0;
-  for (const SmallOut& c : h) {
+  uint64_t reset[2] = {0, 0};
+  *again = false;
+  for (size_t j = 0; j < h.size(); ++j) {
+    const SmallOut& c = h[j];
+    if (!(c.relres <= 1.0)) reset[j / 64] |= uint64_t(1) << (j % 64);
+    if (Scalar<T>::is_complex && !o.one_launch_only &&
+        (c.done == 0 || (c.done == 2 && c.relres > 1e-10) || (c.done == 3 && c.outer > 0)))
+      *again = true;
     worst = std::isfinite(c.relres) ? std::max(worst, c.relres) : c.relres;
     if (c.done == 0 || (c.done == 2 && c.relres > 1e-10)) flag = std::max(flag, 1);
     if ((c.status == 2 && c.relres > 1e-10) || c.done == 3) flag = 2;
@@ -2261,8 +2274,16 @@ static int solve_small(const rb_csr& A, const double* B, T64* X, int64_t k, cons
   // are made from this number
   info.sweep_iters_max = std::min(o.maxiter, (int)ceil_div(info.sweep_iters_max, o.check_every) * o.check_every);
   info.iters += iters;
-  info.flag = std::max(info.flag, flag);
   info.launches += 2;
+  if (*again && !o.use_x0) return RB_OK;
+  if (*again) {
+    const unsigned g = (unsigned)std::min<int64_t>(ceil_div(A.n * k, 256), 148 * 8);
+    small_reset_kernel<T64><<<g, 256, 0, st>>>(A.n, k, reset[0], reset[1], X);
+    RB_LAUNCH_CHECK();
+    info.launches += 1;
+    return RB_OK;
+  }
+  info.flag = std::max(info.flag, flag);
   info.relres = std::max(info.relres, worst);
   return RB_OK;
 }
@@ -2286,8 +2307,12 @@ static int femsolve_t(const rb_csr& A, const double* B, T64* X, int64_t nrhs, co
     if (!mid && !o.coarse && !o.groups && !o.instances && !o.profile && o.check_every > 0 && o.spmm_lanes == 0) {
       const SmallPlan sp = small_plan<T64, T>(n, A.nnz, nrhs);
       static_assert(sizeof(SmallOut) <= sizeof(ColState), "the outcome words share the column states' space");
-      if (small_wins<T>(sp, n, A.nnz, nrhs))
-        return solve_small<T64, T>(A, B, X, nrhs, o, info, reinterpret_cast<SmallOut*>(b.cs), val, dinv, sp, cv, st);
+      if (small_wins<T>(sp, n, A.nnz, nrhs)) {
+        bool again = false;
+        RB_TRY((solve_small<T64, T>(A, B, X, nrhs, o, info, reinterpret_cast<SmallOut*>(b.cs), val, dinv, sp, cv, &again,
+                                    st)));
+        if (!again) return RB_OK;
+      }
     }
   }
   double* Bp = nullptr;

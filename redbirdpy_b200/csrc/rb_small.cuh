@@ -59,8 +59,15 @@ struct SmallArgs {
   T64* X;
   double tol, inner_tol, itol_min, stall;
   int32_t maxiter, max_outer, use_x0;
+  int32_t itcap;  // iterations of a column in all
   SmallOut* out;
 };
+// Complex columns stop after this many iterations (boxes and well-shaped
+// unstructured meshes take 100 to 350).  On meshes with slivers the one-reduction
+// COCG in FP32 needs up to ten times the iterations of the two-reduction form:
+// 12,672 nodes x 16 (Delaunay, tets of 1e-6 of the cube) ended unconverged after
+// 211 ms where the separate kernels take 90; real CG needs as many as theirs.
+constexpr int kSmComplexCap = 600;
 
 __device__ __forceinline__ uint32_t cl_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
 __device__ __forceinline__ uint32_t cl_size() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r)); return r; }
@@ -373,7 +380,7 @@ __global__ void __launch_bounds__(kSmThreads, 1) small_solve_kernel(SmallArgs<T6
           c.itol2 = it * it;
         }
       }
-      if (c.open && outer < a.max_outer) {
+      if (c.open && outer < a.max_outer && c.iters < a.itcap) {
         c.active = 1;
         c.status = 0;
         c.outer += 1;
@@ -470,7 +477,7 @@ __global__ void __launch_bounds__(kSmThreads, 1) small_solve_kernel(SmallArgs<T6
           if (!isfinite(rr) || !finite_c(g)) {
             c.active = 0;
             c.status = 2;
-          } else if (rr == 0.0 || (it > 0 && rr <= c.itol2 * c.rr0) || it == a.maxiter) {
+          } else if (rr == 0.0 || (it > 0 && rr <= c.itol2 * c.rr0) || it == a.maxiter || c.iters + it >= a.itcap) {
             c.active = 0;
           } else {
             cdouble be = make_double2(0.0, 0.0), den = d;
@@ -556,6 +563,15 @@ __global__ void __launch_bounds__(kSmThreads, 1) small_solve_kernel(SmallArgs<T6
     o.sweep_max = c.sweep_max;
   }
   cl_sync();  // no block leaves while another may still read its shared memory
+}
+
+// X[:, c] = 0 for the columns of the mask
+template <typename T64>
+__global__ void small_reset_kernel(int64_t n, int64_t k, uint64_t lo, uint64_t hi, T64* __restrict__ X) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n * k; i += (int64_t)gridDim.x * blockDim.x) {
+    const int c = (int)(i % k);
+    if (((c < 64 ? lo >> c : hi >> (c - 64)) & 1) != 0) X[i] = s_zero(T64());
+  }
 }
 
 // Model time of an iteration in microseconds (fit to the measurements above):

@@ -1014,7 +1014,8 @@ def solve(mat, B, precision="mixed", tol=DEFAULT_TOL, inner_tol=None, maxiter=20
         raise ValueError("instances do not cover the matrix's rows")
     opts = _lib.RbSolveOpts(prec, int(max_outer), int(maxiter), int(check_every), float(tol),
                             float(inner_of(mid if mid is not None else cs)), int(bool(profile)), int(x0 is not None),
-                            ctypes.pointer(cs.struct) if cs is not None else None, None, None, int(spmm_lanes))
+                            ctypes.pointer(cs.struct) if cs is not None else None, None, None, int(spmm_lanes),
+                            int(redo))
     inst_status, inst_relres = [], []
     for c0 in range(0, k, 128):
         kb = min(128, k - c0)

@@ -202,3 +202,44 @@ def test_plans_kept_on_a_mesh_are_finished_when_handed_out():
         torch.cuda.synchronize()
         plan = mesh.coarse_space(512) if build == "coarse" else getattr(mesh, build)()
         assert torch.cuda.current_stream().query() and plan is not None, build
+
+
+def _slivers():
+    """A Delaunay mesh with tets of 1e-6 of the cube, frequency domain."""
+    from scipy.spatial import Delaunay
+
+    rng = np.random.default_rng(0)
+    g = np.stack(np.meshgrid(*[np.arange(float(k)) for k in (24, 24, 22)], indexing="ij"), -1).reshape(-1, 3)
+    node = g + rng.uniform(-0.3, 0.3, g.shape)
+    elem = Delaunay(node).simplices + 1
+    x = node[elem - 1]
+    vol = np.abs(np.einsum("ij,ij->i", np.cross(x[:, 1] - x[:, 0], x[:, 2] - x[:, 0]), x[:, 3] - x[:, 0])) / 6
+    node, elem = 2.0 * node, elem[vol > 1e-6]
+    nn = node.shape[0]
+    prop = np.tile([0.01, 1.0, 0.0, 1.37], (nn, 1))
+    pos = node.max(0)[None] * [[0.4, 0.4, 0.0]] + [[0, 0, 2.0]]
+    cfg = dict(node=node, elem=elem, prop=prop, srcpos=pos, srcdir=np.array([[0, 0, 1.0]]), detpos=pos,
+               detdir=np.array([[0, 0, 1.0]]), omega=2 * np.pi * 1e8)
+    cfg, _ = rbb.meshprep(cfg)
+    mesh = engine.mesh_of(cfg)
+    return engine.assemble(mesh, engine.Optics.from_cfg(mesh, cfg))
+
+
+def test_complex_columns_that_stall_in_one_launch_take_the_separate_kernels():
+    """12,672 nodes x 16 on a mesh with slivers: the one-launch COCG stops at
+    its cap and the separate kernels end the solve (flag 0, the reference FP64
+    solve within the residual times a condition of 1e6); asked for one launch
+    only, the outcome is what it is; a non-finite column is not retried."""
+    mat = _slivers()
+    B = _rhs(mat.n, 16)
+    assert _lib.lib().rb_femsolve_one_launch(mat.n, mat.struct.nnz, 16, 1)
+    X, info = engine.solve(mat, B)
+    assert info["flag"] == 0 and info["launches"] > 2 and info["relres"] <= 1e-12
+    Y, ref = engine.solve(mat, B, precision="fp64")
+    assert ref["flag"] == 0
+    assert float((X - Y).abs().max()) <= 1e-12 * 1e6 * float(Y.abs().max())
+    easy = _matrix((20, 20, 20), 2 * np.pi * 1e8)
+    C = _rhs(easy.n, 4)
+    C[3, 1] = float("nan")
+    _, info = engine.solve(easy, C)
+    assert info["flag"] == 2 and info["launches"] == 2
