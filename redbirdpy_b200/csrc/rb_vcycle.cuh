@@ -679,6 +679,11 @@ __device__ __forceinline__ cdouble vc_rru(int nb, const double* part, const cdou
   return make_double2(rr, 0.0);
 }
 
+// A column whose residual has grown to 1e8 of its start is beyond what FP32
+// brings back: COCG can diverge on meshes with slivers (32,640 nodes x 128, tets
+// of 1e-6 of the cube: 2000 iterations of one column up to 1e27 before the solve
+// was handed to the two-level form).
+constexpr double kVcDiverged = 1e16;  // of squared norms
 template <bool CX>
 __global__ void __launch_bounds__(kFinThreads)
 vc_rr_kernel(int64_t k, int nb, const double* part, const cdouble* part_u, ColState* cs, double tol2,
@@ -693,7 +698,7 @@ vc_rr_kernel(int64_t k, int nb, const double* part, const cdouble* part_u, ColSt
   s.iters += 1;
   s.rr = rr;
   s.pq = u;
-  if (!isfinite(rr)) {
+  if (!(rr <= kVcDiverged * s.rr0)) {  // (or not finite)
     s.active = 0;
     s.status = 2;
   } else if (rr <= (s.tol2 >= 0.0 ? s.tol2 : tol2) * s.rr0) {

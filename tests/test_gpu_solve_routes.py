@@ -204,20 +204,22 @@ def test_plans_kept_on_a_mesh_are_finished_when_handed_out():
         assert torch.cuda.current_stream().query() and plan is not None, build
 
 
-def _slivers():
+def _slivers(m=(24, 24, 22)):
     """A Delaunay mesh with tets of 1e-6 of the cube, frequency domain."""
     from scipy.spatial import Delaunay
 
     rng = np.random.default_rng(0)
-    g = np.stack(np.meshgrid(*[np.arange(float(k)) for k in (24, 24, 22)], indexing="ij"), -1).reshape(-1, 3)
+    g = np.stack(np.meshgrid(*[np.arange(float(k)) for k in m], indexing="ij"), -1).reshape(-1, 3)
     node = g + rng.uniform(-0.3, 0.3, g.shape)
     elem = Delaunay(node).simplices + 1
     x = node[elem - 1]
     vol = np.abs(np.einsum("ij,ij->i", np.cross(x[:, 1] - x[:, 0], x[:, 2] - x[:, 0]), x[:, 3] - x[:, 0])) / 6
     node, elem = 2.0 * node, elem[vol > 1e-6]
     nn = node.shape[0]
-    prop = np.tile([0.01, 1.0, 0.0, 1.37], (nn, 1))
-    pos = node.max(0)[None] * [[0.4, 0.4, 0.0]] + [[0, 0, 2.0]]
+    rng = np.random.default_rng(0)
+    prop = np.column_stack([rng.uniform(0.008, 0.012, nn), rng.uniform(0.9, 1.1, nn), np.zeros(nn),
+                            np.full(nn, 1.37)])
+    pos = node.max(0)[None] * [[0.4, 0.4, 0.0]] + [[0, 0, 1e-3]]
     cfg = dict(node=node, elem=elem, prop=prop, srcpos=pos, srcdir=np.array([[0, 0, 1.0]]), detpos=pos,
                detdir=np.array([[0, 0, 1.0]]), omega=2 * np.pi * 1e8)
     cfg, _ = rbb.meshprep(cfg)
@@ -243,3 +245,24 @@ def test_complex_columns_that_stall_in_one_launch_take_the_separate_kernels():
     C[3, 1] = float("nan")
     _, info = engine.solve(easy, C)
     assert info["flag"] == 2 and info["launches"] == 2
+
+
+def test_diverging_cycle_columns_end_their_sweep(monkeypatch):
+    """COCG columns that diverge on a mesh with slivers are given up when
+    their residual has grown to 1e8 of its start, long before the cap of 2000."""
+    mat = _slivers((34, 32, 30))
+    seen, real = [], engine.call
+
+    def call(name, *a):
+        real(name, *a)
+        if name == "rb_femsolve_mid":
+            seen.append((a[6]._obj.flag, a[6]._obj.sweep_iters_max, a[6]._obj.relres))
+
+    monkeypatch.setattr(engine, "call", call)
+    g = torch.Generator("cuda").manual_seed(128)
+    B = torch.zeros((mat.n, 128), dtype=torch.float64, device="cuda")
+    B.scatter_(0, torch.randint(0, mat.n, (4, 128), device="cuda", generator=g), 1.0)
+    engine.solve(mat, B, maxiter=2000)
+    assert len(seen) == 1
+    flag, sweep, relres = seen[0]
+    assert flag == 0 or (sweep < 1000 and relres < 1e9), seen
